@@ -17,9 +17,9 @@ after every accepted substep, plus that substep's water update):
     27 add/mul + 10 divisions + 2 pow per level
 
 An add, subtract or multiply is one FP64 pipe instruction, as a DFMA is.  A pow
-(clm_math.h, a double-double logarithm and exponential) is a sequence of them; its cost
-in DFMA-equivalents is the ratio of the DFMA rate to its rate, both measured on the
-device by the probe (clm.jl_gb300/probe/fp64_probe.cu).  The divisions run on the
+(clm_math.h: fixed point on the integer pipes, with an FP64 fallback where its rounding
+test does not decide) is charged its time: the ratio of the DFMA rate to its rate, both
+measured on the device by the probe (clm.jl_gb300/probe/fp64_probe.cu).  The divisions run on the
 integer pipes (jl_div: cm_div's 64-bit reciprocal and 2/1 division), not on the FP64
 pipe, so they add nothing to the FP64 work; they are counted separately.  The kernel
 counts the levels of its attempts and refreshes itself (CLMGB_OPT_COUNT_WORK), so

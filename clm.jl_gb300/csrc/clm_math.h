@@ -8,9 +8,8 @@
 //
 // Every operation is an IEEE-754 binary64 add, multiply or fused multiply-add
 // written out explicitly (CUDA: __dadd_rn/__dmul_rn/__fma_rn; C: +, *, fma() built
-// with -ffp-contract=off), so a C build and a CUDA build return the same bits.  On
-// GB300, whose FP64 pipe issues about 1.9 FMA/clk/SM, a pow() here costs about 40 FP64
-// instructions; exponent and table-index handling use the integer pipes.
+// with -ffp-contract=off), so a C build and a CUDA build return the same bits.  The CUDA
+// build forms division, pow and log10 on the integer pipes, with the same bits (below).
 //
 // pow and log10 go through a double-double logarithm (cm_log_dd: Tang's table with an
 // extra-precision log(c) and an exactly formed reduced argument, the error-free sums
@@ -36,7 +35,7 @@
 #if defined(__CUDACC__)
 #define CM_FN static __device__ __forceinline__
 #define CM_TABLE(name, n) static __device__ const double name[n]
-#define CM_TABLE_U16(name, n) static __device__ const uint16_t name[n]
+#define CM_TABLE_OF(type, name, n) static __device__ const type name[n]
 #define CM_LD(p) __ldg(&(p))
 #define CM_FMA(a, b, c) __fma_rn((a), (b), (c))
 #define CM_MUL(a, b) __dmul_rn((a), (b))
@@ -55,7 +54,7 @@
 #include <string.h>
 #define CM_FN static inline
 #define CM_TABLE(name, n) static const double name[n]
-#define CM_TABLE_U16(name, n) static const uint16_t name[n]
+#define CM_TABLE_OF(type, name, n) static const type name[n]
 #define CM_LD(p) (p)
 #define CM_FMA(a, b, c) fma((a), (b), (c))
 #define CM_MUL(a, b) ((a) * (b))
@@ -75,20 +74,30 @@ static inline double cm_as_f64_(uint64_t u) { double x; memcpy(&x, &u, 8); retur
 #include "clm_math_tables.h"
 
 // ---- binary64 division on the integer pipes ----
-// The correctly rounded quotient x / y formed with 64-bit integer arithmetic: on GB300
-// an FP64 instruction occupies its sub-partition's FP64 unit for about 64 cycles (2
-// lanes per clock per SM) while a 32-bit integer multiply-add takes about 2, so a
-// division done in integers leaves the FP64 pipe, which bounds the column kernels, to
-// the rest of the arithmetic.  Method: N. Moller and T. Granlund, "Improved division
-// by invariant integers", IEEE Trans. Computers 60(2), 2011: the reciprocal
-// v = floor((2^128 - 1) / d) - 2^64 of a normalised 64-bit divisor d (their
-// reciprocal_word, seeded from CM_RECIP_V0) and the 2/1 division of a two-word
-// numerator by d with v (div_2by1), which gives the exact quotient and remainder.
-// With d = my * 2^11 and the numerator mx * 2^66 (mx, my the 53-bit significands) the
-// quotient is floor(mx * 2^55 / my), 55 or 56 bits, and the remainder says whether
-// anything was cut off: round to nearest even from there.  Zero, subnormal, infinite
-// or NaN operands, and quotients below the normal range or above it, take the
-// ordinary division (CM_DIV), so the result always equals it.
+// The correctly rounded quotient x / y formed with integer arithmetic: on GB300 an FP64
+// instruction holds its sub-partition's FP64 unit for about 65 cycles (half a lane per
+// clock) while a 32-bit integer multiply-add takes about 2, so a division done in
+// integers leaves the FP64 unit, which bounds the column kernels, to the rest of the
+// arithmetic.  Method: very-high-radix long division with quotient digits from a short
+// reciprocal (D. Wong and M. Flynn, "Fast division using accurate quotient
+// approximations to reduce the number of iterations", IEEE Trans. Computers 41(8),
+// 1992).  With the 53-bit significands X (doubled when below Y, so that X/Y lies in
+// [1, 2)) and Y:
+//   R        an underestimate of 2^83 / Y, from a single-precision reciprocal of Y's
+//            leading 24 bits: 0 <= 2^83/Y - R < 2600 (R >= 2^30 - 2600)
+//   d1       floor-like 23-bit digit of X/Y, deficit below 43; the remainder
+//            X 2^23 - d1 Y < 43 Y, exact modulo 2^64
+//   d2       17 bits of that remainder over Y, deficit below 16
+//   d3       12 bits, deficit below 1.3: X 2^52 = q Y + rem with 0 <= rem < 1.3 Y
+// A quotient of two 53-bit significands is never a midpoint of two neighbours, so
+// q + (2 rem > Y) is the quotient rounded to nearest (for rem in [Y, 1.3 Y) as well).
+// The digits are correct for any R within its bounds, so the result does not depend on
+// the rounding of the single-precision reciprocal.  Zero, subnormal, infinite or NaN
+// operands, and quotients below the normal range or within a binade of overflow, take
+// the ordinary division (CM_DIV), so the result always equals it.  Called out of line, a
+// dependent chain on GB300 measures 408 cycles a division at one warp per sub-partition
+// and 155 issue cycles with four (275 and 112 inlined); the 64-bit reciprocal and 2/1
+// division it replaced measured 857 and 345, the hardware division 569 and 549.
 CM_FN uint64_t cm_umulhi_(uint64_t a, uint64_t b) {
 #if defined(__CUDACC__)
   return __umul64hi(a, b);
@@ -96,70 +105,61 @@ CM_FN uint64_t cm_umulhi_(uint64_t a, uint64_t b) {
   return (uint64_t)(((unsigned __int128)a * b) >> 64);
 #endif
 }
-
-// floor((2^128 - 1) / d) - 2^64 for d >= 2^63
-CM_FN uint64_t cm_recip_word_(uint64_t d) {
-  const uint64_t d0 = d & 1;
-  const uint64_t d9 = d >> 55;                               // 256..511
-  const uint64_t d40 = (d >> 24) + 1;
-  const uint64_t d63 = (d >> 1) + d0;                        // ceil(d / 2)
-  const uint64_t v0 = CM_LD(CM_RECIP_V0[d9 - 256]);
-  const uint64_t v1 = (v0 << 11) - ((v0 * v0 * d40) >> 40) - 1;
-  const uint64_t v2 = (v1 << 13) + ((v1 * ((1ULL << 60) - v1 * d40)) >> 47);
-  const uint64_t e = ((v2 >> 1) & (0 - d0)) - v2 * d63;    // 2^96 - v2 d63 + floor(v2/2) d0, mod 2^64
-  const uint64_t v3 = (v2 << 31) + (cm_umulhi_(v2, e) >> 1);
-  // v3 - floor((v3 + 2^64 + 1) d / 2^64)
-  const uint64_t lo = v3 * d;
-  const uint64_t lo2 = lo + d;
-  const uint64_t hi = cm_umulhi_(v3, d) + (lo2 < lo) + d;
-  return v3 - hi;
+CM_FN uint32_t cm_umulhi32_(uint32_t a, uint32_t b) {
+#if defined(__CUDACC__)
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
 }
 
-// floor((u1 2^64 + u0) / d) and its remainder, for u1 < d, d >= 2^63, v its reciprocal
-CM_FN uint64_t cm_div2by1_(uint64_t u1, uint64_t u0, uint64_t d, uint64_t v, uint64_t* rem) {
-  uint64_t q0 = v * u1;
-  uint64_t q1 = cm_umulhi_(v, u1);
-  q0 += u0;
-  q1 += u1 + (q0 < u0);
-  q1 += 1;
-  uint64_t r = u0 - q1 * d;
-  if (r > q0) {
-    q1 -= 1;
-    r += d;
-  }
-  if (r >= d) {
-    q1 += 1;
-    r -= d;
-  }
-  *rem = r;
-  return q1;
+// R of a significand with the hidden bit set.  The reciprocal is taken of Y's leading
+// 22 bits with the next two set, at most 3 * 2^-23 above Y / 2^52 and always above 1, so
+// that it lies below 1: its fraction is R's.  The argument's distance and the
+// reciprocal's error (2^-23) come to less than 1300 units of 2^-31; R is lowered by as
+// much.
+CM_FN uint32_t cm_div_seed_(uint64_t my) {
+  const uint32_t fb = 0x3f800003u | ((uint32_t)(my >> 29) & 0x7fffffu);
+#if defined(__CUDACC__)
+  float g;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(__uint_as_float(fb)));
+  const uint32_t gb = __float_as_uint(g);
+#else
+  float fv, g;
+  memcpy(&fv, &fb, 4);
+  g = 1.0f / fv;
+  uint32_t gb;
+  memcpy(&gb, &g, 4);
+#endif
+#if defined(CM_DIV_SEED_ULPS)
+  return ((gb << 7) ^ 0xC0000000u) + 128 * CM_DIV_SEED_ULPS - 1300u;   // tests: other roundings
+#else
+  return ((gb << 7) ^ 0xC0000000u) - 1300u;                  // 2^31 g from g's bits, g in [1/2, 1)
+#endif
 }
 
 CM_FN double cm_div(double x, double y) {
   const uint64_t bx = CM_AS_U64(x), by = CM_AS_U64(y);
-  const uint64_t ex = (bx >> 52) & 0x7ff, ey = (by >> 52) & 0x7ff;
-  if (ex - 1 >= 0x7fe || ey - 1 >= 0x7fe) return CM_DIV(x, y);   // zero, subnormal, Inf or NaN
+  const uint32_t ex = (uint32_t)(bx >> 52) & 0x7ff, ey = (uint32_t)(by >> 52) & 0x7ff;
   const uint64_t frac = 0x000fffffffffffffULL, hidden = 0x0010000000000000ULL;
-  const uint64_t sign = (bx ^ by) & 0x8000000000000000ULL;
   const uint64_t mx = (bx & frac) | hidden, my = (by & frac) | hidden;
-  int64_t e = (int64_t)ex - (int64_t)ey + 1023;
-  uint64_t m = mx;                                          // y a power of two: x rescaled
-  if (my != hidden) {
-    const uint64_t d = my << 11;
-    uint64_t r;
-    const uint64_t q = cm_div2by1_(mx << 2, 0, d, cm_recip_word_(d), &r);   // floor(mx 2^55 / my)
-    const int sh = (q >> 55) ? 3 : 2;                       // 56 bits: quotient >= 1
-    if (sh == 2) e -= 1;
-    m = q >> sh;
-    const uint64_t cut = q & ((1ULL << sh) - 1), half = 1ULL << (sh - 1);
-    if (cut > half || (cut == half && (r != 0 || (m & 1)))) m += 1;
-    if (m >> 53) {
-      m >>= 1;
-      e += 1;
-    }
-  }
-  if (e < 1 || e > 0x7fe) return CM_DIV(x, y);             // subnormal or infinite quotient
-  return CM_AS_F64(sign | ((uint64_t)e << 52) | (m & frac));
+  const uint32_t lt = mx < my;
+  const uint32_t e = ex - ey + 1023u - lt;                  // the quotient's exponent field
+  // zero, subnormal, infinite or NaN operands; a quotient not safely normal
+  if (ex - 1u >= 0x7feu || ey - 1u >= 0x7feu || e - 1u >= 0x7fdu) return CM_DIV(x, y);
+  const uint64_t X = mx << lt;
+  const uint32_t R = cm_div_seed_(my);
+  const uint32_t d1 = cm_umulhi32_((uint32_t)(X >> 22), R) >> 6;
+  uint64_t rem = (X << 23) - d1 * my;
+  const uint32_t d2 = cm_umulhi32_((uint32_t)(rem >> 27), R) >> 7;
+  rem = (rem << 17) - d2 * my;
+  const uint32_t d3 = cm_umulhi32_((uint32_t)(rem >> 25), R) >> 14;
+  rem = (rem << 12) - d3 * my;
+  uint64_t m = ((uint64_t)d1 << 29) + ((uint64_t)d2 << 12) + d3;
+  m += (rem << 1) > my;
+  // m is in [2^52, 2^53]: its hidden bit, or the carry of a round up to 2, adds to the
+  // exponent field
+  return CM_AS_F64(((bx ^ by) & 0x8000000000000000ULL) + ((uint64_t)(e - 1) << 52) + m);
 }
 
 // Natural logarithm.
@@ -354,7 +354,7 @@ CM_FN bool cm_pow_by_squaring(uint64_t uy, int64_t* n) {
 // x == 0 -> 0 or Inf; x < 0 with non-integral y -> NaN (Julia raises a DomainError);
 // otherwise exp(y log x) in double-double.  The tests of the common case look at bit
 // patterns (integer pipes).
-CM_FN double cm_pow(double x, double y) {
+CM_FN double cm_pow_dd(double x, double y) {
   const uint64_t ux = CM_AS_U64(x), uy = CM_AS_U64(y);
   if (ux == 0x3ff0000000000000ULL) return 1.0;
   if ((uy << 1) > 0xffe0000000000000ULL) return y;          // y NaN
@@ -384,21 +384,8 @@ CM_FN double cm_pow(double x, double y) {
   return neg ? -v : v;
 }
 
-// x^y for a positive finite x other than 1 whose logarithm lxh + lxl = cm_log_dd(x) the
-// caller formed once: the value of cm_pow(x, y) for every y, without forming the
-// logarithm again.
-CM_FN double cm_pow_lx(double x, double lxh, double lxl, double y) {
-  const uint64_t uy = CM_AS_U64(y);
-  if ((uy << 1) > 0xffe0000000000000ULL) return y;
-  int64_t n;
-  if (cm_pow_by_squaring(uy, &n)) return n == 0 ? 1.0 : jl_pow_int(x, n);
-  const double eh = CM_MUL(y, lxh);
-  const double el = CM_FMA(y, lxl, CM_FMA(y, lxh, -eh));
-  return cm_exp_dd(eh, el);
-}
-
 // Base-10 logarithm: the double-double log times 1/ln10 in two parts.
-CM_FN double cm_log10(double x) {
+CM_FN double cm_log10_dd(double x) {
   const uint64_t ix = CM_AS_U64(x);
   if (ix - 0x0010000000000000ULL >= 0x7ff0000000000000ULL - 0x0010000000000000ULL) {
     if (x != x) return x;                                   // NaN
@@ -413,6 +400,182 @@ CM_FN double cm_log10(double x) {
   const double vl = CM_ADD(CM_FMA(h, CM_INVLN10_HI, -v), CM_FMA(h, CM_INVLN10_LO, CM_MUL(l, CM_INVLN10_HI)));
   return CM_ADD(v, vl);
 }
+
+// ---- pow and log10 on the integer pipes ----
+// cm_pow_dd and cm_log10_dd above take 42 and 31 FP64 instructions, 65 cycles of the FP64 unit
+// each on GB300.  The same values are formed here in fixed point with 32-bit integer
+// multiplies and rounded to nearest, and kept only where the rounding cannot differ from
+// the FP64 functions': both are within a known distance of the true value before their
+// last rounding, so when the fixed-point value lies further than the sum of the two
+// distances from a midpoint of neighbouring doubles, both round to the same double.  The
+// others (0.6 % of the values of pow, 0.3 % of log10 and its arguments near 1) run the
+// FP64 function.  The result is therefore the FP64 function's, bit for bit (Ziv's
+// rounding test: A. Ziv, "Fast evaluation of elementary mathematical functions with
+// correctly rounded last bit", ACM TOMS 17(3), 1991).  Measured on GB300, a chain of
+// cm_pow with 32 different lanes, cycles a call at one warp per sub-partition / issue
+// cycles with four: 3,050 / 3,140 in FP64, 1,600 / 800 so (the FP64 fallback of one lane
+// in some 5 calls of a warp included); cm_log10 2,170 / 2,340 and 890 / 370.
+//
+// log2(x) = k + log2(2^11 / C_i) + log2(1 + r), 1 + r = z C_i / 2^11 formed exactly (C_i
+// of 11 bits for the 256 intervals of the significand z, r in [0, 2^-7.8)), log2(1 + r)
+// its series to r^9, kept to 96 fractional bits: absolute error below 2^-71.
+// 2^t, t in [0, 2^-8), by its series to t^6, times a 64-bit 2^(j/256).
+
+// a*b >> 64 without the low partial product: at most 2 below
+CM_FN uint64_t cm_umulhi_lo_(uint64_t a, uint64_t b) {
+  const uint64_t ah = a >> 32, bh = b >> 32;
+  const uint32_t al = (uint32_t)a, bl = (uint32_t)b;
+  return ah * bh + ((ah * bl) >> 32) + ((al * bh) >> 32);
+}
+
+// |log2(x)| for the bits ix of a positive normal x, as a multiple of 2^-96 in *hi : *lo
+// (128 bits); returns 1 when log2(x) is negative.
+CM_FN uint32_t cm_log2_fx_(uint64_t ix, uint64_t* hi, uint64_t* lo) {
+  const int64_t k = (int64_t)(ix >> 52) - 1023;
+  const uint64_t m = (ix & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
+  const int i = (int)((ix >> 44) & 255);
+  const uint64_t u = (m * (uint64_t)CM_LD(CM_FX_C[i]) - 0x8000000000000000ULL) << 8;   // r 2^7, Q64
+  const uint32_t uh = (uint32_t)(u >> 32);
+  uint32_t q = CM_FX_C8 - (cm_umulhi32_(uh, CM_FX_C9) >> 7);
+  q = CM_FX_C7 - (cm_umulhi32_(uh, q) >> 7);
+  q = CM_FX_C6 - (cm_umulhi32_(uh, q) >> 7);
+  uint64_t p = CM_FX_C5 - (((uint64_t)uh * q) >> 7);
+  p = CM_FX_C4 - (cm_umulhi_lo_(u, p) >> 7);
+  p = CM_FX_C3 - (cm_umulhi_lo_(u, p) >> 7);
+  p = CM_FX_C2 - (cm_umulhi_lo_(u, p) >> 7);
+  p = CM_FX_C1 - (cm_umulhi_lo_(u, p) >> 7);                 // 1 + p = log2(1 + r) / r
+  const uint64_t sl = u * p, sh = u + cm_umulhi_(u, p);      // log2(1 + r) 2^7, Q128
+  const uint64_t th = CM_LD(CM_FX_LHI[i]);
+  const uint64_t tl = (th << 32) | CM_LD(CM_FX_LLO[i]);
+  uint64_t l = (sh << 25) | (sl >> 39);
+  uint64_t h = (sh >> 39) + ((uint64_t)k << 32) + (th >> 32);
+  l += tl;
+  h += l < tl;
+  const uint32_t neg = (uint32_t)(h >> 63);
+  if (neg) {
+    h = ~h + (l == 0);
+    l = 0 - l;
+  }
+  *hi = h;
+  *lo = l;
+  return neg;
+}
+
+// floor(log2 v) - 48 for v >= 2^49
+CM_FN int cm_top_bit_(uint64_t v) {
+#if defined(__CUDACC__)
+  return 15 - __clzll((long long)v);
+#else
+  return 15 - __builtin_clzll(v);
+#endif
+}
+
+// x^y in fixed point; false when the rounding test does not decide, or x and y are not
+// x positive and normal within 2^-60..2^60, y not an integer and 2^-40 <= |y| < 64, or
+// the result is not safely normal.
+CM_FN bool cm_pow_fx(double x, double y, double* out) {
+  const uint64_t ux = CM_AS_U64(x), uy = CM_AS_U64(y);
+  const uint32_t ey = (uint32_t)(uy >> 52) & 0x7ff;
+  const uint64_t my = (uy << 11) | 0x8000000000000000ULL;
+  const bool whole = ey >= 1023 && ((my << 1) << (ey - 1023)) == 0;
+  if (ux - (963ULL << 52) >= (120ULL << 52) || ux == 0x3ff0000000000000ULL || ey - 983u >= 46u || whole) return false;
+  uint64_t h, l;
+  const uint32_t neg = cm_log2_fx_(ux, &h, &l) ^ (uint32_t)(uy >> 63);
+  const uint64_t mh = (h << 26) | (l >> 38);                 // |log2 x| Q58, below 2^6
+  const uint64_t ml = (l << 26) & 0xffffffff00000000ULL;     // its next 32 bits
+  uint64_t pl = my * mh, ph = cm_umulhi_(my, mh);
+  const uint64_t pe = cm_umulhi_lo_(my, ml);
+  pl += pe;
+  ph += pl < pe;                                             // |y log2 x| = ph:pl 2^(ey - 1023 - 121)
+  const uint32_t sh = 1080u - ey;                            // 52..97
+  uint64_t n, f;                                             // integer part, fraction Q64
+  if (sh < 64) {
+    n = ph >> sh;
+    f = (ph << (64 - sh)) | (pl >> sh);
+  } else {
+    n = 0;
+    f = sh == 64 ? ph : ph >> (sh - 64);
+  }
+  if (neg) {
+    n = ~n + (f == 0);
+    f = 0 - f;
+  }
+  if (n + 1000 >= 2000) return false;
+  const int j = (int)(f >> 56);
+  const uint64_t u = f << 8;                                 // t 2^8, Q64
+  const uint32_t uh = (uint32_t)(u >> 32);
+  uint32_t q = CM_FX_D5 + (cm_umulhi32_(uh, CM_FX_D6) >> 8);
+  q = CM_FX_D4 + (cm_umulhi32_(uh, q) >> 8);                 // Q38
+  uint64_t p = CM_FX_D3 + (((uint64_t)uh * q) >> 14);
+  p = CM_FX_D2 + (cm_umulhi_lo_(u, p) >> 8);
+  p = CM_FX_D1 + (cm_umulhi_lo_(u, p) >> 8);
+  p = cm_umulhi_lo_(u, p);                                   // (2^t - 1) 2^8, Q64
+  const uint64_t t = CM_LD(CM_FX_E[j]);
+  const uint64_t r = t + ((cm_umulhi_lo_(t, p) + 128) >> 8);   // 2^f, Q63
+  // The two values' distances from the true one, in units of 2^-63 (r in [2^63, 2^64)).
+  // Here: 1/2 from the table, 1/2 from the last shift, below 0.5 from the logarithm
+  // times y and the series.  cm_exp_dd: below 0.4 from its logarithm times y and its
+  // series, and half a unit in the last place of each of three numbers of |argument|'s
+  // binade times 2^(j/256) (the reduced argument, rounded twice, and expm1) and of the
+  // product.  tm bounds the argument's magnitude / ln2, tm th8/8 the product's.  In 64ths:
+  uint64_t tm = u >> 8;
+  tm = (tm >> 55 ? (1ULL << 56) - tm : tm) + (1ULL << 49);
+  const uint32_t th8 = (uint32_t)(t >> 60) + 1;              // 2^(j/256) < th8 / 8
+  const uint64_t tw = (tm >> 3) * th8 + th8;
+  const uint32_t thr = (128u + (((3u << cm_top_bit_(tm)) * th8) >> 3) + (1u << cm_top_bit_(tw))) >> 6;
+  const uint32_t rest = (uint32_t)r & 0x7ff;
+  if (rest - (0x400u - thr) <= 2 * thr || (r >> 63) == 0) return false;
+  const uint64_t mant = (r >> 11) + (rest >> 10);
+  *out = CM_AS_F64(((n + 1022) << 52) + mant);
+  return true;
+}
+
+// log10(x) in fixed point; false when the rounding test does not decide, x is not
+// positive and normal within 2^-60..2^60, or |log10 x| < 2^-6.
+CM_FN bool cm_log10_fx(double x, double* out) {
+  const uint64_t ux = CM_AS_U64(x);
+  if (ux - (963ULL << 52) >= (120ULL << 52)) return false;
+  uint64_t h, l;
+  const uint32_t neg = cm_log2_fx_(ux, &h, &l);
+  const uint64_t mh = (h << 26) | (l >> 38);                 // Q58
+  const uint64_t ml = (l << 26) & 0xffffffff00000000ULL;
+  uint64_t pl = mh * CM_FX_LOG10_2_HI, ph = cm_umulhi_(mh, CM_FX_LOG10_2_HI);
+  uint64_t pe = cm_umulhi_lo_(ml, CM_FX_LOG10_2_HI) + ((mh >> 32) * CM_FX_LOG10_2_LO);
+  pl += pe;
+  ph += pl < pe;                                             // Q122
+  if (ph < (1ULL << 52)) return false;
+#if defined(__CUDACC__)
+  const int lz = __clzll((long long)ph);
+#else
+  const int lz = __builtin_clzll(ph);
+#endif
+  const uint64_t r = lz ? (ph << lz) | (pl >> (64 - lz)) : ph;
+  // this value's distance from the true one is below 1 unit in the 64th place, cm_log10's
+  // before its last rounding below 1/8
+  const uint32_t rest = (uint32_t)r & 0x7ff;
+  if (rest - 0x3feu <= 4u) return false;
+  const uint64_t mant = (r >> 11) + (rest >> 10);
+  *out = CM_AS_F64(((uint64_t)neg << 63) + ((uint64_t)(1027 - lz) << 52) + mant);
+  return true;
+}
+
+#if defined(__CUDACC__)
+// The kernels' pow and log10 (one out-of-line copy of each, and of the FP64 functions).
+static __device__ __noinline__ double cm_pow_dd_call_(double x, double y) { return cm_pow_dd(x, y); }
+static __device__ __noinline__ double cm_log10_dd_call_(double x) { return cm_log10_dd(x); }
+CM_FN double cm_pow_inl(double x, double y) {
+  double v;
+  return cm_pow_fx(x, y, &v) ? v : cm_pow_dd_call_(x, y);
+}
+static __device__ __noinline__ double cm_pow(double x, double y) { return cm_pow_inl(x, y); }
+static __device__ __noinline__ double cm_log10(double x) {
+  double v;
+  return cm_log10_fx(x, &v) ? v : cm_log10_dd_call_(x);
+}
+#else
+CM_FN double cm_pow(double x, double y) { return cm_pow_dd(x, y); }
+CM_FN double cm_log10(double x) { return cm_log10_dd(x); }
+#endif
 
 // sin and cos of a reduced argument r + lo, |r| <= pi/4, |lo| <= ulp(r) (Taylor
 // polynomials in r^2; lo enters to first order: sin' = cos ~ 1 - r^2/2, cos' = -sin ~ -r).

@@ -61,13 +61,21 @@ struct Dims {
 // Julia Base.max / Base.min on Float64 (NaN propagates, -0.0 < 0.0).  They only
 // select one argument, so they are done on the integer pipes: the bit pattern
 // mapped to a two's-complement key orders doubles exactly (-0.0 below +0.0), and
-// NaN is recognised from its bits.  No FP64 instruction is spent on them.
+// NaN is recognised from its bits.  The bits are moved by an instruction the compiler
+// does not see through: it recognises integer tests of a double's bits and turns them
+// back into FP64 compares, each 65 cycles of the FP64 unit (a chain of jl_max measured
+// 78 issue cycles an operation with four warps per sub-partition, 40 so).
+__device__ __forceinline__ long long dbits(double x) {
+  long long b;
+  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+  return b;
+}
 __device__ __forceinline__ long long ord_key(double x) {
-  const long long b = __double_as_longlong(x);
+  const long long b = dbits(x);
   return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
 __device__ __forceinline__ bool isnan_bits(double x) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+  return (dbits(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
 }
 __device__ __forceinline__ double jl_max(double x, double y) {
   if (isnan_bits(x)) return x;
@@ -80,20 +88,18 @@ __device__ __forceinline__ double jl_min(double x, double y) {
   return ord_key(x) <= ord_key(y) ? x : y;
 }
 // Julia's Float64 x / y (IEEE, round to nearest), formed on the integer pipes.  On
-// GB300 an FP64 instruction holds its sub-partition's FP64 unit for about 64 cycles,
-// and the column kernels are bound by that unit; cm_div (clm_math.h) forms the
-// correctly rounded quotient of normal operands with 64-bit integer arithmetic
-// instead (measured: 141 against 70 G divisions/s alone, and next to FP64 work it
-// costs almost nothing, since it runs on the otherwise idle integer pipes).  A zero x
-// over a finite nonzero y, common in this solve (the ice of unfrozen levels, the
-// excess ice, the phase-change heat of levels that neither melt nor freeze, the band
-// system's zero sub-diagonal), is the zero with the xor of the signs, from the bits;
-// the hardware division is 2.6x slower than usual there (27 against 70 G/s).  Every
-// other case (subnormal, infinite or NaN operands, quotients outside the normal range)
-// is the hardware division.  The result is always the IEEE quotient.
-// (one out-of-line copy of the integer division: measured faster than a copy inlined
-// at every call site, 4.2 against 5.6 ms for the part of a step at 262,144 columns
-// outside the Richards solve, and 10.5 against 17.7 ms for the Richards solve)
+// GB300 an FP64 instruction holds its sub-partition's FP64 unit for about 65 cycles,
+// and the column kernels are bound by that unit and by the length of their serial
+// chains; cm_div (clm_math.h) forms the correctly rounded quotient of normal operands
+// with integer multiplies instead (155 issue cycles against 549 of the hardware
+// division).  A zero x over a finite nonzero y, common in this solve (the ice of
+// unfrozen levels, the excess ice, the phase-change heat of levels that neither melt
+// nor freeze, the band system's zero sub-diagonal), is the zero with the xor of the
+// signs, from the bits.  Every other case (subnormal, infinite or NaN operands,
+// quotients outside the normal range) is the hardware division.  The result is always
+// the IEEE quotient.
+// (one out-of-line copy: a copy inlined at every call site of the soil-temperature
+// kernel measured slower)
 static __device__ __noinline__ double cm_div_call(double x, double y) { return cm_div(x, y); }
 __device__ __forceinline__ double jl_div(double x, double y) {
   const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
@@ -110,7 +116,7 @@ __device__ __forceinline__ auto jl_div(A x, B y) {
 }
 // |x| < t for a positive threshold t, on the integer pipes (false for NaN, as in IEEE).
 __device__ __forceinline__ bool abs_lt(double x, double t) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) < __double_as_longlong(t);
+  return (dbits(x) & 0x7fffffffffffffffLL) < dbits(t);
 }
 // Julia's Float64 x^4 (Base.Math.pow_body, compensated squaring).
 __device__ __forceinline__ double jl_pow4(double x) {
@@ -696,9 +702,6 @@ __device__ inline uint32_t soil_temperature_col(const Dims& D, const clmgb_soilt
   double zz[MAXL + 2];
 
   // ---- soil_therm_prop!: layer conductivity thk (_soil_snow_tk_kernel! :647-716) ----
-  // the logarithms of the two constant bases of tkwat^x and tkice^x, formed once
-  double ln_tkwat_lo, ln_tkice_lo;
-  const double ln_tkwat = cm_log_dd(TKWAT, &ln_tkwat_lo), ln_tkice = cm_log_dd(TKICE, &ln_tkice_lo);
   // thk kept in tk[] first, interface conductivity computed in place afterwards.
   for (int jj = jjtop; jj <= nlev; jj++) {
     tt[jj] = X.T(jj);
@@ -726,8 +729,7 @@ __device__ inline uint32_t soil_temperature_col(const Dims& D, const clmgb_soilt
             const S fl_denom = a1 + jl_div(ice, DENICE * dzv) + jl_div(exi, DENICE * dzv);
             const S fl = jl_div(a1, fl_denom);
             const S dksat =
-                LVc(f.tkmg, c, j, ld) * cm_pow_lx(TKWAT, ln_tkwat, ln_tkwat_lo, fl * ws) *
-                cm_pow_lx(TKICE, ln_tkice, ln_tkice_lo, (1.0 - fl) * ws);
+                LVc(f.tkmg, c, j, ld) * cm_pow(TKWAT, fl * ws) * cm_pow(TKICE, (1.0 - fl) * ws);
             thkv = dke * dksat + (1.0 - dke) * LVc(f.tkdry, c, j, ld);
           } else {
             thkv = LVc(f.tkdry, c, j, ld);
@@ -1096,10 +1098,8 @@ constexpr int LOG_FIN = 3 * MAXSOI + 3;
 // layer), as formed at soil_water_movement.jl:1287-1293.
 template <class ST>
 __device__ __forceinline__ typename ST::S mf_impedance(double e_ice, int j, int nlayers, ST& X) {
-  double ln10_lo;
-  const double ln10 = cm_log_dd(10.0, &ln10_lo);
-  if (j == nlayers) return cm_pow_lx(10.0, ln10, ln10_lo, -e_ice * X.Icefrac(j));
-  return cm_pow_lx(10.0, ln10, ln10_lo, -e_ice * (0.5 * (X.Icefrac(j) + X.Icefrac(j + 1))));
+  if (j == nlayers) return cm_pow(10.0, -e_ice * X.Icefrac(j));
+  return cm_pow(10.0, -e_ice * (0.5 * (X.Icefrac(j) + X.Icefrac(j + 1))));
 }
 __device__ __forceinline__ double mf_impedance(const Dims& D, const clmgb_soilwater_fields& f, double e_ice,
                                                int64_t c, int j, int nlayers) {

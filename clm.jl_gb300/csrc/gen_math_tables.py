@@ -125,12 +125,7 @@ def main():
     p2 = float(mp.pi / 2)
     lines.append("#define CM_PIO2_H (%s)" % hexd(p2))
     lines.append("#define CM_PIO2_L (%s)" % hexd(mp.pi / 2 - mp.mpf(p2)))
-    # seed of the integer reciprocal (Moller and Granlund 2011, reciprocal_word):
-    # floor((2^19 - 3*2^8) / d9) for the top 9 bits d9 = 256..511 of a normalised divisor
-    lines.append("CM_TABLE_U16(CM_RECIP_V0, 256) = {")
-    for i in range(0, 256, 8):
-        lines.append("  " + " ".join("%d," % ((2 ** 19 - 3 * 2 ** 8) // (256 + k)) for k in range(i, i + 8)))
-    lines.append("};")
+    lines += fixed_tables()
     print("\n".join(lines))
 
 
@@ -220,6 +215,53 @@ def expd_tables():
     out.append("#define CM_EXPD_INVLN2N (%s)" % hexd(256 / mp.log(2)))
     for n in range(2, 6):
         out.append("#define CM_EXPD_C%d (%s)" % (n, hexd(1 / mp.factorial(n))))
+    return out
+
+
+def fixed_tables():
+    """Fixed-point tables of the integer pow and log10 (clm_math.h).  Interval i of the
+    significand z in [1, 2), z in [1 + i/256, 1 + (i+1)/256): C_i of 11 bits with
+    z*C_i/2^11 >= 1 over the interval, nearest such; -log2(C_i/2^11) to 96 fractional
+    bits; 2^(j/256) to 63; the series of log2(1+r) = r (c1 - r (c2 - ...)) and
+    2^t = 1 + t (d1 + t (d2 + ...))."""
+    out = []
+    cs, worst = [], Fraction(0)
+    for i in range(256):
+        lo = 1 + Fraction(i, 256)
+        c = -(-2 ** 11 * lo.denominator // lo.numerator)      # ceil(2^11 / lo)
+        if i == 0:
+            c = 2 ** 11
+        cs.append(c)
+        assert lo * c >= 2 ** 11
+        worst = max(worst, (lo + Fraction(1, 256)) * c / 2 ** 11 - 1)
+    assert worst < Fraction(1, 128), float(worst)
+    logs = [-mp.log(mp.mpf(c) / 2 ** 11, 2) for c in cs]
+    hl = [int(mp.nint(v * mp.mpf(2) ** 96)) for v in logs]
+    assert all(0 <= v < 2 ** 96 for v in hl)
+    out.append("// max r over the significand intervals: %.6g" % float(worst))
+    for name, typ, vals, fmt, per in (("CM_FX_C", "uint16_t", cs, "%d", 8),
+                                      ("CM_FX_LHI", "uint64_t", [v >> 32 for v in hl], "0x%xULL", 2),
+                                      ("CM_FX_LLO", "uint32_t", [v & 0xffffffff for v in hl], "0x%xU", 4),
+                                      ("CM_FX_E", "uint64_t",
+                                       [int(mp.nint(mp.mpf(2) ** (63 + mp.mpf(j) / 256))) for j in range(256)],
+                                       "0x%xULL", 2)):
+        out.append("CM_TABLE_OF(%s, %s, 256) = {" % (typ, name))
+        for i in range(0, 256, per):
+            out.append("  " + " ".join((fmt % v) + "," for v in vals[i:i + per]))
+        out.append("};")
+    ln2 = mp.log(2)
+    out.append("#define CM_FX_C1 0x%xULL" % int(mp.nint(mp.mpf(2) ** 64 * (1 / ln2 - 1))))   # Q64 of c1 - 1
+    for k in range(2, 6):                                                                 # Q64
+        out.append("#define CM_FX_C%d 0x%xULL" % (k, int(mp.nint(mp.mpf(2) ** 64 / (k * ln2)))))
+    for k in range(6, 10):                                                                # Q32
+        out.append("#define CM_FX_C%d 0x%xU" % (k, int(mp.nint(mp.mpf(2) ** 32 / (k * ln2)))))
+    for k in range(1, 4):                                                                 # Q64
+        out.append("#define CM_FX_D%d 0x%xULL" % (k, int(mp.nint(mp.mpf(2) ** 64 * ln2 ** k / mp.factorial(k)))))
+    for k in range(4, 7):                                                                 # Q38
+        out.append("#define CM_FX_D%d 0x%xU" % (k, int(mp.nint(mp.mpf(2) ** 38 * ln2 ** k / mp.factorial(k)))))
+    l102 = int(mp.nint(mp.log(2, 10) * mp.mpf(2) ** 96))
+    out.append("#define CM_FX_LOG10_2_HI 0x%xULL" % (l102 >> 32))
+    out.append("#define CM_FX_LOG10_2_LO 0x%xU" % (l102 & 0xffffffff))
     return out
 
 

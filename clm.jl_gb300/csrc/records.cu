@@ -133,8 +133,6 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
   }
   // ---- the record values of this thread's (level, column) pairs, in registers ----
   double v[RC_PER_THREAD][RC_OUT];
-  double ln10_lo;
-  const double ln10 = cm_log_dd(10.0, &ln10_lo);
 #pragma unroll
   for (int e = 0; e < RC_PER_THREAD; e++) {
     const int idx = tid + e * RC_THREADS;
@@ -149,7 +147,7 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
     const int nlayers = (int)nl;
     // mf_impedance (soil_water_movement.jl:1287-1293)
     const double icef = (j == nlayers) ? TL(RI_ICEF, j, cl) : 0.5 * (TL(RI_ICEF, j, cl) + TL(RI_ICEF, j + 1, cl));
-    const double imp = cm_pow_lx(10.0, ln10, ln10_lo, -e_ice * icef);
+    const double imp = cm_pow(10.0, -e_ice * icef);
     imp_cache[(int64_t)(j - 1) * ld_imp + c] = imp;
     v[e][PC_DZW] = TL(RI_DZ, j, cl) * DENH2O;
     v[e][PC_WS] = TL(RI_WS, j, cl);
