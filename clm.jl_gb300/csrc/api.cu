@@ -75,19 +75,13 @@ static const uint32_t HANDLE_MAGIC = 0xC1A9B300u;
 // 262,144 columns: 1 -> 6.8, 2 -> 7.9, 3 -> 7.5, 4 -> 7.2, occupancy limit -> 5.2
 // M column-steps/s.
 static const int64_t CLMGB_DEFAULT_QUEUE_BLOCKS_PER_SM = 2;
-// Lanes of the work-queue kernel that batch the hydraulic block (CLMGB_OPT_QUEUE_FRESH_BATCH).
-// Measured on GB300 at 262,144 columns (2 blocks/SM), Richards ms per call with the
-// packed refresh: 1 -> 12.73, 2 -> 12.73, 4 -> 12.71, 8 -> 12.77, 12 -> 12.84, 20 -> 13.00
-// (the per-lane refresh: 14.82 at 20, its best; 0 -> 10.16, 8 -> 10.36, 16 -> 10.47,
-// 20 -> 10.54, 24 -> 10.51 M column-steps/s when it was the default).
+// Lanes of the per-lane work-queue kernel that batch the hydraulic block
+// (CLMGB_OPT_QUEUE_FRESH_BATCH); 4 measured best with deferral.
 static const int64_t CLMGB_DEFAULT_FRESH_BATCH = 4;
-// Attempts after which the work-queue kernel hands a column to the warp-per-column
-// finish (CLMGB_OPT_QUEUE_DEFER).  Measured on GB300 over the 100 timed steps of the
-// scale workload (262,144 columns), ms per step with the packed refresh: 12 -> 29.3,
-// 16 -> 19.9, 18 -> 18.6, 20 -> 17.37, 22 -> 17.23, 24 -> 17.56, 28 -> 18.93,
-// 32 -> 20.5.  (Over steps 3-12 alone 28 was best: the later steps hold more long
-// columns.)  Below ~20 the deferred backlog, finished at a few times the cost per
-// attempt, outweighs the shorter end of the queue.
+// Attempts after which the per-lane work-queue kernel hands a column to the
+// warp-per-column finish (CLMGB_OPT_QUEUE_DEFER).  Below ~20 the deferred backlog,
+// finished at a few times the cost per attempt, outweighs the shorter end of the queue;
+// above ~24 the longest columns hold the end.
 static const int64_t CLMGB_DEFAULT_QUEUE_DEFER = 22;
 
 using clmgb::Dims;

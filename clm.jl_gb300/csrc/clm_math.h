@@ -95,8 +95,8 @@ static inline double cm_as_f64_(uint64_t u) { double x; memcpy(&x, &u, 8); retur
 // the rounding of the single-precision reciprocal.  Zero, subnormal, infinite or NaN
 // operands, and quotients below the normal range or within a binade of overflow, take
 // the ordinary division (CM_DIV), so the result always equals it.  Called out of line, a
-// dependent chain on GB300 measures 408 cycles a division at one warp per sub-partition
-// and 155 issue cycles with four (275 and 112 inlined); the 64-bit reciprocal and 2/1
+// dependent chain on GB300 measures 359 cycles a division at one warp per sub-partition
+// and 147 issue cycles with four (225 and 110 inlined); the 64-bit reciprocal and 2/1
 // division it replaced measured 857 and 345, the hardware division 569 and 549.
 CM_FN uint64_t cm_umulhi_(uint64_t a, uint64_t b) {
 #if defined(__CUDACC__)
@@ -138,7 +138,9 @@ CM_FN uint32_t cm_div_seed_(uint64_t my) {
 #endif
 }
 
-CM_FN double cm_div(double x, double y) {
+// x / y without a branch, so that independent quotients overlap; *ok is false for the
+// operands and quotients named above (the value is then meaningless).
+CM_FN double cm_div_fx(double x, double y, bool* ok) {
   const uint64_t bx = CM_AS_U64(x), by = CM_AS_U64(y);
   const uint32_t ex = (uint32_t)(bx >> 52) & 0x7ff, ey = (uint32_t)(by >> 52) & 0x7ff;
   const uint64_t frac = 0x000fffffffffffffULL, hidden = 0x0010000000000000ULL;
@@ -146,7 +148,7 @@ CM_FN double cm_div(double x, double y) {
   const uint32_t lt = mx < my;
   const uint32_t e = ex - ey + 1023u - lt;                  // the quotient's exponent field
   // zero, subnormal, infinite or NaN operands; a quotient not safely normal
-  if (ex - 1u >= 0x7feu || ey - 1u >= 0x7feu || e - 1u >= 0x7fdu) return CM_DIV(x, y);
+  *ok = (ex - 1u < 0x7feu) & (ey - 1u < 0x7feu) & (e - 1u < 0x7fdu);
   const uint64_t X = mx << lt;
   const uint32_t R = cm_div_seed_(my);
   const uint32_t d1 = cm_umulhi32_((uint32_t)(X >> 22), R) >> 6;
@@ -160,6 +162,19 @@ CM_FN double cm_div(double x, double y) {
   // m is in [2^52, 2^53]: its hidden bit, or the carry of a round up to 2, adds to the
   // exponent field
   return CM_AS_F64(((bx ^ by) & 0x8000000000000000ULL) + ((uint64_t)(e - 1) << 52) + m);
+}
+
+#if defined(__CUDACC__)
+// out of line, so that the compiler does not run it beside every quotient
+static __device__ __noinline__ double cm_div_ieee_(double x, double y) { return CM_DIV(x, y); }
+#else
+CM_FN double cm_div_ieee_(double x, double y) { return CM_DIV(x, y); }
+#endif
+CM_FN double cm_div(double x, double y) {
+  bool ok;
+  const double q = cm_div_fx(x, y, &ok);
+  if (ok) return q;
+  return cm_div_ieee_(x, y);
 }
 
 // Natural logarithm.
@@ -413,7 +428,7 @@ CM_FN double cm_log10_dd(double x) {
 // rounding test: A. Ziv, "Fast evaluation of elementary mathematical functions with
 // correctly rounded last bit", ACM TOMS 17(3), 1991).  Measured on GB300, a chain of
 // cm_pow with 32 different lanes, cycles a call at one warp per sub-partition / issue
-// cycles with four: 3,050 / 3,140 in FP64, 1,600 / 800 so (the FP64 fallback of one lane
+// cycles with four: 3,050 / 3,140 in FP64, 1,400 / 770 so (the FP64 fallback of one lane
 // in some 5 calls of a warp included); cm_log10 2,170 / 2,340 and 890 / 370.
 //
 // log2(x) = k + log2(2^11 / C_i) + log2(1 + r), 1 + r = z C_i / 2^11 formed exactly (C_i
@@ -470,15 +485,15 @@ CM_FN int cm_top_bit_(uint64_t v) {
 #endif
 }
 
-// x^y in fixed point; false when the rounding test does not decide, or x and y are not
-// x positive and normal within 2^-60..2^60, y not an integer and 2^-40 <= |y| < 64, or
-// the result is not safely normal.
+// x^y in fixed point, without a branch; false when the rounding test does not decide, or
+// unless x is positive, normal and within 2^-60..2^60 and not 1, y not an integer and
+// 2^-40 <= |y| < 64, and the result safely normal.
 CM_FN bool cm_pow_fx(double x, double y, double* out) {
   const uint64_t ux = CM_AS_U64(x), uy = CM_AS_U64(y);
   const uint32_t ey = (uint32_t)(uy >> 52) & 0x7ff;
   const uint64_t my = (uy << 11) | 0x8000000000000000ULL;
-  const bool whole = ey >= 1023 && ((my << 1) << (ey - 1023)) == 0;
-  if (ux - (963ULL << 52) >= (120ULL << 52) || ux == 0x3ff0000000000000ULL || ey - 983u >= 46u || whole) return false;
+  const bool whole = (ey >= 1023) & (((my << 1) << ((ey - 1023) & 63)) == 0);
+  bool ok = (ux - (963ULL << 52) < (120ULL << 52)) & (ux != 0x3ff0000000000000ULL) & (ey - 983u < 46u) & !whole;
   uint64_t h, l;
   const uint32_t neg = cm_log2_fx_(ux, &h, &l) ^ (uint32_t)(uy >> 63);
   const uint64_t mh = (h << 26) | (l >> 38);                 // |log2 x| Q58, below 2^6
@@ -488,19 +503,13 @@ CM_FN bool cm_pow_fx(double x, double y, double* out) {
   pl += pe;
   ph += pl < pe;                                             // |y log2 x| = ph:pl 2^(ey - 1023 - 121)
   const uint32_t sh = 1080u - ey;                            // 52..97
-  uint64_t n, f;                                             // integer part, fraction Q64
-  if (sh < 64) {
-    n = ph >> sh;
-    f = (ph << (64 - sh)) | (pl >> sh);
-  } else {
-    n = 0;
-    f = sh == 64 ? ph : ph >> (sh - 64);
-  }
-  if (neg) {
-    n = ~n + (f == 0);
-    f = 0 - f;
-  }
-  if (n + 1000 >= 2000) return false;
+  pl = sh >= 64 ? ph : pl;
+  ph = sh >= 64 ? 0 : ph;
+  uint64_t n = ph >> (sh & 63);                              // integer part
+  uint64_t f = ((ph << 1) << (63 - (sh & 63))) | (pl >> (sh & 63));   // fraction, Q64
+  n = neg ? ~n + (f == 0) : n;
+  f = neg ? 0 - f : f;
+  ok &= n + 1000 < 2000;
   const int j = (int)(f >> 56);
   const uint64_t u = f << 8;                                 // t 2^8, Q64
   const uint32_t uh = (uint32_t)(u >> 32);
@@ -524,10 +533,9 @@ CM_FN bool cm_pow_fx(double x, double y, double* out) {
   const uint64_t tw = (tm >> 3) * th8 + th8;
   const uint32_t thr = (128u + (((3u << cm_top_bit_(tm)) * th8) >> 3) + (1u << cm_top_bit_(tw))) >> 6;
   const uint32_t rest = (uint32_t)r & 0x7ff;
-  if (rest - (0x400u - thr) <= 2 * thr || (r >> 63) == 0) return false;
   const uint64_t mant = (r >> 11) + (rest >> 10);
   *out = CM_AS_F64(((n + 1022) << 52) + mant);
-  return true;
+  return ok & (rest - (0x400u - thr) > 2 * thr) & ((r >> 63) != 0);
 }
 
 // log10(x) in fixed point; false when the rounding test does not decide, x is not

@@ -91,7 +91,7 @@ __device__ __forceinline__ double jl_min(double x, double y) {
 // GB300 an FP64 instruction holds its sub-partition's FP64 unit for about 65 cycles,
 // and the column kernels are bound by that unit and by the length of their serial
 // chains; cm_div (clm_math.h) forms the correctly rounded quotient of normal operands
-// with integer multiplies instead (155 issue cycles against 549 of the hardware
+// with integer multiplies instead (147 issue cycles against 549 of the hardware
 // division).  A zero x over a finite nonzero y, common in this solve (the ice of
 // unfrozen levels, the excess ice, the phase-change heat of levels that neither melt
 // nor freeze, the band system's zero sub-diagonal), is the zero with the xor of the
@@ -1057,8 +1057,6 @@ __device__ __forceinline__ void water_fractions_col(const Dims& D, const clmgb_s
 // ===========================================================================
 template <class S>
 struct MfLaneT {
-  static constexpr bool kRefreshInline = true;   // mf_attempt runs mf_refresh itself
-  static constexpr bool kDzw = false;            // dzv holds dz (mf_dzw forms 1000*dz)
   int64_t c;
   int nlayers;
   int nsub;
@@ -1078,14 +1076,6 @@ struct MfLaneT {
   S gam[MAXSOI + 1], dwat[MAXSOI + 1];
 };
 typedef MfLaneT<double> MfLane;
-
-// 1000*dz of level j of a lane: the product M_TO_MM*dz, or the lane's own copy of it
-// (LT::kDzw), which has the same bits (DENH2O*dz of the column record)
-template <class LT>
-__device__ __forceinline__ double mf_dzw(const LT& L, int j) {
-  if constexpr (LT::kDzw) return L.dzv[j];
-  else return M_TO_MM * L.dzv[j];
-}
 
 // Substep log record (clmgb_substep_log): the liquid water of levels 1..nlevsoi at
 // the start of an accepted substep, its dtsub, the time done before it.  After a
@@ -1234,9 +1224,7 @@ __device__ __forceinline__ void mf_refresh(MfLaneT<typename ST::S>& L, const Dim
   L.fresh = false;
 }
 
-// one attempt; returns true when the column's substep loop has finished.  LT is
-// MfLaneT or a lane whose refresh is run elsewhere (LT::kRefreshInline false: the
-// caller has refreshed it before the attempt).
+// one attempt; returns true when the column's substep loop has finished
 template <class LT, class ST>
 __device__ __forceinline__ bool mf_attempt(LT& L, const Dims& D, const clmgb_soilwater_fields& f,
                                            const clmgb_swm_config& cfg, double dtime, ST& X) {
@@ -1264,16 +1252,14 @@ __device__ __forceinline__ bool mf_attempt(LT& L, const Dims& D, const clmgb_soi
         if (ev + (ea - eb) > 0 && ev + (ea - eb) < 2047 && ev > 0)
           L.dt_dz[j] = __longlong_as_double(v + shift);
         else
-          L.dt_dz[j] = jl_div(dtsub, mf_dzw(L, j));
+          L.dt_dz[j] = jl_div(dtsub, M_TO_MM * L.dzv[j]);
       }
     } else {
-      for (int j = 1; j <= nlayers; j++) L.dt_dz[j] = jl_div(dtsub, mf_dzw(L, j));
+      for (int j = 1; j <= nlayers; j++) L.dt_dz[j] = jl_div(dtsub, M_TO_MM * L.dzv[j]);
     }
     L.dt_cur = dtsub;
   }
-  if constexpr (LT::kRefreshInline) {
-    if (L.fresh) mf_refresh(L, D, f, cfg, X);
-  }
+  if (L.fresh) mf_refresh(L, D, f, cfg, X);
   // ---- RHS / LHS (:1380-1397) fused into the Thomas forward sweep (:1421-1438) ----
   S bet, dwat_prev;
   {
@@ -1332,7 +1318,7 @@ __device__ __forceinline__ bool mf_attempt(LT& L, const Dims& D, const clmgb_soi
     return false;
   }
   // ---- accept (:1466-1483) ----
-  for (int j = 1; j <= nlayers; j++) L.liq[j] = L.liq[j] + L.dwat[j] * mf_dzw(L, j);
+  for (int j = 1; j <= nlayers; j++) L.liq[j] = L.liq[j] + L.dwat[j] * (M_TO_MM * L.dzv[j]);
   L.fresh = true;
   S qcTemp;
   if (lower_bc == CLMGB_BC_FLUX) qcTemp = L.hk_bot + L.dhkdw_bot * L.dwat[nlayers];

@@ -301,380 +301,6 @@ k_moisture_form_queue(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_co
   }
 }
 
-// ---------------------------------------------------------------------------
-// The work-queue kernel with a packed hydraulic refresh.  A refresh (the hydraulic
-// properties, fluxes and flux derivatives of an accepted substep's water, mf_refresh)
-// costs about three attempts and runs for the lanes whose substep was just accepted;
-// run lane by lane it leaves the warp's other lanes idle.  Here the warp runs the
-// refresh of all its fresh lanes' columns together: the (column, level) pairs are
-// spread over the 32 lanes, in four passes over the levels (saturation, hydraulic
-// properties, fluxes, net flux), each reading what the pass before wrote.  The
-// arrays other lanes read or write live in the warp's shared memory, laid out
-// [array][level][lane]; within a pass every lane reads its inputs, the warp syncs,
-// then the lanes write, so no level is overwritten before its neighbour has read it.
-// Every value is formed by mf_refresh's expression and the attempts are mf_attempt,
-// so the results are the per-lane kernel's bits.
-
-// level j (1-based) of one lane's array in the warp's shared memory
-struct LevelView {
-  double* p;
-  __device__ __forceinline__ double& operator[](int j) const { return p[(j - 1) * 32]; }
-};
-
-struct MfLaneP {
-  static constexpr bool kRefreshInline = false;   // refreshed by mfp_refresh
-  static constexpr bool kDzw = true;              // dzv holds 1000*dz (the record's PC_DZW)
-  int64_t c;
-  int nlayers;
-  int nsub;
-  bool fresh;
-  uint32_t status;
-  double dtsub, dtdone, dt_cur;
-  double qc, qin1, hk_bot, dhkdw_bot;
-  double dzv[MAXSOI + 1], dt_dz[MAXSOI + 1];
-  double liq[MAXSOI + 1], gam[MAXSOI + 1], dwat[MAXSOI + 1];
-  LevelView qout, dqodw1, dqodw2, fnet1;
-};
-
-// mf_end's destination in the packed kernel: the column's water goes to its record
-// (the post-pass k_column_outputs moves it to the state), qcharge to the state
-struct RecordOut {
-  double* rec;
-  int joff, nls;
-  double* qc;
-  __device__ __forceinline__ double& Liq(int jj) const { return rec[PC_LIQ * nls + (jj - joff) - 1]; }
-  __device__ __forceinline__ double& Qcharge() const { return *qc; }
-};
-
-// shared-memory doubles per warp: 4 level arrays and the bottom conductivity pair
-__host__ __device__ constexpr int64_t packed_warp_doubles(int nlevsoi) { return (4LL * nlevsoi + 2) * 32; }
-// threads per block of k_moisture_form_packed: 5 warps at 21 KB of shared memory each
-// (20 levels) put 2 blocks, 10 warps, on an SM
-constexpr int PBLOCK = 160;
-
-// mf_begin for the packed lane (the impedances stay in the cache the refresh reads;
-// the water and 1000*dz come from the column's record)
-__device__ __forceinline__ bool mfp_begin(MfLaneP& L, const Dims& D, const clmgb_soilwater_fields& f,
-                                          const clmgb_swm_config& cfg, double dtime, int64_t c,
-                                          const double* dt_init, const double* pcache) {
-  const int nls = D.nlevsoi;
-  L.c = c;
-  L.status = 0;
-  const int64_t nl = f.col_nbedrock[c];
-  if (nl < 1 || nl > D.nlevsoi) {
-    L.status = CLMGB_COL_LEVEL_RANGE;
-    return false;
-  }
-  const int nlayers = (int)nl;
-  L.nlayers = nlayers;
-  const double* rec = pcache + c * (int64_t)(PC_ALL * nls);
-  for (int j = 1; j <= nlayers; j++) {
-    L.liq[j] = rec[PC_LIQ * nls + j - 1];
-    L.dzv[j] = rec[PC_DZW * nls + j - 1];
-  }
-  L.nsub = 0;
-  L.dtsub = dtime;
-  if (dt_init) {
-    const double d = dt_init[c];
-    if (d == d) L.dtsub = jl_min(jl_max(d, cfg.dtmin), dtime);   // NaN keeps dtime
-  }
-  L.dtdone = 0.0;
-  L.qc = 0.0;
-  L.fresh = true;
-  L.dt_cur = -1.0;
-  return true;
-}
-
-// The refresh of the lanes in `mask`, called by all 32 lanes of the warp.  wsm: the
-// warp's shared block; nls: D.nlevsoi; pcache: the columns' input records
-// ([column][PC_FIELDS][nls], k_impedance).
-__device__ __forceinline__ void mfp_refresh(MfLaneP& L, unsigned mask, const Dims& D,
-                                            const clmgb_soilwater_fields& f, const clmgb_swm_config& cfg,
-                                            double* pcache, double* wsm, int nls) {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int64_t ld = D.ldc;
-  const int joff = D.nlevsno, joff_zi = D.nlevsno + 1, nlevsoi = D.nlevsoi;
-  const int lower_bc = cfg.lower_boundary_condition;
-  const bool mine = (mask >> lane) & 1u;
-  // (column, level) items: lane k's levels are items off_k .. off_k + nl_k - 1
-  const int nl_own = mine ? L.nlayers : 0;
-  int incl = nl_own;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int off_own = incl - nl_own;
-  const int T = __shfl_sync(FULL, incl, 31);
-  const int64_t c_own = mine ? L.c : 0;
-  double* const sb = wsm + 4LL * nls * 32;                       // hk, dhkdw of the bottom level
-  auto A = [&](int a, int k, int j) -> double& { return wsm[((int64_t)a * nls + (j - 1)) * 32 + k]; };
-  // input `fld` of level j of column c
-  auto P = [&](int64_t c, int fld, int j) -> double {
-    return pcache[c * (int64_t)(PC_ALL * nls) + (int64_t)fld * nls + (j - 1)];
-  };
-  enum { QOUT = 0, D1 = 1, D2 = 2, FN = 3 };
-  struct Item { int k, j, nl; int64_t c; bool ok; };
-  auto item = [&](int base) -> Item {
-    const int t = base + lane;
-    int k = 0;                                     // the last lane whose first item is <= t
-    for (int step = 16; step > 0; step >>= 1) {
-      const int oc = __shfl_sync(FULL, off_own, k + step);
-      if (oc <= t) k += step;
-    }
-    Item it;
-    it.k = k;
-    it.c = __shfl_sync(FULL, c_own, k);
-    it.nl = __shfl_sync(FULL, nl_own, k);
-    it.j = t - __shfl_sync(FULL, off_own, k) + 1;
-    it.ok = t < T;
-    return it;
-  };
-  // the refreshed lanes' water (kept in their local memory) into FN, where the other
-  // lanes of the warp can read it; their net fluxes there are about to be re-formed
-  if (mine)
-    for (int j = 1; j <= L.nlayers; j++) A(FN, lane, j) = L.liq[j];
-  __syncwarp();
-  // pass 1: saturation of every level (:1283-1287), kept in FN
-  for (int base = 0; base < T; base += 32) {
-    const Item it = item(base);
-    if (it.ok) {
-      const double vwc = jl_div(jl_max(A(FN, it.k, it.j), 1.0e-6), P(it.c, PC_DZW, it.j));
-      double s = jl_div(vwc, P(it.c, PC_WS, it.j));
-      s = jl_min(s, 1.0);
-      A(FN, it.k, it.j) = jl_max(0.01, s);
-    }
-  }
-  __syncwarp();
-  // pass 2: hydraulic properties (:1288-1308): hk, dhkdw, smp, dsmpdw into QOUT, D1, D2, FN
-  for (int base = 0; base < T; base += 32) {
-    const Item it = item(base);
-    double hkv = 0.0, dhkds = 0.0, smpv = 0.0, dsmpdw = 0.0;
-    if (it.ok) {
-      const int j = it.j;
-      const int64_t c = it.c;
-      const double sj = A(FN, it.k, j);
-      const double sn = (j < it.nl) ? A(FN, it.k, j + 1) : sj;
-      double s1 = (j == it.nl) ? sj : 0.5 * (sj + sn);
-      s1 = jl_min(s1, 1.0);
-      s1 = jl_max(0.01, s1);
-      const double b = P(c, PC_BSW, j);
-      hkv = P(c, PC_IMP, j) * P(c, PC_KS, j) * cm_pow(s1, 2.0 * b + 3.0);
-      dhkds = jl_div((2.0 * b + 3.0) * hkv, s1);
-      smpv = -P(c, PC_SUC, j) * cm_pow(sj, -b);
-      const double dsmpds = jl_div(-b * smpv, sj);
-      dsmpdw = jl_div(dsmpds, P(c, PC_WS, j));
-      double* rec = pcache + c * (int64_t)(PC_ALL * nls);
-      rec[PC_SMP * nls + j - 1] = smpv;
-      rec[PC_HK * nls + j - 1] = hkv;
-    }
-    __syncwarp();
-    if (it.ok) {
-      A(QOUT, it.k, it.j) = hkv;
-      A(D1, it.k, it.j) = dhkds;
-      A(D2, it.k, it.j) = smpv;
-      A(FN, it.k, it.j) = dsmpdw;
-    }
-    __syncwarp();
-  }
-  // pass 3: fluxes and derivatives between levels (:1310-1345) and at the bottom
-  // (:1347-1370), over the properties into QOUT, D1, D2
-  for (int base = 0; base < T; base += 32) {
-    const Item it = item(base);
-    double qo = 0.0, d1 = 0.0, d2 = 0.0;
-    if (it.ok) {
-      const int j = it.j;
-      const int64_t c = it.c;
-      const double hk = A(QOUT, it.k, j), dhkdw = A(D1, it.k, j), smp = A(D2, it.k, j), dsmpdw = A(FN, it.k, j);
-      if (j < it.nl) {
-        const double dhkds1 = jl_div(0.5 * dhkdw, P(c, PC_WS, j));
-        const double dhkds2 = jl_div(0.5 * dhkdw, P(c, PC_WS, j + 1));
-        const double num = A(D2, it.k, j + 1) - smp;
-        const double den = P(c, PC_DEN, j);
-        qo = jl_div(-hk * num, den) + hk;
-        d1 = jl_div(hk * dsmpdw - dhkds1 * num, den) + dhkds1;
-        d2 = jl_div(-hk * A(FN, it.k, j + 1) - dhkds2 * num, den) + dhkds2;
-      } else {
-        sb[it.k] = hk;
-        sb[32 + it.k] = dhkdw;
-        if (lower_bc == CLMGB_BC_WATERTABLE) {
-          int jwt = nlevsoi;
-          for (int jj = 1; jj <= nlevsoi; jj++) {
-            if (f.zwt[c] <= LVc(f.zi, c, joff_zi + jj, ld)) { jwt = jj - 1; break; }
-          }
-          if (j <= jwt) {
-            const double dhkds1l = dhkdw / P(c, PC_WS, j);
-            const double num = -smp;
-            const double den = M_TO_MM * (f.zwt[c] - LVc(f.z, c, joff + j, ld));
-            qo = jl_div(-hk * num, den) + hk;
-            d1 = (hk * dsmpdw - dhkds1l * num) / den + dhkds1l;
-          }
-        } else if (lower_bc == CLMGB_BC_FLUX) {
-          qo = hk;
-          d1 = dhkdw / P(c, PC_WS, j);
-        }
-      }
-    }
-    __syncwarp();
-    if (it.ok) {
-      A(QOUT, it.k, it.j) = qo;
-      A(D1, it.k, it.j) = d1;
-      A(D2, it.k, it.j) = d2;
-    }
-    __syncwarp();
-  }
-  // pass 4: net flux of every level (:1372-1378); the inflow of level j > 1 is the
-  // outflow of level j-1
-  for (int base = 0; base < T; base += 32) {
-    const Item it = item(base);
-    if (it.ok) {
-      const double qin = (it.j == 1) ? f.qflx_infl[it.c] : A(QOUT, it.k, it.j - 1);
-      A(FN, it.k, it.j) = qin - A(QOUT, it.k, it.j) - P(it.c, PC_ROOT, it.j);
-    }
-  }
-  __syncwarp();
-  if (mine) {
-    L.qin1 = f.qflx_infl[L.c];
-    L.hk_bot = sb[lane];
-    L.dhkdw_bot = sb[32 + lane];
-    L.fresh = false;
-  }
-  __syncwarp();
-}
-
-// k_moisture_form_queue with the packed refresh; reads the column records
-// (QueueScratch::pcache) k_column_records (records.cu) wrote before it.  With
-// LOG it writes the same substep log (the starting water of each accepted substep,
-// its dtsub and the time done before it, then the solve's outputs).  Dynamic shared
-// memory: packed_warp_doubles(nlevsoi) doubles per warp.
-template <bool LOG>
-__global__ void __launch_bounds__(PBLOCK)
-k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_config cfg, double dtime,
-                       uint32_t* col_status, int or_status, uint32_t* dev_status, unsigned long long* queue,
-                       const uint32_t* order, const unsigned int* nlisted_ptr, const double* dt_init,
-                       SubstepLogView lg, int fresh_batch, QueueScratch qs) {
-  extern __shared__ double smem_packed[];
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int nls = D.nlevsoi;
-  double* const wsm = smem_packed + (int64_t)(threadIdx.x >> 5) * packed_warp_doubles(nls);
-  const unsigned long long nq = order ? (unsigned long long)(*(volatile const unsigned int*)nlisted_ptr)
-                                      : (unsigned long long)nc;
-  const int batch = fresh_batch > 0 ? fresh_batch : 1;
-  MfLaneP L;
-  L.qout.p = wsm + (0LL * nls) * 32 + lane;
-  L.dqodw1.p = wsm + (1LL * nls) * 32 + lane;
-  L.dqodw2.p = wsm + (2LL * nls) * 32 + lane;
-  L.fnet1.p = wsm + (3LL * nls) * 32 + lane;
-  int nacc = 0;
-  bool active = false, exhausted = false, kept = false;
-  for (;;) {
-    const bool need = !active && !exhausted;
-    const unsigned m = __ballot_sync(FULL, need);
-    if (m) {
-      const int leader = __ffs(m) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(m));
-      base = __shfl_sync(FULL, base, leader);
-      if (need) {
-        const unsigned long long k = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
-        if (k >= nq) {
-          exhausted = true;
-        } else {
-          const int64_t c = order ? (int64_t)order[k] : (int64_t)k;
-          if (order || f.mask_hydrology[c]) {
-            if (mfp_begin(L, D, f, cfg, dtime, c, dt_init, qs.pcache)) {
-              active = true;
-              nacc = 0;
-              kept = false;
-            } else {
-              const uint32_t st = L.status;
-              if (col_status) col_status[c] = or_status ? (col_status[c] | st) : st;
-              if (st && dev_status) atomicOr(dev_status, st);
-            }
-          } else if (col_status && !or_status) {
-            col_status[c] = 0;
-          }
-        }
-      }
-    }
-    if (!__any_sync(FULL, active)) {
-      if (__all_sync(FULL, exhausted)) {
-        if (!LOG && qs.defer > 0) coop_drain(D, f, cfg, dtime, col_status, or_status, dev_status, qs);
-        break;
-      }
-      continue;
-    }
-    // lanes whose substep was accepted wait for the packed refresh until `batch` of
-    // them need it or no lane can attempt
-    const bool want = active && L.fresh && L.nsub < D.attempt_cap;
-    const unsigned wm = __ballot_sync(FULL, want);
-    const unsigned tm = __ballot_sync(FULL, active && !want);
-    if (wm && (__popc(wm) >= batch || tm == 0)) {
-      if (LOG && want && nacc < lg.cap) {
-        double* r0 = lg.rec + L.c * lg.stride + (int64_t)nacc * SUB_REC;
-        for (int j = 1; j <= L.nlayers; j++) r0[j - 1] = L.liq[j];
-      }
-      if (qs.work) {
-        const unsigned lv = __reduce_add_sync(FULL, want ? (unsigned)L.nlayers : 0u);
-        if (lane == 0) atomicAdd(qs.work + 1, (unsigned long long)lv);
-      }
-      mfp_refresh(L, wm, D, f, cfg, qs.pcache, wsm, nls);
-    }
-    const bool can_try = active && !(L.fresh && L.nsub < D.attempt_cap);
-    if (qs.work) {
-      const unsigned lv = __reduce_add_sync(FULL, can_try ? (unsigned)L.nlayers : 0u);
-      if (lane == 0) atomicAdd(qs.work, (unsigned long long)lv);
-    }
-    if (!can_try) continue;
-    double* rec = nullptr;
-    double dts = 0.0, dtd = 0.0;
-    if (LOG) {
-      rec = lg.rec + L.c * lg.stride;
-      if (L.fresh && nacc < lg.cap)
-        for (int j = 1; j <= L.nlayers; j++) rec[(int64_t)nacc * SUB_REC + j - 1] = L.liq[j];
-      dts = L.dtsub;
-      dtd = L.dtdone;
-    }
-    FieldState<clmgb_soilwater_fields> X(f, L.c, D.ldc);
-    const bool fin = mf_attempt(L, D, f, cfg, dtime, X);
-    if (LOG && L.dtdone != dtd) {
-      if (nacc < lg.cap) {
-        rec[(int64_t)nacc * SUB_REC + MAXSOI] = dts;
-        rec[(int64_t)nacc * SUB_REC + MAXSOI + 1] = dtd;
-      }
-      nacc++;
-    }
-    if (!LOG && !fin && qs.defer > 0 && L.fresh && L.nsub >= qs.defer && !kept) {
-      // hand the column over; a slot the drain gave back leaves it with this lane
-      if (coop_defer(L, qs)) {
-        active = false;
-        continue;
-      }
-      kept = true;
-    }
-    if (fin) {
-      RecordOut RO{qs.pcache + L.c * (int64_t)(PC_ALL * nls), D.nlevsno, nls, f.qcharge + L.c};
-      const uint32_t st = mf_end(L, D, f, RO);
-      if (LOG) {
-        double* out = rec + (int64_t)lg.cap * SUB_REC;
-        for (int j = 1; j <= L.nlayers; j++) {
-          out[j - 1] = L.liq[j];
-          out[MAXSOI + j - 1] = RO.rec[PC_SMP * nls + j - 1];
-          out[2 * MAXSOI + j - 1] = RO.rec[PC_HK * nls + j - 1];
-        }
-        out[3 * MAXSOI] = L.qc;
-        out[3 * MAXSOI + 1] = (double)L.nsub;
-        out[3 * MAXSOI + 2] = (double)st;
-        lg.count[L.c] = nacc;
-      }
-      if (col_status) col_status[L.c] = or_status ? (col_status[L.c] | st) : st;
-      if (st && dev_status) atomicOr(dev_status, st);
-      active = false;
-    }
-  }
-}
-
 // compute_qcharge! after a moisture-form solve with the water-table lower boundary
 // (soil_water_movement.jl:1575-1598): one thread per hydrology column the solve
 // could take (nbedrock in range).
@@ -1033,8 +659,11 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
   if (e != cudaSuccess) return e;
   if (log && (e = cudaMemsetAsync(log->count, 0xff, (size_t)nc * sizeof(int32_t), s)) != cudaSuccess) return e;
   const bool use = qs.capacity >= nc && qs.order && qs.bins && qs.imp;
+  // the packed kernel hands no column over; the options that test the hand-over's bounded
+  // wait (polls of a list slot, a late index) select the per-lane kernel, which does
+  const bool packed = use && qs.packed && qs.pcache && qs.poll_limit == DEFER_POLL_LIMIT && qs.publish_delay == 0;
   if (use) {
-    if (qs.packed && qs.pcache) {
+    if (packed) {
       if ((e = launch_column_records(D, nc, f, cfg.e_ice, qs.imp, qs.capacity, qs.pcache, qs.records_tma != 0,
                                      dev_status, s, qs.records_tma_used)) != cudaSuccess)
         return e;
@@ -1059,29 +688,15 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
   const double* imp = use ? qs.imp : nullptr;
   const int64_t ldi = use ? qs.capacity : 0;
   QueueScratch q = qs;
-  if (!use || log || !q.d_count) q.defer = 0;              // deferral needs the reserved scratch
+  if (!use || packed || log || !q.d_count) q.defer = 0;    // deferral needs the reserved scratch
   if (q.defer > 0) {                                       // empty list, zero claim/publish/consume counts
     if ((e = cudaMemsetAsync(q.d_count, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(q.d_list, 0xff, (size_t)nc * sizeof(uint32_t), s)) != cudaSuccess) return e;
   }
-  if (use && qs.packed && qs.pcache) {
-    const size_t smem = (size_t)(PBLOCK / 32) * (size_t)packed_warp_doubles(D.nlevsoi) * sizeof(double);
-    auto kern = log ? k_moisture_form_packed<true> : k_moisture_form_packed<false>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+  if (packed) {
+    if ((e = launch_moisture_form_packed(D, nc, f, cfg, dtime, col_status, or_status, dev_status, queue, ord, nl,
+                                         dt_init, log, grid_blocks, q, s)) != cudaSuccess)
       return e;
-    // the blocks that fit on the GPU at once (the kernel's warps wait on one another
-    // only through the bounded waits of the deferred-column list)
-    int dev = 0, nsm = 0, nb = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, PBLOCK, smem)) != cudaSuccess) return e;
-    if (nb < 1) return cudaErrorInvalidConfiguration;
-    int gp = grid > 0 ? grid : 1;
-    if (gp > nb * nsm) gp = nb * nsm;
-    q.out_records = 1;
-    kern<<<gp, PBLOCK, smem, s>>>(D, nc, f, cfg, dtime, col_status, or_status, dev_status, queue, ord, nl, dt_init,
-                                 log ? *log : SubstepLogView{nullptr, nullptr, 0, 0}, qs.fresh_batch, q);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the solved columns' water, smp_l and hk_l from their records to the state
     if ((e = launch_column_outputs(D, nc, f, qs.pcache, s)) != cudaSuccess) return e;
   } else if (log)

@@ -19,19 +19,17 @@ struct QueueScratch {
   unsigned int* bins;
   int longest_first;
   int fresh_batch;   // CLMGB_OPT_QUEUE_FRESH_BATCH (0: refresh at once)
-  // CLMGB_OPT_QUEUE_PACKED_REFRESH: the warp refreshes its fresh lanes' columns
-  // together, (column, level) pairs spread over the 32 lanes (k_moisture_form_packed)
+  // CLMGB_OPT_QUEUE_PACKED_REFRESH: the solve runs over (column, level) items of a
+  // warp's columns (k_moisture_form_packed, richards_packed.cu)
   int packed;
   // one record per column, contiguous: [capacity][PC_ALL][nlevsoi] (PcField): the
   // packed refresh's inputs (the pre-pass k_column_records fills them), so that a pass
   // over one column's levels reads consecutive addresses and the resident columns'
-  // inputs stay in L2, and the column's water, smp_l and hk_l during the solve
+  // inputs stay in L2, and the column's water, smp_l and hk_l during the solve (the
+  // post-pass k_column_outputs writes them to the state at its end)
   double* pcache;
-  // 1 while the solve keeps a column's water, smp_l and hk_l in its record (the packed
-  // kernel); the post-pass k_column_outputs writes them to the state at the end
-  int out_records = 0;
-  // CLMGB_OPT_QUEUE_DEFER: a column still unfinished after `defer` attempts leaves the
-  // work queue at its next accepted substep; its state (water [nlevsoi][capacity],
+  // CLMGB_OPT_QUEUE_DEFER (the per-lane kernel): a column still unfinished after `defer`
+  // attempts leaves the work queue at its next accepted substep; its state (water [nlevsoi][capacity],
   // dtsub, dtdone, qcharge so far, attempts, status at index c) and its index (list)
   // are kept for the warp-per-column finish (richards_coop.cuh).  d_count: the
   // claimed, published and consumed list slots.  0: off.
@@ -47,9 +45,8 @@ struct QueueScratch {
   // production: it lets a test make that wait run out)
   int poll_limit = DEFER_POLL_LIMIT;
   int publish_delay = 0;
-  // CLMGB_OPT_COUNT_WORK: when set, the packed kernel and the warp-per-column finish add
-  // the levels of every substep attempt to work[0] and of every hydraulic refresh to
-  // work[1] (the FP64 work model of the solve, clmgb/flops_model.py); NULL otherwise
+  // CLMGB_OPT_COUNT_WORK: when set, the packed kernel adds the levels of every substep
+  // attempt to work[0] and of every hydraulic refresh to work[1] (the FP64 work model of the solve, clmgb/flops_model.py); NULL otherwise
   unsigned long long* work = nullptr;
   // CLMGB_OPT_RECORDS_TMA: the column-record pre-pass stages its tiles with tensor copies
   int records_tma = 1;
@@ -165,6 +162,13 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
                                        int or_status, uint32_t* dev_status, unsigned long long* queue,
                                        int grid_blocks, const QueueScratch& qs, cudaStream_t s,
                                        const double* dt_init = nullptr, const SubstepLogView* log = nullptr);
+// The packed work-queue solve (richards_packed.cu) over columns whose records are written,
+// at most max_blocks blocks; leaves its water, smp_l and hk_l in the records.
+cudaError_t launch_moisture_form_packed(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,
+                                        const clmgb_swm_config& cfg, double dtime, uint32_t* col_status, int or_status,
+                                        uint32_t* dev_status, unsigned long long* queue, const uint32_t* order,
+                                        const unsigned int* nlisted, const double* dt_init, const SubstepLogView* log,
+                                        int max_blocks, const QueueScratch& qs, cudaStream_t s);
 // compute_qcharge! over the solved state when cfg's lower boundary is the water table
 // (a no-op otherwise); every moisture-form entry point runs it after its solve.
 cudaError_t launch_compute_qcharge(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,

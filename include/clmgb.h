@@ -700,34 +700,37 @@ int32_t clmgb_last_cuda_error(clmgb_handle h);
 #define   CLMGB_ADJ_ST_CLOSED_FORM       0 /*   hand-written reverse of every stage, no tape (default;
                                                  used when CLMGB_OPT_ADJ_RICHARDS is closed form too) */
 #define   CLMGB_ADJ_ST_RECORDED          1 /*   replayed through the recording scalar and swept */
-#define CLMGB_OPT_QUEUE_FRESH_BATCH   14 /* work-queue Richards kernel: lanes whose substep was accepted wait
+#define CLMGB_OPT_QUEUE_FRESH_BATCH   14 /* per-lane work-queue Richards kernel: lanes whose substep was accepted wait
                                             for the hydraulic block until this many lanes of the warp need it
                                             (or no lane can attempt), then run it together (default 4); 0 = at
                                             once.  Results do not depend on it. */
-#define CLMGB_OPT_QUEUE_DEFER         16 /* work-queue Richards kernel with reserved scratch: a column not done
+#define CLMGB_OPT_QUEUE_DEFER         16 /* per-lane work-queue Richards kernel with reserved scratch (the
+                                            packed one hands no column over): a column not done
                                             after this many attempts (default 22) leaves the queue at its next
                                             accepted substep and is finished by one warp (one level per lane);
                                             0 = off.  Results do not depend on it. */
 #define CLMGB_OPT_QUEUE_PACKED_REFRESH 17 /* work-queue Richards kernel with reserved scratch: 1 (default) = the
-                                            warp runs the hydraulic refresh of its waiting lanes' columns
-                                            together, column levels spread over the 32 lanes; 0 = each lane
-                                            runs its own.  Results do not depend on it. */
+                                            packed kernel, a warp's columns spread over its lanes by
+                                            (column, level); 0 = the per-lane kernel, a column per lane.
+                                            Results do not depend on it. */
 #define CLMGB_OPT_ATTEMPT_CAP         18 /* Richards substep attempts after which a column stops with
                                             CLMGB_COL_SUBSTEP_CAP (1..4096, default 4096: never reached by a
                                             valid configuration, whose attempts dtmin bounds) */
 #define CLMGB_OPT_QUEUE_POLL_LIMIT    19 /* polls of a deferred column's list slot before the finishing warp
                                             gives the slot back to the deferring lane (0..2^20, default
-                                            2^20).  Results do not depend on it. */
+                                            2^20; any other value selects the per-lane kernel).
+                                            Results do not depend on it. */
 #define CLMGB_OPT_QUEUE_PUBLISH_DELAY 20 /* for tests of the bounded wait: a deferring lane counts an even
                                             list slot published before writing the column's index, and
                                             writes it once a finishing warp has taken the slot or after
                                             this many ns; a warp with nothing to finish keeps looking for
-                                            as long (0..1e7, default 0: index first, no lingering).  Results
-                                            do not depend on it. */
-#define CLMGB_OPT_COUNT_WORK          21 /* 1: the work-queue Richards kernel with reserved scratch (packed
-                                            refresh) and its warp-per-column finish count, over the calls that
-                                            follow, the levels of every substep attempt and of every hydraulic
-                                            refresh (setting 1 zeroes the counts; 0 = off, the default) */
+                                            as long (0..1e7, default 0: index first, no lingering; any
+                                            other value selects the per-lane kernel).  Results do not
+                                            depend on it. */
+#define CLMGB_OPT_COUNT_WORK          21 /* 1: the work-queue Richards kernel with reserved scratch (the packed
+                                            kernel) counts, over the calls that follow, the levels of every
+                                            substep attempt and of every hydraulic refresh (setting 1 zeroes
+                                            the counts; 0 = off, the default) */
 #define CLMGB_OPT_WORK_LEVEL_ATTEMPTS 22 /* read-only (synchronises): that count of attempt levels */
 #define CLMGB_OPT_WORK_LEVEL_REFRESHES 23 /* read-only (synchronises): that count of refreshed levels */
 #define CLMGB_OPT_RECORDS_TMA         24 /* the Richards pre-pass stages each tile of 32 columns with 2-D
