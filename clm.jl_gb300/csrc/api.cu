@@ -64,7 +64,7 @@ struct clmgb_handle_s {
   int64_t records_tma;          // CLMGB_OPT_RECORDS_TMA
   int records_tma_used;         // CLMGB_OPT_RECORDS_TMA_USED
   int64_t tridiag_method;       // CLMGB_OPT_TRIDIAG_METHOD
-  int64_t st_block;             // CLMGB_OPT_ST_BLOCK
+  int64_t st_block;             // CLMGB_OPT_ST_BLOCK (kept and read back, selects nothing)
   cudaError_t last_error;
 };
 
@@ -126,9 +126,7 @@ static Dims make_dims(const clmgb_varpar& vp, const clmgb_bounds& b, int64_t c0 
 }
 
 static Dims hdims(clmgb_handle h, const clmgb_bounds& b) {
-  Dims D = make_dims(h->vp, b, h->column_base, (int)h->attempt_cap);
-  D.st_block = (int)h->st_block;
-  return D;
+  return make_dims(h->vp, b, h->column_base, (int)h->attempt_cap);
 }
 
 // every pointer member after struct_size must be non-NULL

@@ -486,14 +486,15 @@ CM_FN int cm_top_bit_(uint64_t v) {
 }
 
 // x^y in fixed point, without a branch; false when the rounding test does not decide, or
-// unless x is positive, normal and within 2^-60..2^60 and not 1, y not an integer and
+// unless x is 1, or x is positive, normal and within 2^-60..2^60, y not an integer and
 // 2^-40 <= |y| < 64, and the result safely normal.
 CM_FN bool cm_pow_fx(double x, double y, double* out) {
   const uint64_t ux = CM_AS_U64(x), uy = CM_AS_U64(y);
   const uint32_t ey = (uint32_t)(uy >> 52) & 0x7ff;
   const uint64_t my = (uy << 11) | 0x8000000000000000ULL;
   const bool whole = (ey >= 1023) & (((my << 1) << ((ey - 1023) & 63)) == 0);
-  bool ok = (ux - (963ULL << 52) < (120ULL << 52)) & (ux != 0x3ff0000000000000ULL) & (ey - 983u < 46u) & !whole;
+  const bool one = ux == 0x3ff0000000000000ULL;
+  bool ok = (ux - (963ULL << 52) < (120ULL << 52)) & (ey - 983u < 46u) & !whole;
   uint64_t h, l;
   const uint32_t neg = cm_log2_fx_(ux, &h, &l) ^ (uint32_t)(uy >> 63);
   const uint64_t mh = (h << 26) | (l >> 38);                 // |log2 x| Q58, below 2^6
@@ -534,8 +535,8 @@ CM_FN bool cm_pow_fx(double x, double y, double* out) {
   const uint32_t thr = (128u + (((3u << cm_top_bit_(tm)) * th8) >> 3) + (1u << cm_top_bit_(tw))) >> 6;
   const uint32_t rest = (uint32_t)r & 0x7ff;
   const uint64_t mant = (r >> 11) + (rest >> 10);
-  *out = CM_AS_F64(((n + 1022) << 52) + mant);
-  return ok & (rest - (0x400u - thr) > 2 * thr) & ((r >> 63) != 0);
+  *out = CM_AS_F64(one ? ux : ((n + 1022) << 52) + mant);    // x == 1: 1 for every y
+  return one | (ok & (rest - (0x400u - thr) > 2 * thr) & ((r >> 63) != 0));
 }
 
 // log10(x) in fixed point; false when the rounding test does not decide, x is not

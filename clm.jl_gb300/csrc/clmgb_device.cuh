@@ -55,7 +55,6 @@ struct Dims {
   int64_t ldc, ldp, np;
   int64_t c0 = 0;    // global index of the call's first column (patch_column holds global indices)
   int attempt_cap = MF_ATTEMPT_CAP;   // Richards attempts after which a column stops (CLMGB_COL_SUBSTEP_CAP)
-  int st_block = 320;                 // threads per block of the soil-temperature kernels (CLMGB_OPT_ST_BLOCK)
 };
 
 // Julia Base.max / Base.min on Float64 (NaN propagates, -0.0 < 0.0).  They only
@@ -98,16 +97,15 @@ __device__ __forceinline__ double jl_min(double x, double y) {
 // signs, from the bits.  Every other case (subnormal, infinite or NaN operands,
 // quotients outside the normal range) is the hardware division.  The result is always
 // the IEEE quotient.
-// (one out-of-line copy: a copy inlined at every call site of the soil-temperature
-// kernel measured slower)
-static __device__ __noinline__ double cm_div_call(double x, double y) { return cm_div(x, y); }
-__device__ __forceinline__ double jl_div(double x, double y) {
+// (one out-of-line copy, the zero test in it: the column kernels' code runs at the size
+// of the instruction cache, and copies inlined at the call sites measured slower)
+static __device__ __noinline__ double jl_div(double x, double y) {
   const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
   const unsigned long long by = (unsigned long long)__double_as_longlong(y);
   // (by << 1) - 1 < 0xffdffffffffffffe: y is nonzero and finite
   if ((bx << 1) == 0 && (by << 1) - 1ull < 0xffdffffffffffffeull)
     return __longlong_as_double((long long)((bx ^ by) & 0x8000000000000000ull));
-  return cm_div_call(x, y);
+  return cm_div(x, y);
 }
 // other scalar types (the recording adjoint's): their own division
 template <class A, class B>
@@ -1017,21 +1015,27 @@ __device__ inline uint32_t soil_temperature_col(const Dims& D, const clmgb_soilt
 // set_soil_water_fractions! kernel (soil_hydrology.jl:110-130), column c.
 // ===========================================================================
 template <class ST>
-__device__ __forceinline__ void water_fractions_col(const Dims& D, const clmgb_soilwater_fields& f, int64_t c,
-                                                    ST& X) {
+__device__ __forceinline__ void water_fractions_level(const Dims& D, const clmgb_soilwater_fields& f, int64_t c, int j,
+                                                      ST& X) {
   typedef typename ST::S S;
   const int64_t ld = D.ldc;
   const int joff = D.nlevsno;
-  for (int j = 1; j <= D.nlevsoi; j++) {
-    const double exi = LV(f.excess_ice, c, j, ld);
-    const double dz_ext = LVc(f.dz, c, j + joff, ld) + jl_div(exi, DENICE);
-    const S ws = X.Watsat(j);
-    const S vol_ice = jl_min(ws, jl_div(X.Ice(j + joff) + exi, dz_ext * DENICE));
-    LV(f.eff_porosity, c, j, ld) = jl_max(0.01, VAL(ws) - VAL(vol_ice));
-    X.Icefrac(j) = jl_min(1.0, jl_div(vol_ice, ws));
-  }
+  const double exi = LV(f.excess_ice, c, j, ld);
+  const double dz_ext = LVc(f.dz, c, j + joff, ld) + jl_div(exi, DENICE);
+  const S ws = X.Watsat(j);
+  const S vol_ice = jl_min(ws, jl_div(X.Ice(j + joff) + exi, dz_ext * DENICE));
+  LV(f.eff_porosity, c, j, ld) = jl_max(0.01, VAL(ws) - VAL(vol_ice));
+  X.Icefrac(j) = jl_min(1.0, jl_div(vol_ice, ws));
 }
-
+__device__ __forceinline__ void water_fractions_level(const Dims& D, const clmgb_soilwater_fields& f, int64_t c, int j) {
+  FieldState<clmgb_soilwater_fields> X(f, c, D.ldc);
+  water_fractions_level(D, f, c, j, X);
+}
+template <class ST>
+__device__ __forceinline__ void water_fractions_col(const Dims& D, const clmgb_soilwater_fields& f, int64_t c,
+                                                    ST& X) {
+  for (int j = 1; j <= D.nlevsoi; j++) water_fractions_level(D, f, c, j, X);
+}
 __device__ __forceinline__ void water_fractions_col(const Dims& D, const clmgb_soilwater_fields& f, int64_t c) {
   FieldState<clmgb_soilwater_fields> X(f, c, D.ldc);
   water_fractions_col(D, f, c, X);

@@ -14,54 +14,6 @@ __device__ __forceinline__ void report(uint32_t st, uint32_t* col_status, uint32
   if (st && dev_status) atomicOr(dev_status, st);
 }
 
-// The column of this thread in the soil-temperature kernels: the block's NB
-// consecutive columns, reordered by snow-layer count (a counting sort in shared
-// memory), so the lanes of a warp run level loops and band solves of about the same
-// length.  Accesses stay inside the block's columns; each column's arithmetic is
-// unchanged, so results do not depend on the order.  Every thread of the block must
-// call it; returns -1 past the last column.
-template <int NB>
-__device__ __forceinline__ int64_t snl_sorted_column(int64_t nc, const int64_t* col_snl, int nlevsno) {
-  __shared__ unsigned int s_cnt[16];
-  __shared__ unsigned short s_perm[NB];
-  const int64_t base = (int64_t)blockIdx.x * NB;
-  if (threadIdx.x < 16) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t c0 = base + threadIdx.x;
-  int key = 15;
-  if (c0 < nc) {
-    const int64_t s = -col_snl[c0];
-    key = (s < 0 || s > nlevsno || s > 13) ? 14 : (int)s;
-  }
-  const unsigned int r = atomicAdd(&s_cnt[key], 1u);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int run = 0;
-    for (int k = 0; k < 16; k++) {
-      const unsigned int t = s_cnt[k];
-      s_cnt[k] = run;
-      run += t;
-    }
-  }
-  __syncthreads();
-  s_perm[s_cnt[key] + r] = (unsigned short)threadIdx.x;
-  __syncthreads();
-  const int64_t c = base + s_perm[threadIdx.x];
-  return c < nc ? c : -1;
-}
-
-// NB threads per block, sorted together; 640 / NB resident blocks (20 warps per SM)
-template <int NB>
-__global__ void __launch_bounds__(NB, 640 / NB)
-k_soil_temperature(Dims D, int64_t nc, clmgb_soiltemp_fields f, double dtime, int snow_method,
-                   uint32_t* col_status, uint32_t* dev_status) {
-  const int64_t c = snl_sorted_column<NB>(nc, f.col_snl, D.nlevsno);
-  if (c < 0) return;
-  uint32_t st = 0;
-  if (f.mask_nolakec[c]) st = soil_temperature_col(D, f, c, dtime, snow_method);
-  report(st, col_status, dev_status, c);
-}
-
 __global__ void __launch_bounds__(BLOCK)
 k_water_fractions(Dims D, int64_t nc, clmgb_soilwater_fields f) {
   const int64_t c = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
@@ -99,68 +51,6 @@ k_column_step(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fiel
     water_fractions_col(D, fw, c);
     st |= moisture_form_col(D, fw, cfg, dtime, c);
   }
-  report(st, col_status, dev_status, c);
-}
-
-// The production state accessor whose band solve also keeps the factorisation in the
-// column's soil_temperature! record (StLog); the solution is band_lu_solve's bits.
-struct FieldStateStLog : FieldState<clmgb_soiltemp_fields> {
-  double* rec;
-  __device__ __forceinline__ FieldStateStLog(const clmgb_soiltemp_fields& ff, int64_t cc, int64_t l, double* r)
-      : FieldState<clmgb_soiltemp_fields>(ff, cc, l), rec(r) {}
-  __device__ __forceinline__ void band_solve(double* ab, double* x, int n) const {
-    uint8_t piv[MAXROWS];
-    band_lu_factor_solve<2, 2>(ab, x, piv, n);
-    rec[ST_N] = (double)n;
-    for (int k = 0; k < n * 7; k++) rec[ST_LU + k] = ab[k];
-    for (int r = 0; r < n; r++) rec[ST_X + r] = x[r];
-    uint8_t* pv = reinterpret_cast<uint8_t*>(rec + ST_PIV);
-    for (int r = 0; r < n; r++) pv[r] = piv[r];
-  }
-};
-
-// soil_temperature! then set_soil_water_fractions! for one column per thread (the
-// first half of a column step; the Richards solve follows in k_moisture_form_queue).
-// With LOG every column soil_temperature! runs on also gets its record in st_log.
-template <bool LOG, int NB>
-__global__ void __launch_bounds__(NB, 640 / NB)
-k_soil_temperature_fractions(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fields fw,
-                             double dtime, int snow_method, double* t_ssbef, double* t_h2osfc_bef,
-                             uint32_t* col_status, uint32_t* dev_status, double* st_log) {
-  const int64_t c = snl_sorted_column<NB>(nc, ft.col_snl, D.nlevsno);
-  if (c < 0) return;
-  uint32_t st = 0;
-  if (ft.mask_nolakec[c]) {
-    if (t_ssbef) {
-      const int L = D.nlevsno + D.nlevmax;
-      for (int jj = 1; jj <= L; jj++) LV(t_ssbef, c, jj, D.ldc) = LV(ft.t_soisno, c, jj, D.ldc);
-    }
-    if (t_h2osfc_bef) t_h2osfc_bef[c] = ft.t_h2osfc[c];
-    if (LOG) {
-      double* rec = st_log + c * (int64_t)CLMGB_LOG_ST_STRIDE;
-      rec[ST_N] = 0.0;
-      FieldStateStLog X(ft, c, D.ldc, rec);
-      const uint32_t s1 = soil_temperature_col(D, ft, c, dtime, snow_method, X);
-      st |= s1;
-      rec[ST_STATUS] = (double)s1;
-      const int64_t snl = ft.col_snl[c];
-      if (snl <= 0 && snl >= -D.nlevsno) {     // the levels the call may have changed
-        const int jjtop = (int)snl + 1 + D.nlevsno;
-        const int nw = D.nlevsno + D.nlevgrnd, nlev = D.nlevsno + D.nlevmax;
-        for (int jj = jjtop; jj <= nlev; jj++) rec[ST_T + jj - 1] = LV(ft.t_soisno, c, jj, D.ldc);
-        for (int jj = jjtop; jj <= nw; jj++) {
-          rec[ST_LIQ + jj - 1] = LV(ft.h2osoi_liq, c, jj, D.ldc);
-          rec[ST_ICE + jj - 1] = LV(ft.h2osoi_ice, c, jj, D.ldc);
-          rec[ST_FACT + jj - 1] = LV(ft.fact, c, jj, D.ldc);
-        }
-      }
-      rec[ST_TG] = ft.t_grnd[c];
-      rec[ST_TH] = ft.t_h2osfc[c];
-    } else {
-      st |= soil_temperature_col(D, ft, c, dtime, snow_method);
-    }
-  }
-  if (fw.mask_hydrology[c]) water_fractions_col(D, fw, c);
   report(st, col_status, dev_status, c);
 }
 
@@ -593,18 +483,6 @@ k_synth_forcing(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fi
 }
 
 // ---------------------------------------------------------------------------
-cudaError_t launch_soil_temperature(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& f, double dtime,
-                                    int snow_method, uint32_t* col_status, uint32_t* dev_status,
-                                    cudaStream_t s) {
-  const unsigned g = (unsigned)((nc + D.st_block - 1) / D.st_block);
-  if (D.st_block == 640)
-    k_soil_temperature<640><<<g, 640, 0, s>>>(D, nc, f, dtime, snow_method, col_status, dev_status);
-  else if (D.st_block == 320)
-    k_soil_temperature<320><<<g, 320, 0, s>>>(D, nc, f, dtime, snow_method, col_status, dev_status);
-  else
-    k_soil_temperature<128><<<g, 128, 0, s>>>(D, nc, f, dtime, snow_method, col_status, dev_status);
-  return cudaGetLastError();
-}
 cudaError_t launch_water_fractions(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, cudaStream_t s) {
   k_water_fractions<<<grid_for(nc), BLOCK, 0, s>>>(D, nc, f);
   return cudaGetLastError();
@@ -621,27 +499,6 @@ cudaError_t launch_column_step(const Dims& D, int64_t nc, const clmgb_soiltemp_f
                                uint32_t* dev_status, cudaStream_t s) {
   k_column_step<<<grid_for(nc), BLOCK, 0, s>>>(D, nc, ft, fw, cfg, dtime, snow_method, t_ssbef, t_h2osfc_bef,
                                                col_status, dev_status);
-  return cudaGetLastError();
-}
-cudaError_t launch_soiltemp_fractions(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,
-                                      const clmgb_soilwater_fields& fw, double dtime, int snow_method,
-                                      double* t_ssbef, double* t_h2osfc_bef, uint32_t* col_status,
-                                      uint32_t* dev_status, cudaStream_t s, double* st_log) {
-  const int nb = (D.st_block == 640 || D.st_block == 320) ? D.st_block : 128;
-  const unsigned g = (unsigned)((nc + nb - 1) / nb);
-#define CLMGB_STF(L, NB) \
-  k_soil_temperature_fractions<L, NB><<<g, NB, 0, s>>>(D, nc, ft, fw, dtime, snow_method, t_ssbef, t_h2osfc_bef, \
-                                                      col_status, dev_status, st_log)
-  if (st_log) {
-    if (nb == 640) CLMGB_STF(true, 640);
-    else if (nb == 320) CLMGB_STF(true, 320);
-    else CLMGB_STF(true, 128);
-  } else {
-    if (nb == 640) CLMGB_STF(false, 640);
-    else if (nb == 320) CLMGB_STF(false, 320);
-    else CLMGB_STF(false, 128);
-  }
-#undef CLMGB_STF
   return cudaGetLastError();
 }
 int queue_blocks_per_sm() {
