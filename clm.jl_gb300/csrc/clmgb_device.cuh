@@ -116,6 +116,54 @@ __device__ __forceinline__ auto jl_div(A x, B y) {
 __device__ __forceinline__ bool abs_lt(double x, double t) {
   return (dbits(x) & 0x7fffffffffffffffLL) < dbits(t);
 }
+// Comparisons as IEEE makes them, on the integer pipes: x > 0, x < 0, x finite, x = +-0,
+// y finite and nonzero; x > t, x >= t, x < t for a positive normal t; |a| > |b|.
+__device__ __forceinline__ bool pos(double x) { return (unsigned long long)(dbits(x) - 1) < 0x7ff0000000000000ULL; }
+__device__ __forceinline__ bool negv(double x) {
+  return ((unsigned long long)dbits(x) ^ 0x8000000000000000ULL) - 1ULL < 0x7ff0000000000000ULL;
+}
+__device__ __forceinline__ bool finite_bits(double x) { return ((dbits(x) >> 52) & 0x7ff) != 0x7ff; }
+__device__ __forceinline__ bool zero_bits(double x) { return (dbits(x) << 1) == 0; }
+__device__ __forceinline__ bool finite_nonzero(double y) {
+  return (unsigned long long)(dbits(y) << 1) - 1ull < 0xffdffffffffffffeull;
+}
+__device__ __forceinline__ bool above(double x, double t) { return dbits(x) > dbits(t) && !isnan_bits(x); }
+__device__ __forceinline__ bool at_least(double x, double t) { return dbits(x) >= dbits(t) && !isnan_bits(x); }
+__device__ __forceinline__ bool below(double x, double t) { return dbits(x) < dbits(t) && !isnan_bits(x); }
+__device__ __forceinline__ bool abs_gt(double a, double b) {
+  const long long x = dbits(a) & 0x7fffffffffffffffLL, y = dbits(b) & 0x7fffffffffffffffLL;
+  return x > y && x <= 0x7ff0000000000000LL;
+}
+// x/2, the exponent lowered by one where that is exact
+__device__ __forceinline__ double half_of(double x) {
+  const long long b = dbits(x);
+  if ((((unsigned)(b >> 52) & 0x7ffu) - 2u) < 0x7fdu) return __longlong_as_double(b - (1LL << 52));
+  return 0.5 * x;
+}
+// a zero over a finite nonzero y
+__device__ __forceinline__ double zero_quotient(double x, double y) {
+  return __longlong_as_double((dbits(x) ^ dbits(y)) & (long long)0x8000000000000000ULL);
+}
+// jl_div's quotient formed in line, for chains of dependent divisions (225 cycles against
+// 359 through the call)
+__device__ __forceinline__ double div_chain(double x, double y) {
+  bool ok;
+  const double q = cm_div_fx(x, y, &ok);
+  const bool zero = zero_bits(x) && finite_nonzero(y);
+  if (ok | zero) return zero ? zero_quotient(x, y) : q;
+  return cm_div_ieee_(x, y);
+}
+// x1 / y and x2 / y in line without a branch, so that they overlap and share the
+// divisor's reciprocal
+__device__ __forceinline__ void div_pair(double x1, double x2, double y, double& q1, double& q2) {
+  bool ok1, ok2;
+  q1 = cm_div_fx(x1, y, &ok1);
+  q2 = cm_div_fx(x2, y, &ok2);
+  if (!(ok1 & ok2)) {
+    q1 = jl_div(x1, y);
+    q2 = jl_div(x2, y);
+  }
+}
 // Julia's Float64 x^4 (Base.Math.pow_body, compensated squaring).
 __device__ __forceinline__ double jl_pow4(double x) {
   double x2 = __dmul_rn(x, x);

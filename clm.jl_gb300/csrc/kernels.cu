@@ -314,66 +314,167 @@ k_phase_change(Dims D, int64_t nc, clmgb_soiltemp_fields f, double dtime, const 
   else phase_change_beta_col(D, f, c, dtime, dhsdT[c]);
 }
 
+// batched_band_solve! (band_diagonal.jl:87-170), a thread per column: band_lu_solve's
+// elimination with its window of KL+1 rows in registers, the rows entering it straight
+// from the band matrix and the right-hand side; the thread keeps the rows of U, and
+// tvector the eliminated right-hand side until the back substitution.  Row exchanges are
+// decided on the bits.  65,537 systems of 26 to 38 rows with five full bands: 186 us,
+// 342 with the band copied to a 2.5 KB stack first and FP64 comparisons.  28 FP64
+// instructions a row, 65 cycles of the sub-partition's FP64 unit each, bound it (110 us).
 template <int KL, int KU>
 __global__ void __launch_bounds__(BLOCK)
 k_band_solve(int64_t nc, int64_t ldc, int nlev, double* tvector, const double* __restrict__ bmatrix,
              const double* __restrict__ rvector, const int64_t* jtop, const int64_t* jbot,
              const uint8_t* mask, int nlevsno_off) {
-  constexpr int W = 2 * KL + KU + 1;
-  constexpr int NB = KL + KU + 1;
+  constexpr int R = KL + 1, C = KL + KU + 1;
   const int64_t c = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (c >= nc || !mask[c]) return;
   const int64_t jt = jtop[c] + nlevsno_off + 1;
   const int64_t n64 = jbot[c] - jtop[c] + 1;
   if (n64 <= 0 || jt < 1 || jt + n64 - 1 > nlev || n64 > MAXROWS + 1) return;
   const int n = (int)n64;
-  double ab[(MAXROWS + 1) * W];
-  double x[MAXROWS + 1];
-  for (int k = 0; k < n * W; k++) ab[k] = 0.0;
-  for (int i = 0; i < n; i++) {
-    const int64_t lev = jt + i;   // 1-based level of row i
-    for (int j = max(0, i - KL); j <= min(n - 1, i + KU); j++) {
-      const int band = (i - j) + KL;   // 0-based band
-      ab[i * W + (j - i + KL)] = bmatrix[c + (int64_t)band * ldc + (lev - 1) * ldc * NB];
-    }
-    x[i] = rvector[c + (lev - 1) * ldc];
+  const double* const bm = bmatrix + c + (jt - 1) * ldc * C;
+  const double* const rv = rvector + c + (jt - 1) * ldc;
+  double* const tv = tvector + c + (jt - 1) * ldc;
+  // A[i, j] of the band (j = i - KL .. i + KU), 0 outside the system
+  auto entry = [&](int i, int j) -> double {
+    return j >= 0 && j < n ? bm[(int64_t)(i - j + KL) * ldc + (int64_t)i * ldc * C] : 0.0;
+  };
+  double u[(MAXROWS + 1) * C];
+  double w[R][C], x[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+#pragma unroll
+    for (int k = 0; k < C; k++) w[i][k] = i < n && k - i <= KU ? entry(i, k) : 0.0;
+    x[i] = i < n ? rv[i * ldc] : 0.0;
   }
-  band_lu_solve<KL, KU>(ab, x, n);
-  for (int i = 0; i < n; i++) tvector[c + (jt + i - 1) * ldc] = x[i];
+  for (int k = 0; k < n; k++) {
+    const int r = k + 1 + KL;                       // the row that enters below
+    double nw[C], nx = 0.0;
+#pragma unroll
+    for (int i = 0; i < C; i++) nw[i] = r < n ? entry(r, k + 1 + i) : 0.0;
+    if (r < n) nx = rv[(int64_t)r * ldc];
+    int piv = 0;
+    long long maxv = dbits(w[0][0]) & 0x7fffffffffffffffLL;
+#pragma unroll
+    for (int i = 1; i < R; i++) {
+      const long long v = dbits(w[i][0]) & 0x7fffffffffffffffLL;
+      if (k + i < n && v > maxv && v <= 0x7ff0000000000000LL) {
+        maxv = v;
+        piv = i;
+      }
+    }
+#pragma unroll
+    for (int i = 1; i < R; i++) {
+      const bool sw = i == piv;
+#pragma unroll
+      for (int e = 0; e < C; e++) {
+        const double t = w[0][e];
+        w[0][e] = sw ? w[i][e] : t;
+        w[i][e] = sw ? t : w[i][e];
+      }
+      const double t = x[0];
+      x[0] = sw ? x[i] : t;
+      x[i] = sw ? t : x[i];
+    }
+    double f[R];
+    if (k + R - 1 < n) {
+      if constexpr (R == 3) div_pair(w[1][0], w[2][0], w[0][0], f[1], f[2]);
+      else f[1] = jl_div(w[1][0], w[0][0]);
+    } else if (k + 1 < n) {
+      f[1] = jl_div(w[1][0], w[0][0]);
+    }
+#pragma unroll
+    for (int i = 1; i < R; i++) {
+      if (k + i < n) {
+#pragma unroll
+        for (int e = 1; e < C; e++) w[i][e] = w[i][e] - f[i] * w[0][e];
+        x[i] = x[i] - f[i] * x[0];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < C; e++) u[k * C + e] = w[0][e];
+    tv[(int64_t)k * ldc] = x[0];
+    // slide down a row and right a column
+#pragma unroll
+    for (int i = 0; i < R - 1; i++) {
+#pragma unroll
+      for (int e = 0; e < C - 1; e++) w[i][e] = w[i + 1][e + 1];
+      w[i][C - 1] = 0.0;
+      x[i] = x[i + 1];
+    }
+#pragma unroll
+    for (int e = 0; e < C; e++) w[R - 1][e] = nw[e];
+    x[R - 1] = nx;
+  }
+  double y[C];                                      // x of the rows below
+#pragma unroll
+  for (int e = 0; e < C; e++) y[e] = 0.0;
+  for (int i = n - 1; i >= 0; i--) {
+    double s = tv[(int64_t)i * ldc];
+#pragma unroll
+    for (int e = 1; e < C; e++)
+      if (i + e < n) s = s - u[i * C + e] * y[e - 1];
+    const double xi = jl_div(s, u[i * C]);
+#pragma unroll
+    for (int e = C - 1; e > 0; e--) y[e] = y[e - 1];
+    y[0] = xi;
+    tv[(int64_t)i * ldc] = xi;
+  }
 }
 
 constexpr int MAXTRI = 64;
 
+// tridiagonal_multi! (tridiagonal.jl:86-127), a thread per column.  The coefficients are
+// loaded three levels ahead (one level ahead measured 72 us for the case below: a level's
+// arithmetic is shorter than a load); of the sweep's two results per level one waits in
+// shared memory ([level][thread], no bank conflicts), the other in u.  100,003 systems of
+// 21 levels: 37 us, 113 with the hardware division, FP64 comparisons, loads in step and
+// the results in local memory.  Six FP64 instructions a level (20 us) and 101 MB of memory
+// traffic (15 us) bound it.
 __global__ void __launch_bounds__(BLOCK)
 k_tridiagonal_multi(int64_t ncols, int64_t ld, int nlevs, double* u, const double* __restrict__ a,
                     const double* __restrict__ b, const double* __restrict__ cc, const double* __restrict__ r,
                     const int64_t* jtop, const uint8_t* mask) {
-  const int64_t col = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
+  extern __shared__ double smem_tri[];
+  const int nt = blockDim.x;
+  const int64_t col = (int64_t)blockIdx.x * nt + threadIdx.x;
   if (col >= ncols || !mask[col]) return;
   const int64_t j64 = jtop[col];
   if (j64 < 1 || j64 > nlevs) return;
   const int j = (int)j64;
-  double cpv[MAXTRI + 1], dpv[MAXTRI + 1];
+  double* const cp = smem_tri + threadIdx.x;
   const double tiny = 1e-30;
-  double bet = LVc(b, col, j, ld);
-  if (fabs(bet) < tiny) bet = tiny;
-  double cp_prev = LVc(cc, col, j, ld) / bet;
-  double dp_prev = LVc(r, col, j, ld) / bet;
-  cpv[j] = cp_prev;
-  dpv[j] = dp_prev;
-  for (int jj = j + 1; jj <= nlevs; jj++) {
-    double denom = LVc(b, col, jj, ld) - LVc(a, col, jj, ld) * cp_prev;
-    if (fabs(denom) < tiny) denom = copysign(tiny, denom == 0.0 ? 1.0 : denom);
-    cp_prev = LVc(cc, col, jj, ld) / denom;
-    dp_prev = (LVc(r, col, jj, ld) - LVc(a, col, jj, ld) * dp_prev) / denom;
-    cpv[jj] = cp_prev;
-    dpv[jj] = dp_prev;
+  struct Level { double a, b, c, r; };
+  auto load = [&](int jj) -> Level {
+    if (jj > nlevs) return Level{0.0, 0.0, 0.0, 0.0};
+    return Level{LVc(a, col, jj, ld), LVc(b, col, jj, ld), LVc(cc, col, jj, ld), LVc(r, col, jj, ld)};
+  };
+  Level v = load(j), v1 = load(j + 1), v2 = load(j + 2);
+  double cp_prev = 0.0, dp_prev = 0.0;
+  for (int jj = j; jj <= nlevs; jj++) {
+    const Level v3 = load(jj + 3);
+    double denom = v.b, num = v.r;
+    if (jj == j) {
+      if (abs_lt(denom, tiny)) denom = tiny;
+    } else {
+      denom = v.b - v.a * cp_prev;
+      if (abs_lt(denom, tiny)) denom = copysign(tiny, denom == 0.0 ? 1.0 : denom);
+      num = v.r - v.a * dp_prev;
+    }
+    div_pair(v.c, num, denom, cp_prev, dp_prev);
+    cp[(jj - 1) * nt] = cp_prev;
+    LV(u, col, jj, ld) = dp_prev;
+    v = v1;
+    v1 = v2;
+    v2 = v3;
   }
-  double u_next = dp_prev;
-  LV(u, col, nlevs, ld) = u_next;
+  double u_next = dp_prev, d = nlevs > j ? LV(u, col, nlevs - 1, ld) : 0.0;
   for (int jj = nlevs - 1; jj >= j; jj--) {
-    u_next = dpv[jj] - cpv[jj] * u_next;
+    const double dn = jj > j ? LV(u, col, jj - 1, ld) : 0.0;
+    u_next = d - cp[(jj - 1) * nt] * u_next;
     LV(u, col, jj, ld) = u_next;
+    d = dn;
   }
 }
 
@@ -606,8 +707,15 @@ cudaError_t launch_tridiagonal_multi(int64_t ncols, int64_t ldc, int nlevs, doub
   if (method == CLMGB_TRIDIAG_PCR)
     k_tridiagonal_multi_pcr<<<(unsigned)((ncols + PCR_WARPS - 1) / PCR_WARPS), 32 * PCR_WARPS, 0, s>>>(
         ncols, ldc, nlevs, u, a, b, c, r, jtop, mask);
-  else
-    k_tridiagonal_multi<<<grid_for(ncols), BLOCK, 0, s>>>(ncols, ldc, nlevs, u, a, b, c, r, jtop, mask);
+  else {
+    const int nt = BLOCK;          // 64 KB at MAXTRI levels: three blocks on an SM
+    const size_t smem = (size_t)nlevs * nt * sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(k_tridiagonal_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return e;
+    k_tridiagonal_multi<<<(unsigned)((ncols + nt - 1) / nt), nt, smem, s>>>(ncols, ldc, nlevs, u, a, b, c, r, jtop,
+                                                                           mask);
+  }
   return cudaGetLastError();
 }
 cudaError_t launch_synth_forcing(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,

@@ -68,23 +68,6 @@ __host__ __device__ constexpr int64_t warp_bytes(int nls, bool expensive) {
   return level_doubles(nls, expensive) * 8 + (int64_t)((sizeof(SlotArea) + 15) / 16 * 16);
 }
 
-// x/2, the exponent lowered by one where that is exact
-__device__ __forceinline__ double half_of(double x) {
-  const long long b = dbits(x);
-  if ((((unsigned)(b >> 52) & 0x7ffu) - 2u) < 0x7fdu) return __longlong_as_double(b - (1LL << 52));
-  return 0.5 * x;
-}
-__device__ __forceinline__ bool finite_bits(double x) { return ((dbits(x) >> 52) & 0x7ff) != 0x7ff; }
-
-// jl_div with the quotient formed in line, for the recurrences' chain of dependent
-// divisions
-__device__ __forceinline__ double div_inl(double x, double y) {
-  const unsigned long long bx = (unsigned long long)dbits(x), by = (unsigned long long)dbits(y);
-  if ((bx << 1) == 0 && (by << 1) - 1ull < 0xffdffffffffffffeull)
-    return __longlong_as_double((long long)((bx ^ by) & 0x8000000000000000ull));
-  return cm_div(x, y);
-}
-
 template <bool LOG, bool EXPENSIVE>
 __global__ void __launch_bounds__(PBLOCK, 2)
 k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_config cfg, double dtime,
@@ -422,7 +405,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
           w = up ? A(LA_R, j, s) : A(LA_B, j, s);
           cn = A(LA_C, j, s);
         }
-        const double q = div_inl(u, __shfl_sync(FULL, bet, s));
+        const double q = div_chain(u, __shfl_sync(FULL, bet, s));
         const double v = w - a * q;
         if (j <= ns + 1 && ns) A(up ? LA_R : LA_C, j - 1, s) = q;     // dwat of level j-1, gam of level j
         if (j <= ns) {

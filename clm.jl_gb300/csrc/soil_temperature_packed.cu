@@ -44,45 +44,8 @@ constexpr int TWARPS = 4, TBLOCK = 32 * TWARPS;
 constexpr int WARP_FORM = 40;
 constexpr int TROWS = MAXROWS;                 // snow levels, the surface-water row, ground levels
 
-__device__ __forceinline__ bool finite_bits(double x) { return ((dbits(x) >> 52) & 0x7ff) != 0x7ff; }
-// x/2, the exponent lowered by one where that is exact
-__device__ __forceinline__ double half_of(double x) {
-  const long long b = dbits(x);
-  if ((((unsigned)(b >> 52) & 0x7ffu) - 2u) < 0x7fdu) return __longlong_as_double(b - (1LL << 52));
-  return 0.5 * x;
-}
-// x > 0, x < 0 (false for NaN)
-__device__ __forceinline__ bool pos(double x) { return (unsigned long long)(dbits(x) - 1) < 0x7ff0000000000000ULL; }
-__device__ __forceinline__ bool negv(double x) {
-  return ((unsigned long long)dbits(x) ^ 0x8000000000000000ULL) - 1ULL < 0x7ff0000000000000ULL;
-}
-// x > t, x >= t, x < t for a positive normal t (false for NaN)
-__device__ __forceinline__ bool above(double x, double t) { return dbits(x) > dbits(t) && !isnan_bits(x); }
-__device__ __forceinline__ bool at_least(double x, double t) { return dbits(x) >= dbits(t) && !isnan_bits(x); }
-__device__ __forceinline__ bool below(double x, double t) { return dbits(x) < dbits(t) && !isnan_bits(x); }
-// |a| > |b| as IEEE compares them (false with a NaN)
-__device__ __forceinline__ bool abs_gt(double a, double b) {
-  const long long x = dbits(a) & 0x7fffffffffffffffLL, y = dbits(b) & 0x7fffffffffffffffLL;
-  return x > y && x <= 0x7ff0000000000000LL;
-}
 // -0, or a number so small that its upper word is -0's
 __device__ __forceinline__ bool minus_zero(double x) { return (uint32_t)((unsigned long long)dbits(x) >> 32) == 0x80000000u; }
-__device__ __forceinline__ bool zero_bits(double x) { return (dbits(x) << 1) == 0; }
-// a zero over a finite nonzero y
-__device__ __forceinline__ double zero_quotient(double x, double y) {
-  return __longlong_as_double((dbits(x) ^ dbits(y)) & (long long)0x8000000000000000ULL);
-}
-__device__ __forceinline__ bool finite_nonzero(double y) {
-  return (unsigned long long)(dbits(y) << 1) - 1ull < 0xffdffffffffffffeull;
-}
-// a quotient of the banded solve's chain, formed in line
-__device__ __forceinline__ double div_chain(double x, double y) {
-  bool ok;
-  const double q = cm_div_fx(x, y, &ok);
-  const bool zero = zero_bits(x) && finite_nonzero(y);
-  if (ok | zero) return zero ? zero_quotient(x, y) : q;
-  return cm_div_ieee_(x, y);
-}
 
 // a column's rows in shared memory, [array][row][slot]: row jj-1 of snow level jj, row
 // nlevsno of the surface water, row jj of soil level jj.  RS, RD, RP hold A[r, r-1 .. r+1],
