@@ -42,6 +42,9 @@ _SIGS = {
     "clmgb_mlp_silu_backward": ([P, I64, P, P, P, P], I32),
     "clmgb_mlp_loss": ([P, I64, P, P, C.c_float, C.c_float, P, P, P], I32),
     "clmgb_mlp_adam": ([P, I64, I64, P, P, P, P, C.c_float, C.c_float, C.c_float, C.c_float, I32, P, P, P], I32),
+    "clmgb_mlp_forward": ([P, I64, P, P, P, P, P, P, P, P], I32),
+    "clmgb_mlp_gradients": ([P, I64, P, P, P, P, P, P, P, P, P], I32),
+    "clmgb_mlp_adam_net": ([P, P, P, C.c_float, C.c_float, C.c_float, C.c_float, I32, P], I32),
     "clmgb_mlp_features": ([P, P, P, P, F64, P, P, P, P], I32),
     "clmgb_mlp_first_dt": ([P, I64, P, F64, C.c_float, I32, P, P], I32),
     "clmgb_column_step_vjp": ([P, P, P, P, P, F64, I32, P, P, P, P, P], I32),

@@ -123,6 +123,17 @@ class SwmConfig(C.Structure):
         return cls(MOISTURE_FORM, BC_FLUX, BC_ZERO_FLUX, 1, 60.0, 1.0e-8, 1.0e-1, 1.0e-2, 6.0)
 
 
+class MlpNet(C.Structure):
+    """clmgb_mlp_net: the warm-start network's parameters and optimiser state."""
+    _fields_ = [("struct_size", C.c_int64)] + [(n, C.c_void_p * 3)
+                                               for n in ("w", "b", "wb", "wt", "mw", "vw", "mb", "vb")]
+
+
+class MlpGrad(C.Structure):
+    """clmgb_mlp_grad: the gradients of the weights and biases."""
+    _fields_ = [("struct_size", C.c_int64), ("dw", C.c_void_p * 3), ("db", C.c_void_p * 3)]
+
+
 # clmgb_surface_hydrology stages (CLMGB_SH_*), in the driver's order
 SH_FLOODC, SH_SAT_EXCESS, SH_QFLX_INPUTS, SH_INFL_EXCESS, SH_ROUTE = 1, 2, 4, 8, 16
 SH_UPDATE_H2OSFC, SH_INFILTRATION, SH_TOTAL_RUNOFF, SH_URBAN_PONDING = 32, 64, 128, 256

@@ -9,8 +9,8 @@ accepts or halves the proposal like any substep, so the result meets the same
 tolerance as the plain solve.
 
 Training pairs come from the plain FP64 solver (clmgb_mlp_samples); training and
-inference run on the GPU through the library's kernels (mma.sync linear layers,
-CUDA-core weight gradients, Adam).  torch only holds the buffers.
+inference run on the GPU through the library's kernels (one launch for the forward pass,
+one for the backward pass, both on mma.sync, and one for Adam).  torch only holds the buffers.
 """
 import ctypes as C
 import math
@@ -31,6 +31,18 @@ def _p(t):
 def _s(stream):
     import torch
     return C.c_void_p((stream or torch.cuda.current_stream()).cuda_stream)
+
+
+_P3 = C.c_void_p * 3
+
+
+def _aligned(t, stream):
+    """t, or a copy on a 16-byte boundary: the fused passes load 16 bytes at a time."""
+    if t.data_ptr() % 16 == 0:
+        return t
+    import torch
+    with torch.cuda.stream(stream or torch.cuda.current_stream()):
+        return t.clone()
 
 
 class WarmStartMLP:
@@ -61,22 +73,28 @@ class WarmStartMLP:
         self.step = 0
 
     # ---- forward / backward through the library kernels ----
+    @staticmethod
+    def _net(**arrays):
+        """clmgb_mlp_net with the members that a call reads."""
+        net = abi.MlpNet(C.sizeof(abi.MlpNet))
+        for name, ts in arrays.items():
+            setattr(net, name, _P3(*(t.data_ptr() for t in ts)))
+        return net
+
     def forward(self, X, keep=False, stream=None):
         """X: [M, 64] bf16 (normalised).  Returns Y [M, 32] fp32 (and activations)."""
         torch = self.torch
         M = X.shape[0]
-        lib, h, st = self.h.lib, self.h.h, _s(stream)
-        Z1 = torch.empty((M, HID), dtype=torch.float32, device=X.device)
-        H1 = torch.empty((M, HID), dtype=torch.bfloat16, device=X.device)
-        Z2 = torch.empty_like(Z1)
-        H2 = torch.empty_like(H1)
+        X, wb = _aligned(X, stream), [_aligned(w, stream) for w in self.wb]
         Y = torch.empty((M, OUTP), dtype=torch.float32, device=X.device)
-        check(lib.clmgb_mlp_linear(h, M, HID, IN, _p(X), IN, _p(self.wb[0]), _p(self.b[0]), 1, _p(Z1), HID,
-                                   _p(H1), HID, st), "mlp_linear 1")
-        check(lib.clmgb_mlp_linear(h, M, HID, HID, _p(H1), HID, _p(self.wb[1]), _p(self.b[1]), 1, _p(Z2), HID,
-                                   _p(H2), HID, st), "mlp_linear 2")
-        check(lib.clmgb_mlp_linear(h, M, OUTP, HID, _p(H2), HID, _p(self.wb[2]), _p(self.b[2]), 0, _p(Y), OUTP,
-                                   None, OUTP, st), "mlp_linear 3")
+        Z1 = Z2 = H1 = H2 = None
+        if keep:
+            Z1 = torch.empty((M, HID), dtype=torch.float32, device=X.device)
+            H1 = torch.empty((M, HID), dtype=torch.bfloat16, device=X.device)
+            Z2 = torch.empty_like(Z1)
+            H2 = torch.empty_like(H1)
+        check(self.h.lib.clmgb_mlp_forward(self.h.h, M, _p(X), C.byref(self._net(b=self.b, wb=wb)), _p(Z1), _p(H1), _p(Z2),
+                                           _p(H2), _p(Y), _s(stream)), "mlp_forward")
         if keep:
             return Y, (X, Z1, H1, Z2, H2)
         return Y
@@ -84,25 +102,20 @@ class WarmStartMLP:
     def gradients(self, acts, dY, stream=None):
         """Backward pass: returns (dW, db) per layer (fp32)."""
         torch = self.torch
-        X, Z1, H1, Z2, H2 = acts
+        X, Z1, H1, Z2, H2 = (_aligned(t, stream) for t in acts)
+        dY, wt = _aligned(dY, stream), [_aligned(w, stream) for w in self.wt]
         M = X.shape[0]
-        lib, h, st = self.h.lib, self.h.h, _s(stream)
-        dW = [torch.zeros_like(w) for w in self.w]
-        db = [torch.zeros_like(b) for b in self.b]
-        check(lib.clmgb_mlp_linear_dw(h, M, OUTP, HID, _p(dY), OUTP, _p(H2), HID, _p(dW[2]), _p(db[2]), st), "dw3")
-        dH2 = torch.empty((M, HID), dtype=torch.bfloat16, device=X.device)
-        check(lib.clmgb_mlp_linear(h, M, HID, OUTP, _p(dY), OUTP, _p(self.wt[2]), None, 0, None, HID, _p(dH2), HID,
-                                   st), "dx3")
-        dZ2 = torch.empty_like(dH2)
-        check(lib.clmgb_mlp_silu_backward(h, M * HID, _p(Z2), _p(dH2), _p(dZ2), st), "silu2")
-        check(lib.clmgb_mlp_linear_dw(h, M, HID, HID, _p(dZ2), HID, _p(H1), HID, _p(dW[1]), _p(db[1]), st), "dw2")
-        dH1 = torch.empty_like(dH2)
-        check(lib.clmgb_mlp_linear(h, M, HID, HID, _p(dZ2), HID, _p(self.wt[1]), None, 0, None, HID, _p(dH1), HID,
-                                   st), "dx2")
-        dZ1 = torch.empty_like(dH1)
-        check(lib.clmgb_mlp_silu_backward(h, M * HID, _p(Z1), _p(dH1), _p(dZ1), st), "silu1")
-        check(lib.clmgb_mlp_linear_dw(h, M, HID, IN, _p(dZ1), HID, _p(X), IN, _p(dW[0]), _p(db[0]), st), "dw1")
+        g = torch.empty(sum(o * i + o for o, i in LAYERS), dtype=torch.float32, device=X.device)
+        parts = g.split([o * i for o, i in LAYERS] + [o for o, _ in LAYERS])
+        dW, db = [p.view(s) for p, s in zip(parts, LAYERS)], list(parts[3:])
+        check(self.h.lib.clmgb_mlp_gradients(self.h.h, M, _p(X), _p(Z1), _p(H1), _p(Z2), _p(H2), _p(dY),
+                                             C.byref(self._net(wt=wt)), C.byref(self._grad(dW, db)), _s(stream)),
+              "mlp_gradients")
         return dW, db
+
+    @staticmethod
+    def _grad(dW, db):
+        return abi.MlpGrad(C.sizeof(abi.MlpGrad), *(_P3(*(t.data_ptr() for t in ts)) for ts in (dW, db)))
 
     def loss(self, Y, T, w_dt=1.0, w_incr=1.0, stream=None):
         torch = self.torch
@@ -115,12 +128,9 @@ class WarmStartMLP:
 
     def adam(self, dW, db, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8, stream=None):
         self.step += 1
-        lib, h, st = self.h.lib, self.h.h, _s(stream)
-        for li, (o, i) in enumerate(LAYERS):
-            check(lib.clmgb_mlp_adam(h, o, i, _p(self.w[li]), _p(dW[li]), _p(self.mw[li]), _p(self.vw[li]),
-                                     lr, b1, b2, eps, self.step, _p(self.wb[li]), _p(self.wt[li]), st), "adam w")
-            check(lib.clmgb_mlp_adam(h, 1, o, _p(self.b[li]), _p(db[li]), _p(self.mb[li]), _p(self.vb[li]),
-                                     lr, b1, b2, eps, self.step, None, None, st), "adam b")
+        net = self._net(w=self.w, b=self.b, wb=self.wb, wt=self.wt, mw=self.mw, vw=self.vw, mb=self.mb, vb=self.vb)
+        check(self.h.lib.clmgb_mlp_adam_net(self.h.h, C.byref(net), C.byref(self._grad(dW, db)), lr, b1, b2, eps,
+                                            self.step, _s(stream)), "adam")
 
     # ---- data ----
     def set_normalisation(self, F, T):

@@ -1190,6 +1190,61 @@ int32_t clmgb_mlp_adam(clmgb_handle h, int64_t rows, int64_t cols, float* w, con
   return ce == cudaSuccess ? CLMGB_OK : cuda_fail(h, ce);
 }
 
+static bool aligned16(std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if ((uintptr_t)p & 15) return false;
+  return true;
+}
+
+int32_t clmgb_mlp_forward(clmgb_handle h, int64_t M, const uint16_t* X, const clmgb_mlp_net* net, float* Z1,
+                          uint16_t* H1, float* Z2, uint16_t* H2, float* Y, void* stream) {
+  if (!handle_ok(h)) return CLMGB_ERR_HANDLE;
+  if (!net) return CLMGB_ERR_NULL_ARG;
+  if (net->struct_size != (int64_t)sizeof(*net)) return CLMGB_ERR_ABI;
+  if (M < 0) return CLMGB_ERR_DIMS;
+  if (!X || !Y) return CLMGB_ERR_NULL_ARG;
+  const int kept = (Z1 != nullptr) + (H1 != nullptr) + (Z2 != nullptr) + (H2 != nullptr);
+  if (kept != 0 && kept != 4) return CLMGB_ERR_NULL_ARG;
+  for (int i = 0; i < 3; i++)
+    if (!net->wb[i] || !net->b[i]) return CLMGB_ERR_NULL_ARG;
+  if (!aligned16({X, Z1, H1, Z2, H2, Y, net->wb[0], net->wb[1], net->wb[2]})) return CLMGB_ERR_UNSUPPORTED;
+  cudaError_t ce = clmgb::launch_mlp_forward(M, X, *net, Z1, H1, Z2, H2, Y, h->num_sms, (cudaStream_t)stream);
+  return ce == cudaSuccess ? CLMGB_OK : cuda_fail(h, ce);
+}
+
+int32_t clmgb_mlp_gradients(clmgb_handle h, int64_t M, const uint16_t* X, const float* Z1, const uint16_t* H1,
+                            const float* Z2, const uint16_t* H2, const uint16_t* dY, const clmgb_mlp_net* net,
+                            const clmgb_mlp_grad* grad, void* stream) {
+  if (!handle_ok(h)) return CLMGB_ERR_HANDLE;
+  if (!net || !grad) return CLMGB_ERR_NULL_ARG;
+  if (net->struct_size != (int64_t)sizeof(*net) || grad->struct_size != (int64_t)sizeof(*grad))
+    return CLMGB_ERR_ABI;
+  if (M < 0) return CLMGB_ERR_DIMS;
+  if (!X || !Z1 || !H1 || !Z2 || !H2 || !dY) return CLMGB_ERR_NULL_ARG;
+  if (!net->wt[1] || !net->wt[2]) return CLMGB_ERR_NULL_ARG;
+  for (int i = 0; i < 3; i++)
+    if (!grad->dw[i] || !grad->db[i]) return CLMGB_ERR_NULL_ARG;
+  if (!aligned16({X, Z1, H1, Z2, H2, dY, net->wt[1], net->wt[2], grad->dw[0], grad->dw[1], grad->dw[2]}))
+    return CLMGB_ERR_UNSUPPORTED;
+  cudaError_t ce = clmgb::launch_mlp_gradients(M, X, Z1, H1, Z2, H2, dY, *net, *grad, (cudaStream_t)stream);
+  return ce == cudaSuccess ? CLMGB_OK : cuda_fail(h, ce);
+}
+
+int32_t clmgb_mlp_adam_net(clmgb_handle h, const clmgb_mlp_net* net, const clmgb_mlp_grad* grad, float lr,
+                           float beta1, float beta2, float eps, int32_t step, void* stream) {
+  if (!handle_ok(h)) return CLMGB_ERR_HANDLE;
+  if (!net || !grad) return CLMGB_ERR_NULL_ARG;
+  if (net->struct_size != (int64_t)sizeof(*net) || grad->struct_size != (int64_t)sizeof(*grad))
+    return CLMGB_ERR_ABI;
+  if (step < 1) return CLMGB_ERR_DIMS;
+  for (int i = 0; i < 3; i++)
+    if (!net->w[i] || !net->b[i] || !net->mw[i] || !net->vw[i] || !net->mb[i] || !net->vb[i] || !grad->dw[i] ||
+        !grad->db[i])
+      return CLMGB_ERR_NULL_ARG;
+  cudaError_t ce = clmgb::launch_mlp_adam_net(*net, *grad, lr, beta1, beta2, eps, step, (cudaStream_t)stream);
+  return ce == cudaSuccess ? CLMGB_OK : cuda_fail(h, ce);
+}
+
 int32_t clmgb_mlp_features(clmgb_handle h, const clmgb_bounds* b, const clmgb_soilwater_fields* f,
                            const clmgb_swm_config* cfg, double dtime, const float* mean, const float* istd,
                            uint16_t* X, void* stream) {

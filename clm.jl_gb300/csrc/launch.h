@@ -233,6 +233,13 @@ cudaError_t launch_mlp_loss(int64_t M, const float* Y, const float* T, float w0,
                             cudaStream_t s);
 cudaError_t launch_mlp_adam(int64_t rows, int64_t cols, float* w, const float* g, float* m, float* v, float lr,
                             float b1, float b2, float eps, int step, void* wb, void* wbt, cudaStream_t s);
+cudaError_t launch_mlp_forward(int64_t M, const void* X, const clmgb_mlp_net& net, float* Z1, void* H1, float* Z2,
+                               void* H2, float* Y, int num_sms, cudaStream_t s);
+cudaError_t launch_mlp_gradients(int64_t M, const void* X, const float* Z1, const void* H1, const float* Z2,
+                                 const void* H2, const void* dY, const clmgb_mlp_net& net, const clmgb_mlp_grad& g,
+                                 cudaStream_t s);
+cudaError_t launch_mlp_adam_net(const clmgb_mlp_net& net, const clmgb_mlp_grad& g, float lr, float b1, float b2,
+                                float eps, int step, cudaStream_t s);
 cudaError_t launch_richards_samples(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,
                                     const clmgb_swm_config& cfg, double dtime, int rmax, float* feat, float* targ,
                                     unsigned int* count, int64_t capacity, uint32_t* col_status, cudaStream_t s);

@@ -13,6 +13,8 @@
 //   k_richards_samples    the plain solver, recording training pairs at the first R
 //                         substep starts of every column: features, and the label
 //                         found by trial attempts at remaining/2^k, k = 0, 1, ...
+// The passes over all layers are in mlp_fused.cu; the per-layer kernels here serve the
+// per-layer entry points.
 //   k_linear<K, N>        Y = act(X W^T + b) with mma.sync m16n8k16 (bf16 x bf16 ->
 //                         fp32); one warp owns 16 rows and all N outputs
 //   k_linear_dw<N, K>     dW += dZ^T X, db += sum dZ over a chunk of rows (CUDA cores,
@@ -44,39 +46,43 @@ __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 //   63     log2(dtime / 60 s) / 6
 // liq(j) gives the liquid water of soil level j.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float feature_saturation(double liq, double dz, double watsat) {
+  return (float)liq / (1000.0f * (float)dz * (float)watsat);
+}
+
+// s, ice: the level's saturation and ice fraction; below, ice_below: those of the next
+// level, not used at the lowest one
+__device__ __forceinline__ float feature_log_conductivity(bool lowest, float s, float below, double ice,
+                                                          double ice_below, double bsw, double hksat, float e_ice) {
+  float s1 = lowest ? s : 0.5f * (s + below);
+  s1 = fminf(fmaxf(s1, 0.01f), 1.0f);
+  const float fi = lowest ? (float)ice : 0.5f * (float)(ice + ice_below);
+  return log10f((float)hksat) + (2.0f * (float)bsw + 3.0f) * log10f(s1) - e_ice * fi;
+}
+
 template <class LiqF>
 __device__ __forceinline__ void column_features(const Dims& D, const clmgb_soilwater_fields& f,
                                                 const clmgb_swm_config& cfg, int64_t c, int nlayers, LiqF liq,
                                                 double rem, double dtime, float* x) {
   const int64_t ld = D.ldc;
-  const int joff = D.nlevsno;
-  float s[FEAT_LEVELS + 2];
+  float s[FEAT_LEVELS + 2] = {};
   float sink = 0.0f;
   for (int j = 1; j <= FEAT_LEVELS; j++) {
     const bool in = j <= nlayers;
     float sv = 0.0f;
     if (in) {
-      const float dz = (float)LVc(f.dz, c, joff + j, ld);
-      const float ws = (float)LVc(f.watsat, c, j, ld);
-      sv = (float)liq(j) / (1000.0f * dz * ws);
+      sv = feature_saturation(liq(j), LVc(f.dz, c, D.nlevsno + j, ld), LVc(f.watsat, c, j, ld));
       sink += (float)LVc(f.qflx_rootsoi, c, j, ld);
     }
     s[j] = sv;
     x[j - 1] = sv;
     x[19 + j] = in ? (float)LV(f.icefrac, c, j, ld) : 0.0f;
   }
-  for (int j = 1; j <= FEAT_LEVELS; j++) {
-    if (j > nlayers) {
-      x[39 + j] = -30.0f;
-      continue;
-    }
-    float s1 = (j == nlayers) ? s[j] : 0.5f * (s[j] + s[j + 1]);
-    s1 = fminf(fmaxf(s1, 0.01f), 1.0f);
-    const float fi = (j == nlayers) ? (float)LV(f.icefrac, c, j, ld)
-                                    : 0.5f * (float)(LV(f.icefrac, c, j, ld) + LV(f.icefrac, c, j + 1, ld));
-    const float b = (float)LVc(f.bsw, c, j, ld);
-    x[39 + j] = log10f((float)LVc(f.hksat, c, j, ld)) + (2.0f * b + 3.0f) * log10f(s1) - (float)cfg.e_ice * fi;
-  }
+  for (int j = 1; j <= FEAT_LEVELS; j++)
+    x[39 + j] = j > nlayers ? -30.0f
+                            : feature_log_conductivity(j == nlayers, s[j], s[j + 1], LV(f.icefrac, c, j, ld),
+                                                       j == nlayers ? 0.0 : LV(f.icefrac, c, j + 1, ld),
+                                                       LVc(f.bsw, c, j, ld), LVc(f.hksat, c, j, ld), (float)cfg.e_ice);
   x[60] = (float)(f.qflx_infl[c] * 1.0e3);
   x[61] = sink * 1.0e3f;
   x[62] = (float)(rem / dtime);
@@ -260,29 +266,38 @@ __global__ void k_silu_backward(int64_t n, const float* Z, const __nv_bfloat16* 
   dZ[i] = __float2bfloat16(__bfloat162float(dY[i]) * s * (1.0f + z * (1.0f - s)));
 }
 
-// loss = sum_m [w0 (y0 - t0)^2 + w1/20 sum_{j=1..20} (yj - tj)^2] / M ; dY bf16 [M x 32]
-__global__ void k_mlp_loss(int64_t M, const float* Y, const float* T, float w0, float w1, float* loss,
-                           __nv_bfloat16* dY) {
-  const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  const float* y = Y + m * MLP_OUTP;
-  const float* t = T + m * MLP_OUTP;
+// loss = sum_m [w0 (y0 - t0)^2 + w1/20 sum_{j=1..20} (yj - tj)^2] / M ; dY bf16 [M x 32].
+// A lane is an output, a warp takes LOSS_ROWS rows: coalesced rows and one atomic per block
+// (a thread per row took 12 us at 4,096 rows: strided rows and 4,096 atomics; this, 3 us).
+constexpr int LOSS_WARPS = 8, LOSS_ROWS = 4;
+__global__ void __launch_bounds__(32 * LOSS_WARPS)
+k_mlp_loss(int64_t M, const float* Y, const float* T, float w0, float w1, float* loss, __nv_bfloat16* dY) {
+  static_assert(MLP_OUTP == 32, "a lane per output");
+  __shared__ float part[LOSS_WARPS];
+  const int warp = threadIdx.x >> 5, j = threadIdx.x & 31;
+  const int64_t m0 = ((int64_t)blockIdx.x * LOSS_WARPS + warp) * LOSS_ROWS;
+  const float inv = 1.0f / (float)M, w = j == 0 ? w0 : w1 / FEAT_LEVELS;
   float l = 0.0f;
-  const float inv = 1.0f / (float)M;
-  for (int j = 0; j < MLP_OUTP; j++) {
+#pragma unroll
+  for (int i = 0; i < LOSS_ROWS; i++) {
+    const int64_t m = m0 + i;
+    if (m >= M) break;
     float d = 0.0f;
-    if (j == 0) {
-      const float e = y[0] - t[0];
-      l += w0 * e * e;
-      d = 2.0f * w0 * e * inv;
-    } else if (j <= FEAT_LEVELS) {
-      const float e = y[j] - t[j];
-      l += (w1 / FEAT_LEVELS) * e * e;
-      d = 2.0f * (w1 / FEAT_LEVELS) * e * inv;
+    if (j <= FEAT_LEVELS) {
+      const float e = Y[m * MLP_OUTP + j] - T[m * MLP_OUTP + j];
+      l += w * e * e;
+      d = 2.0f * w * e * inv;
     }
     dY[m * MLP_OUTP + j] = __float2bfloat16(d);
   }
-  atomicAdd(loss, l * inv);
+  for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  if (j == 0) part[warp] = l;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    l = 0.0f;
+    for (int i = 0; i < LOSS_WARPS; i++) l += part[i];
+    atomicAdd(loss, l * inv);
+  }
 }
 
 // Adam on fp32 master weights [rows x cols]; writes the bf16 copy and its transpose
@@ -301,22 +316,95 @@ __global__ void k_adam(int64_t rows, int64_t cols, float* w, const float* g, flo
   if (wbt) wbt[(i % cols) * rows + i / cols] = __float2bfloat16(wi);
 }
 
-// normalised bf16 features of every column at the start of a solve (first substep)
-__global__ void k_mlp_features(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_config cfg, double dtime,
-                               const float* mean, const float* istd, __nv_bfloat16* X) {
-  const int64_t c = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (c >= nc) return;
-  float x[MLP_IN];
-  const int64_t nl = f.col_nbedrock[c];
-  if (f.mask_hydrology[c] && nl >= 1 && nl <= D.nlevsoi) {
-    const int64_t ld = D.ldc;
-    const int joff = D.nlevsno;
-    column_features(D, f, cfg, c, (int)nl, [&](int j) { return LV(f.h2osoi_liq, c, joff + j, ld); }, dtime,
-                    dtime, x);
-  } else {
-    for (int i = 0; i < MLP_IN; i++) x[i] = 0.0f;
+// Normalised bf16 features of every column at the start of a solve (first substep); zeros
+// before the normalisation where a column has no solve.  A block takes FT_COLS columns as
+// (level, column) items, column fastest, so that the level arrays are read in rows, and
+// writes its rows of X as one range.  A thread per column read the
+// same bytes in 225 us at 131,072 columns (one level's chain of loads after another, 64
+// scattered 2-byte stores); this takes 51 us, bound by the FP64 unit that the
+// double-to-float conversions go through (85 % busy).  In integer instructions the
+// conversions took the same 51 us, then bound by instructions issued.
+constexpr int FT_COLS = 32, FT_PARTS = 10, FT_LD = MLP_IN + 2;   // FT_LD: an odd number of words
+constexpr int FT_PER = FEAT_LEVELS / FT_PARTS;                    // levels of a thread
+static_assert(FEAT_LEVELS % FT_PARTS == 0, "the levels split evenly");
+__global__ void __launch_bounds__(FT_COLS * FT_PARTS)
+k_mlp_features(Dims D, int64_t nc, clmgb_soilwater_fields f, float e_ice, float remaining, float minutes,
+               const float* __restrict__ mean, const float* __restrict__ istd, __nv_bfloat16* X, int words) {
+  __shared__ float sat[FEAT_LEVELS + 2][FT_COLS], root[FEAT_LEVELS + 1][FT_COLS], norm[2][MLP_IN];
+  __shared__ __align__(16) __nv_bfloat16 out[FT_COLS][FT_LD];
+  const int64_t ld = D.ldc, c0 = (int64_t)blockIdx.x * FT_COLS;
+  const int col = threadIdx.x % FT_COLS, part = threadIdx.x / FT_COLS;
+  const int64_t c = c0 + col;
+  if (threadIdx.x < MLP_IN) {
+    norm[0][threadIdx.x] = mean[threadIdx.x];
+    norm[1][threadIdx.x] = istd[threadIdx.x];
   }
-  for (int i = 0; i < MLP_IN; i++) X[c * MLP_IN + i] = __float2bfloat16((x[i] - mean[i]) * istd[i]);
+  // every load of the thread before any of them is used, those of columns without a solve
+  // and of levels below a column's lowest included: whether they count is itself a load
+  uint8_t live = 0;
+  int64_t bed = 0;
+  if (c < nc) {
+    live = f.mask_hydrology[c];
+    bed = f.col_nbedrock[c];
+  }
+  double liq[FT_PER], dz[FT_PER], ws[FT_PER], rt[FT_PER], ice[FT_PER], below[FT_PER], bsw[FT_PER], hksat[FT_PER];
+#pragma unroll
+  for (int i = 0; i < FT_PER; i++) {
+    const int j = 1 + part + i * FT_PARTS;
+    liq[i] = dz[i] = ws[i] = rt[i] = ice[i] = below[i] = bsw[i] = hksat[i] = 0.0;
+    if (c < nc && j <= D.nlevsoi) {
+      liq[i] = LV(f.h2osoi_liq, c, D.nlevsno + j, ld);
+      dz[i] = LVc(f.dz, c, D.nlevsno + j, ld);
+      ws[i] = LVc(f.watsat, c, j, ld);
+      rt[i] = LVc(f.qflx_rootsoi, c, j, ld);
+      ice[i] = LV(f.icefrac, c, j, ld);
+      if (j < D.nlevsoi) below[i] = LV(f.icefrac, c, j + 1, ld);
+      bsw[i] = LVc(f.bsw, c, j, ld);
+      hksat[i] = LVc(f.hksat, c, j, ld);
+    }
+  }
+  const int nl = live && bed >= 1 && bed <= D.nlevsoi ? (int)bed : 0;
+  float sv[FT_PER], xi[FT_PER];
+#pragma unroll
+  for (int i = 0; i < FT_PER; i++) {
+    const int j = 1 + part + i * FT_PARTS;
+    const bool in = j <= nl;
+    sv[i] = in ? feature_saturation(liq[i], dz[i], ws[i]) : 0.0f;
+    xi[i] = in ? (float)ice[i] : 0.0f;
+    sat[j][col] = sv[i];
+    root[j][col] = in ? (float)rt[i] : 0.0f;
+  }
+  if (part == 0) sat[FEAT_LEVELS + 1][col] = 0.0f;
+  __syncthreads();
+  auto put = [&](int i, float x) { out[col][i] = __float2bfloat16((x - norm[0][i]) * norm[1][i]); };
+#pragma unroll
+  for (int i = 0; i < FT_PER; i++) {
+    const int j = 1 + part + i * FT_PARTS;
+    float xc = nl ? -30.0f : 0.0f;
+    if (j <= nl)
+      xc = feature_log_conductivity(j == nl, sv[i], sat[j + 1][col], ice[i], below[i], bsw[i], hksat[i], e_ice);
+    put(j - 1, sv[i]);
+    put(19 + j, xi[i]);
+    put(39 + j, xc);
+  }
+  if (part == 0) {
+    float sink = 0.0f;
+    for (int j = 1; j <= FEAT_LEVELS && j <= nl; j++) sink += root[j][col];
+    put(60, nl ? (float)(f.qflx_infl[c] * 1.0e3) : 0.0f);
+    put(61, nl ? sink * 1.0e3f : 0.0f);
+    put(62, nl ? remaining : 0.0f);
+    put(63, nl ? log2f(minutes) / 6.0f : 0.0f);
+  }
+  __syncthreads();
+  const int rows = (int)(nc - c0 < FT_COLS ? nc - c0 : FT_COLS);
+  if (words) {                                      // X on a 4-byte boundary
+    uint32_t* X32 = reinterpret_cast<uint32_t*>(X + c0 * MLP_IN);
+    for (int i = threadIdx.x; i < rows * MLP_IN / 2; i += FT_COLS * FT_PARTS)
+      X32[i] = *reinterpret_cast<const uint32_t*>(&out[i / (MLP_IN / 2)][i % (MLP_IN / 2) * 2]);
+  } else {
+    for (int i = threadIdx.x; i < rows * MLP_IN; i += FT_COLS * FT_PARTS)
+      X[c0 * MLP_IN + i] = out[i / MLP_IN][i % MLP_IN];
+  }
 }
 
 // first substep = dtime / 2^k, k = clamp(ceil(y0 - margin), 0, kmax)
@@ -386,7 +474,8 @@ cudaError_t launch_mlp_silu_backward(int64_t n, const float* Z, const void* dY, 
 cudaError_t launch_mlp_loss(int64_t M, const float* Y, const float* T, float w0, float w1, float* loss, void* dY,
                             cudaStream_t s) {
   if (M <= 0) return cudaSuccess;
-  k_mlp_loss<<<(unsigned int)((M + 127) / 128), 128, 0, s>>>(M, Y, T, w0, w1, loss, (__nv_bfloat16*)dY);
+  constexpr int rows = LOSS_WARPS * LOSS_ROWS;
+  k_mlp_loss<<<(unsigned int)((M + rows - 1) / rows), 32 * LOSS_WARPS, 0, s>>>(M, Y, T, w0, w1, loss, (__nv_bfloat16*)dY);
   return cudaGetLastError();
 }
 
@@ -411,8 +500,9 @@ cudaError_t launch_richards_samples(const Dims& D, int64_t nc, const clmgb_soilw
 cudaError_t launch_mlp_features(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,
                                 const clmgb_swm_config& cfg, double dtime, const float* mean, const float* istd,
                                 void* X, cudaStream_t s) {
-  k_mlp_features<<<(unsigned int)((nc + 127) / 128), 128, 0, s>>>(D, nc, f, cfg, dtime, mean, istd,
-                                                                  (__nv_bfloat16*)X);
+  k_mlp_features<<<(unsigned int)((nc + FT_COLS - 1) / FT_COLS), FT_COLS * FT_PARTS, 0, s>>>(
+      D, nc, f, (float)cfg.e_ice, (float)(dtime / dtime), (float)(dtime / 60.0), mean, istd, (__nv_bfloat16*)X,
+      ((uintptr_t)X & 3) == 0);
   return cudaGetLastError();
 }
 

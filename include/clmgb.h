@@ -1125,6 +1125,48 @@ int32_t clmgb_mlp_adam(clmgb_handle h, int64_t rows, int64_t cols, float* w, con
                        float* v, float lr, float beta1, float beta2, float eps, int32_t step,
                        uint16_t* w_bf16, uint16_t* wt_bf16, void* stream);
 
+/* The network's parameters: layer i (0..2) has FP32 master weights w[i] [out x in] and
+ * biases b[i], the BF16 copy wb[i], its transpose wt[i] [in x out], and Adam's moments
+ * (mw, vw of the weights, mb, vb of the biases).  A call reads only the members that its
+ * comment names; the others may be NULL. */
+typedef struct clmgb_mlp_net {
+  int64_t struct_size;
+  float* w[3];
+  float* b[3];
+  uint16_t* wb[3];
+  uint16_t* wt[3];
+  float* mw[3];
+  float* vw[3];
+  float* mb[3];
+  float* vb[3];
+} clmgb_mlp_net;
+
+/* FP32 gradients of the weights and biases. */
+typedef struct clmgb_mlp_grad {
+  int64_t struct_size;
+  float* dw[3];
+  float* db[3];
+} clmgb_mlp_grad;
+
+/* The three layers in one launch: Y [M x 32] FP32 = the outputs of X [M x 64] BF16, the
+ * same bits as three clmgb_mlp_linear calls.  Z1, H1, Z2, H2 [M x 128] (FP32
+ * pre-activations and BF16 activations, what clmgb_mlp_gradients reads) are all given or
+ * all NULL.  Reads wb and b.  Arrays start on 16-byte boundaries (CLMGB_ERR_UNSUPPORTED
+ * otherwise). */
+int32_t clmgb_mlp_forward(clmgb_handle h, int64_t M, const uint16_t* X, const clmgb_mlp_net* net, float* Z1,
+                          uint16_t* H1, float* Z2, uint16_t* H2, float* Y, void* stream);
+
+/* The backward pass of clmgb_mlp_forward in one launch: grad = the gradients for the output
+ * gradient dY [M x 32] BF16 (overwritten, not added to).  Reads wt[1] and wt[2].  Arrays
+ * start on 16-byte boundaries, but those of db on their own. */
+int32_t clmgb_mlp_gradients(clmgb_handle h, int64_t M, const uint16_t* X, const float* Z1, const uint16_t* H1,
+                            const float* Z2, const uint16_t* H2, const uint16_t* dY, const clmgb_mlp_net* net,
+                            const clmgb_mlp_grad* grad, void* stream);
+
+/* clmgb_mlp_adam on all parameters in one launch.  wb and wt may be NULL. */
+int32_t clmgb_mlp_adam_net(clmgb_handle h, const clmgb_mlp_net* net, const clmgb_mlp_grad* grad, float lr,
+                           float beta1, float beta2, float eps, int32_t step, void* stream);
+
 /* Normalised BF16 features [nc x 64] of every column at the start of a solve
  * ((x - mean) * istd per feature). */
 int32_t clmgb_mlp_features(clmgb_handle h, const clmgb_bounds* b, const clmgb_soilwater_fields* f,
