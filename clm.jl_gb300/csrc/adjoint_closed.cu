@@ -35,9 +35,11 @@
 //
 // With a substep log (clmgb_substep_log, written by clmgb_column_step_logged) the
 // Richards forward is not run again: its accepted substeps' starting water comes
-// from the log, and so do the solve's outputs.  Without one (or for a column the
-// log could not hold) the substep loop runs on values here, keeping the same
-// checkpoints in the reserved per-slot storage.
+// from the log, and so do the solve's outputs; with the soil_temperature! records
+// too, the solve is reversed beforehand by a kernel with a thread per level
+// (k_richards_reverse, adjoint_richards_packed.cu).  Without a log (or for a column
+// the log could not hold) the substep loop runs on values here, keeping the same
+// checkpoints in the reserved per-slot storage, and is reversed here.
 #include "adjoint_richards.cuh"
 #include "clmgb_device.cuh"
 #include "launch.h"
@@ -831,7 +833,6 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
   const int nw = nlevsno + nlevgrnd;
   const int joff = nlevsno;
   const int64_t slot = (int64_t)blockIdx.x * CF_BLOCK + threadIdx.x;
-  const double LN10 = cm_log(10.0);
   CfBand band;
   for (;;) {
     const int64_t k = (int64_t)atomicAdd(queue, 1ULL);
@@ -913,19 +914,24 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
     bool rich = false;
     int nacc = 0;
     const double* logc = nullptr;     // this column's log region, when it holds the solve
+    // k_richards_reverse has reversed the solve: adj holds the adjoints before it
+    const bool reversed = do_w && richards_reversed_here(D, ft, fw, lg, c);
+    const int32_t cnt = do_w && lg.rec ? lg.count[c] : -1;
     if (do_w) {
-      water_fractions_col(D, fw, c, V);
-      rich = mf_begin(L, D, fw, cfg, dtime, c, V);
-      if (!rich) {
+      if (!reversed) {
+        water_fractions_col(D, fw, c, V);
+        rich = mf_begin(L, D, fw, cfg, dtime, c, V);
+      }
+      if (!reversed && !rich) {
         st |= L.status;
       } else {
-        const int32_t cnt = lg.rec ? lg.count[c] : -1;
-        if (cnt >= 0 && cnt <= lg.cap) {
+        if (reversed || (cnt >= 0 && cnt <= lg.cap)) {
           logc = lg.rec + c * lg.stride;
           nacc = cnt;
           const double* fin = logc + (int64_t)lg.cap * SUB_REC;
           uint32_t rs = (uint32_t)fin[3 * MAXSOI + 2];
-          for (int j = 1; j <= L.nlayers; j++) {
+          const int nl = (int)fw.col_nbedrock[c];
+          for (int j = 1; j <= nl; j++) {
             V.liq[joff + j] = fin[j - 1];
             LV(fw.smp_l, c, j, ld) = fin[MAXSOI + j - 1];
             LV(fw.hk_l, c, j, ld) = fin[2 * MAXSOI + j - 1];
@@ -960,7 +966,7 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
       LV(ft.h2osoi_ice, c, jj, ld) = V.ice[jj];
       if (do_t) LV(ft.fact, c, jj, ld) = V.fact[jj];
     }
-    if (do_w)
+    if (do_w && !reversed)
       for (int j = 1; j <= nlevsoi; j++) LV(fw.icefrac, c, j, ld) = V.icefrac[j];
     ft.t_grnd[c] = V.tg;
     ft.t_h2osfc[c] = V.th;
@@ -975,13 +981,12 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
         iceb[jj] = LV(adj.lam_h2osoi_ice, c, jj, ld);
       }
       double tgb = adj.lam_t_grnd[c], thb = adj.lam_t_h2osfc[c], forcb = 0.0;
-      double wsb[MAXGRND + 2], bsb[MAXGRND + 2], sucb[MAXGRND + 2], ksb[MAXSOI + 2];
+      double wsb[MAXGRND + 2], bsb[MAXGRND + 2], sucb[MAXGRND + 2];
       for (int j = 1; j <= nlevgrnd; j++) {
         wsb[j] = 0.0;
         bsb[j] = 0.0;
         sucb[j] = 0.0;
       }
-      for (int j = 1; j <= nlevsoi; j++) ksb[j] = 0.0;
       // ---- the substeps in reverse ----
       if (rich) {
         const int nl = L.nlayers;
@@ -991,7 +996,7 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
         RichardsBar RB;
         for (int j = 1; j <= nl; j++) {
           lamL[j] = liqb[joff + j];
-          RB.ws[j] = 0.0; RB.b[j] = 0.0; RB.suc[j] = 0.0; RB.ks[j] = 0.0; RB.imp[j] = 0.0;
+          RB.ws[j] = 0.0; RB.b[j] = 0.0; RB.e[j] = 0.0; RB.suc[j] = 0.0; RB.hp[j] = 0.0;
           wsv[j] = LV(fw.watsat, c, j, ld);
           bbv[j] = LV(fw.bsw, c, j, ld);
           sucv[j] = LV(fw.sucsat, c, j, ld);
@@ -1009,39 +1014,18 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
           }
           mf_substep_reverse(D, fw, cfg, dtime, c, nl, L.dzv, L.imp, wsv, bbv, sucv, ksv, dts, liqs, lamL, lamQ, RB);
         }
+        // the ice impedance 10^(-e_ice icefrac) and set_soil_water_fractions!
+        double half_above = 0.0;
         for (int j = 1; j <= nl; j++) {
+          const double ib = rv_impedance_bar(cfg.e_ice, RB.hp[j], ksv[j], L.imp[j]);
+          iceb[j + joff] += rv_fractions_reverse(ib, half_above, j == nl, wsv[j], V.ice[j + joff],
+                                                 LV(ft.excess_ice, c, j, ld), LVc(fw.dz, c, j + joff, ld), RB.ws[j]);
+          half_above = 0.5 * ib;
           liqb[joff + j] = lamL[j];
-          wsb[j] += RB.ws[j];
-          bsb[j] += RB.b[j];
-          sucb[j] += RB.suc[j];
-          ksb[j] += RB.ks[j];
-        }
-        // ice impedance 10^(-e_ice icef) and set_soil_water_fractions!
-        double icefb[MAXSOI + 2];
-        for (int j = 1; j <= nl + 1; j++) icefb[j] = 0.0;
-        for (int j = 1; j <= nl; j++) {
-          const double ib = -cfg.e_ice * (RB.imp[j] * L.imp[j] * LN10);
-          if (j == nl) {
-            icefb[j] += ib;
-          } else {
-            icefb[j] += 0.5 * ib;
-            icefb[j + 1] += 0.5 * ib;
-          }
-        }
-        for (int j = 1; j <= nl; j++) {
-          if (icefb[j] == 0.0) continue;
-          const double exi = LV(ft.excess_ice, c, j, ld);
-          const double dz_ext = LVc(fw.dz, c, j + joff, ld) + jl_div(exi, DENICE);
-          const double ws = wsv[j];
-          const double y = jl_div(V.ice[j + joff] + exi, dz_ext * DENICE);
-          const double vol_ice = jl_min(ws, y);
-          const double v = jl_div(vol_ice, ws);
-          const double icef = jl_min(1.0, v);
-          if (same_bits(icef, 1.0)) continue;
-          wsb[j] -= icefb[j] * v / ws;
-          const double vb = icefb[j] / ws;
-          if (same_bits(vol_ice, ws)) wsb[j] += vb;
-          else iceb[j + joff] += vb / (dz_ext * DENICE);
+          if (adj.grad_watsat) LV(adj.grad_watsat, c, j, ld) += RB.ws[j];
+          if (adj.grad_bsw) LV(adj.grad_bsw, c, j, ld) += rv_fma(2.0, RB.e[j], RB.b[j]);
+          if (adj.grad_sucsat) LV(adj.grad_sucsat, c, j, ld) += RB.suc[j];
+          if (adj.grad_hksat) LV(adj.grad_hksat, c, j, ld) += RB.hp[j] * L.imp[j];
         }
       }
       // ---- soil_temperature! in reverse ----
@@ -1061,7 +1045,6 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
         if (adj.grad_watsat) LV(adj.grad_watsat, c, j, ld) += wsb[j];
         if (adj.grad_bsw) LV(adj.grad_bsw, c, j, ld) += bsb[j];
         if (adj.grad_sucsat) LV(adj.grad_sucsat, c, j, ld) += sucb[j];
-        if (adj.grad_hksat) LV(adj.grad_hksat, c, j, ld) += ksb[j];
       }
     }
     if (col_status) col_status[c] = st;
@@ -1143,6 +1126,8 @@ cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soi
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     order = qs.order;
   }
+  if (lg.rec && lg.st && (e = launch_richards_reverse(D, nc, ft, fw, cfg, dtime, adj, lg, order, s)) != cudaSuccess)
+    return e;
   int64_t blocks = grid_blocks;
   const int64_t max_blocks = tp.slots / CF_BLOCK;
   if (blocks > max_blocks) blocks = max_blocks;

@@ -491,7 +491,7 @@ k_column_step_vjp(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_
             double impv[MAXSOI + 1], liqs[MAXSOI + 1];
             double wsv[MAXSOI + 2], bbv[MAXSOI + 2], sucv[MAXSOI + 2], ksv[MAXSOI + 2];
             for (int j = 1; j <= LA.nlayers; j++) {
-              RB.ws[j] = 0.0; RB.b[j] = 0.0; RB.suc[j] = 0.0; RB.ks[j] = 0.0; RB.imp[j] = 0.0;
+              RB.ws[j] = 0.0; RB.b[j] = 0.0; RB.e[j] = 0.0; RB.suc[j] = 0.0; RB.hp[j] = 0.0;
               impv[j] = LA.imp[j].v;
               wsv[j] = X.watsat[j].v;
               bbv[j] = X.bsw[j].v;
@@ -505,10 +505,10 @@ k_column_step_vjp(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_
             }
             for (int j = 1; j <= LA.nlayers; j++) {
               adj_add(X.watsat[j].i, RB.ws[j]);
-              adj_add(X.bsw[j].i, RB.b[j]);
+              adj_add(X.bsw[j].i, rv_fma(2.0, RB.e[j], RB.b[j]));
               adj_add(X.sucsat[j].i, RB.suc[j]);
-              adj_add(X.hksat[j].i, RB.ks[j]);
-              adj_add(LA.imp[j].i, RB.imp[j]);
+              adj_add(X.hksat[j].i, RB.hp[j] * impv[j]);
+              adj_add(LA.imp[j].i, RB.hp[j] * ksv[j]);
             }
           } else {
             for (int sidx = nacc - 1; sidx >= 0; sidx--) {

@@ -205,6 +205,10 @@ cudaError_t launch_colbalance(int64_t nc, const clmgb_colbalance_fields& f, doub
 cudaError_t launch_soil_fluxes(const Dims& D, int64_t nc, int64_t nl, const clmgb_soilflux_fields& f, double dtime,
                                uint32_t* dev_status, cudaStream_t s);
 int vjp_cf_blocks_per_sm();
+cudaError_t launch_richards_reverse(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,
+                                    const clmgb_soilwater_fields& fw, const clmgb_swm_config& cfg, double dtime,
+                                    const clmgb_step_adjoint& adj, const SubstepLogView& lg, const uint32_t* order,
+                                    cudaStream_t s);
 cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,
                                       const clmgb_soilwater_fields& fw, const clmgb_swm_config& cfg, double dtime,
                                       int snow_method, double* t_ssbef, double* t_h2osfc_bef,
