@@ -43,6 +43,7 @@
 #include "adjoint_richards.cuh"
 #include "clmgb_device.cuh"
 #include "launch.h"
+#include "work_order.cuh"
 
 namespace clmgb {
 
@@ -1053,54 +1054,31 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
 }
 
 // Work order of the adjoint: the 32 columns a warp runs side by side should take
-// the same paths, so columns are handed out sorted (counting sort, descending) on
-// a key of the Richards work (accepted substeps from the log, else the previous
-// call's attempt count) and the number of snow layers.  Columns the step leaves
-// alone sort last.  The order does not change any result.
-constexpr int VJP_BINS = 64;
-__device__ __forceinline__ int vjp_key(const clmgb_soiltemp_fields& ft, const clmgb_soilwater_fields& fw,
-                                       const SubstepLogView& lg, int64_t c) {
-  if (!ft.mask_nolakec[c] && !fw.mask_hydrology[c]) return 0;
-  int a;
-  if (lg.rec) {
-    const int32_t n = lg.count[c];
-    a = n < 0 ? 0 : (n > lg.cap ? 15 : n);
-  } else {
-    const double ns = fw.num_substeps[c];
-    a = ns > 0.0 ? (ns >= 15.0 ? 15 : (int)ns) : 0;
+// the same paths, so the key is the Richards work (accepted substeps from the log, else
+// the previous call's attempt count) and the number of snow layers.  Columns the step
+// leaves alone come last.
+struct VjpKey {
+  clmgb_soiltemp_fields ft;
+  clmgb_soilwater_fields fw;
+  SubstepLogView lg;
+  __device__ int operator()(int64_t c) const {
+    if (!ft.mask_nolakec[c] && !fw.mask_hydrology[c]) return 0;
+    int a;
+    if (lg.rec) {
+      const int32_t n = lg.count[c];
+      a = n < 0 ? 0 : (n > lg.cap ? 15 : n);
+    } else {
+      const double ns = fw.num_substeps[c];
+      a = ns > 0.0 ? (ns >= 15.0 ? 15 : (int)ns) : 0;
+    }
+    if (a > 15) a = 15;
+    const int64_t snl = ft.col_snl[c];
+    int sb = (int)((-snl + 3) / 4);
+    sb = sb < 0 ? 0 : (sb > 3 ? 3 : sb);
+    return a * 4 + sb;
   }
-  if (a > 15) a = 15;
-  const int64_t snl = ft.col_snl[c];
-  int sb = (int)((-snl + 3) / 4);
-  sb = sb < 0 ? 0 : (sb > 3 ? 3 : sb);
-  return a * 4 + sb;
-}
-__global__ void k_vjp_hist(int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fields fw, SubstepLogView lg,
-                           unsigned int* bins) {
-  __shared__ unsigned int sh[VJP_BINS];
-  for (int i = threadIdx.x; i < VJP_BINS; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < nc) atomicAdd(&sh[vjp_key(ft, fw, lg, c)], 1u);
-  __syncthreads();
-  for (int i = threadIdx.x; i < VJP_BINS; i += blockDim.x)
-    if (sh[i]) atomicAdd(&bins[i], sh[i]);
-}
-__global__ void k_vjp_scan(unsigned int* bins) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned int run = 0;
-  for (int b = VJP_BINS - 1; b >= 0; b--) {
-    bins[VJP_BINS + b] = run;
-    run += bins[b];
-  }
-}
-__global__ void k_vjp_scatter(int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fields fw, SubstepLogView lg,
-                              unsigned int* bins, uint32_t* order) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const unsigned int pos = atomicAdd(&bins[VJP_BINS + vjp_key(ft, fw, lg, c)], 1u);
-  order[pos] = (uint32_t)c;
-}
+  __device__ void unlisted(int64_t) const {}
+};
 
 int vjp_cf_blocks_per_sm() {
   int nb = 0;
@@ -1118,12 +1096,7 @@ cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soi
   if (e != cudaSuccess) return e;
   const uint32_t* order = nullptr;
   if (qs.capacity >= nc && qs.order && qs.bins && nc < (int64_t)0xffffffffLL) {
-    const unsigned g = (unsigned)((nc + 127) / 128);
-    if ((e = cudaMemsetAsync(qs.bins, 0, 2 * VJP_BINS * sizeof(unsigned int), s)) != cudaSuccess) return e;
-    k_vjp_hist<<<g, 128, 0, s>>>(nc, ft, fw, lg, qs.bins);
-    k_vjp_scan<<<1, 32, 0, s>>>(qs.bins);
-    k_vjp_scatter<<<g, 128, 0, s>>>(nc, ft, fw, lg, qs.bins, qs.order);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_order(nc, VjpKey{ft, fw, lg}, qs.bins, qs.order, s)) != cudaSuccess) return e;
     order = qs.order;
   }
   if (lg.rec && lg.st && (e = launch_richards_reverse(D, nc, ft, fw, cfg, dtime, adj, lg, order, s)) != cudaSuccess)

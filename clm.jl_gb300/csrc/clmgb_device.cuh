@@ -1442,15 +1442,14 @@ __device__ inline uint32_t moisture_form_col(const Dims& D, const clmgb_soilwate
 // is zero and the recharge written is a signed zero, for every column whose water table
 // lies within the soil column (jwt < nlevsoi); the other columns keep the solve's qcharge.
 // ===========================================================================
-// jwt: the number of soil levels above the water table (:1177-1184)
+// jwt: the number of soil levels above the water table (:1177-1184).  From the bottom up
+// without leaving early, so that the levels' loads do not wait for one another.
 __device__ __forceinline__ int watertable_level(const Dims& D, const clmgb_soilwater_fields& f, int64_t c) {
   int jwt = D.nlevsoi;
-  for (int j = 1; j <= D.nlevsoi; j++) {
-    if (f.zwt[c] <= LVc(f.zi, c, D.nlevsno + 1 + j, D.ldc)) {
-      jwt = j - 1;
-      break;
-    }
-  }
+  const double zwt = f.zwt[c];
+#pragma unroll 5
+  for (int j = D.nlevsoi; j >= 1; j--)
+    if (zwt <= LVc(f.zi, c, D.nlevsno + 1 + j, D.ldc)) jwt = j - 1;
   return jwt;
 }
 
@@ -1473,10 +1472,10 @@ __device__ inline bool compute_qcharge_col(const Dims& D, const clmgb_soilwater_
   const int jp = jwt + 1;
   const double zwt = f.zwt[c];
   const double wh_zwt = -LVc(f.sucsat, c, jp, ld) - zwt * M_TO_MM;
-  const double vwc = jp <= nlayers ? jl_max(LV(f.h2osoi_liq, c, joff + jp, ld), 1.0e-6) /
-                                         (LVc(f.dz, c, joff + jp, ld) * DENH2O)
+  const double vwc = jp <= nlayers ? jl_div(jl_max(LV(f.h2osoi_liq, c, joff + jp, ld), 1.0e-6),
+                                                LVc(f.dz, c, joff + jp, ld) * DENH2O)
                                    : 0.0;
-  double s1 = jl_max(vwc / LVc(f.watsat, c, jp, ld), 0.01);
+  double s1 = jl_max(jl_div(vwc, LVc(f.watsat, c, jp, ld)), 0.01);
   s1 = jl_min(1.0, s1);
   const double imped = 0.0, smp = 0.0;   // the zeroed scratch rows the reference passes
   const double b = LVc(f.bsw, c, jp, ld);
@@ -1486,11 +1485,11 @@ __device__ inline bool compute_qcharge_col(const Dims& D, const clmgb_soilwater_
   const double wh = smp1 - LVc(f.z, c, joff + jm, ld) * M_TO_MM;
   double q;
   if (jwt == 0)
-    q = -ka * (wh_zwt - wh) / ((zwt + 1.0e-3) * M_TO_MM);
+    q = jl_div(-ka * (wh_zwt - wh), (zwt + 1.0e-3) * M_TO_MM);
   else
-    q = -ka * (wh_zwt - wh) / ((zwt - LVc(f.z, c, joff + jwt, ld)) * M_TO_MM * 2.0);
-  q = jl_max(-10.0 / dtime, q);
-  q = jl_min(10.0 / dtime, q);
+    q = jl_div(-ka * (wh_zwt - wh), (zwt - LVc(f.z, c, joff + jwt, ld)) * M_TO_MM * 2.0);
+  q = jl_max(jl_div(-10.0, dtime), q);
+  q = jl_min(jl_div(10.0, dtime), q);
   f.qcharge[c] = q;
   return true;
 }

@@ -1,6 +1,7 @@
 // kernels.cu — CUDA kernels of the soil/snow column solve (one thread per column).
 #include "clmgb_device.cuh"
 #include "launch.h"
+#include "work_order.cuh"
 #include "richards_coop.cuh"
 
 namespace clmgb {
@@ -14,11 +15,13 @@ __device__ __forceinline__ void report(uint32_t st, uint32_t* col_status, uint32
   if (st && dev_status) atomicOr(dev_status, st);
 }
 
+// a thread per column and level (a thread per column: 17 us at 1,024 columns, a chain of 20
+// levels' divisions; this, 2.6)
 __global__ void __launch_bounds__(BLOCK)
 k_water_fractions(Dims D, int64_t nc, clmgb_soilwater_fields f) {
   const int64_t c = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (c >= nc) return;
-  if (f.mask_hydrology[c]) water_fractions_col(D, f, c);
+  if (f.mask_hydrology[c]) water_fractions_level(D, f, c, 1 + (int)blockIdx.y);
 }
 
 __global__ void __launch_bounds__(BLOCK)
@@ -244,49 +247,23 @@ k_impedance(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, double* 
   for (int j = 1; j <= nlayers; j++) imp_cache[(int64_t)(j - 1) * ld_imp + c] = mf_impedance(D, f, e_ice, c, j, nlayers);
 }
 
-// Longest-expected-first order of the hydrology columns: counting sort on the
-// previous call's substep count (num_substeps, the state field), descending.
-// Bins 0..63; NaN or non-positive counts go to bin 0.  The order within a bin is
-// arbitrary and does not affect any result.
-constexpr int ORDER_BINS = 64;
-__device__ __forceinline__ int order_bin(double ns) {
-  if (!(ns > 0.0)) return 0;
-  return ns >= (double)(ORDER_BINS - 1) ? ORDER_BINS - 1 : (int)ns;
-}
-__global__ void __launch_bounds__(BLOCK)
-k_order_hist(int64_t nc, const uint8_t* mask, const double* num_substeps, unsigned int* bins) {
-  __shared__ unsigned int sh[ORDER_BINS];
-  for (int i = threadIdx.x; i < ORDER_BINS; i += BLOCK) sh[i] = 0;
-  __syncthreads();
-  const int64_t c = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
-  if (c < nc && mask[c]) atomicAdd(&sh[order_bin(num_substeps[c])], 1u);
-  __syncthreads();
-  for (int i = threadIdx.x; i < ORDER_BINS; i += BLOCK)
-    if (sh[i]) atomicAdd(&bins[i], sh[i]);
-}
-// bins[0..63] counts -> bins[64+b] start offset of bin b (descending bins first),
-// bins[128] = total listed
-__global__ void k_order_scan(unsigned int* bins) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned int run = 0;
-  for (int b = ORDER_BINS - 1; b >= 0; b--) {
-    bins[ORDER_BINS + b] = run;
-    run += bins[b];
+// Longest-expected-first order of the hydrology columns: the key is the previous call's
+// substep count (num_substeps, the state field); NaN or non-positive counts are key 0.
+struct SubstepKey {
+  const uint8_t* mask;
+  const double* num_substeps;
+  uint32_t* col_status;
+  int or_status;
+  __device__ int operator()(int64_t c) const {
+    if (!mask[c]) return -1;
+    const double ns = num_substeps[c];
+    if (!(ns > 0.0)) return 0;
+    return ns >= (double)(ORDER_BINS - 1) ? ORDER_BINS - 1 : (int)ns;
   }
-  bins[2 * ORDER_BINS] = run;
-}
-__global__ void __launch_bounds__(BLOCK)
-k_order_scatter(int64_t nc, const uint8_t* mask, const double* num_substeps, unsigned int* bins, uint32_t* order,
-                uint32_t* col_status, int or_status) {
-  const int64_t c = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
-  if (c >= nc) return;
-  if (!mask[c]) {
+  __device__ void unlisted(int64_t c) const {
     if (col_status && !or_status) col_status[c] = 0;
-    return;
   }
-  const unsigned int slot = atomicAdd(&bins[ORDER_BINS + order_bin(num_substeps[c])], 1u);
-  order[slot] = (uint32_t)c;
-}
+};
 
 // Evaluates the shared transcendentals (clm_math.h) elementwise; op 0 log, 1 exp,
 // 2 pow, 3 log10.  Used to check that GPU and CPU builds return identical bits.
@@ -585,7 +562,7 @@ k_synth_forcing(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fi
 
 // ---------------------------------------------------------------------------
 cudaError_t launch_water_fractions(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, cudaStream_t s) {
-  k_water_fractions<<<grid_for(nc), BLOCK, 0, s>>>(D, nc, f);
+  k_water_fractions<<<dim3((unsigned)grid_for(nc), (unsigned)D.nlevsoi), BLOCK, 0, s>>>(D, nc, f);
   return cudaGetLastError();
 }
 cudaError_t launch_moisture_form(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,
@@ -630,12 +607,8 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (qs.longest_first) {
-      if ((e = cudaMemsetAsync(qs.bins, 0, (2 * ORDER_BINS + 1) * sizeof(unsigned int), s)) != cudaSuccess) return e;
-      k_order_hist<<<grid_for(nc), BLOCK, 0, s>>>(nc, f.mask_hydrology, f.num_substeps, qs.bins);
-      k_order_scan<<<1, 32, 0, s>>>(qs.bins);
-      k_order_scatter<<<grid_for(nc), BLOCK, 0, s>>>(nc, f.mask_hydrology, f.num_substeps, qs.bins, qs.order,
-                                                     col_status, or_status);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      const SubstepKey key = {f.mask_hydrology, f.num_substeps, col_status, or_status};
+      if ((e = launch_order(nc, key, qs.bins, qs.order, s)) != cudaSuccess) return e;
     }
   }
   const int64_t need = (nc + BLOCK - 1) / BLOCK;

@@ -147,7 +147,8 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
     const int nlayers = (int)nl;
     // mf_impedance (soil_water_movement.jl:1287-1293)
     const double icef = (j == nlayers) ? TL(RI_ICEF, j, cl) : 0.5 * (TL(RI_ICEF, j, cl) + TL(RI_ICEF, j + 1, cl));
-    const double imp = cm_pow(10.0, -e_ice * icef);
+    const double y = -e_ice * icef;
+    const double imp = zero_bits(y) ? 1.0 : cm_pow(10.0, y);       // no ice: x^0
     imp_cache[(int64_t)(j - 1) * ld_imp + c] = imp;
     v[e][PC_DZW] = TL(RI_DZ, j, cl) * DENH2O;
     v[e][PC_WS] = TL(RI_WS, j, cl);
@@ -174,10 +175,8 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
   __syncthreads();
   const int64_t ncols = (nc - c0) < RC_COLS ? (nc - c0) : RC_COLS;
   double* out = pcache + c0 * stride;
-  for (int idx = tid; idx < ncols * rec; idx += RC_THREADS) {
-    const int cl = idx / rec, r = idx % rec;
-    out[(int64_t)cl * stride + r] = out_t[cl * pitch + r];
-  }
+  for (int cl = tid / 32; cl < ncols; cl += RC_THREADS / 32)     // a warp per record
+    for (int r = tid % 32; r < rec; r += 32) out[(int64_t)cl * stride + r] = out_t[cl * pitch + r];
 }
 
 // The post-pass: water, smp_l and hk_l of levels 1..nbedrock of every column the solve
@@ -194,10 +193,8 @@ k_column_outputs(Dims D, int64_t nc, clmgb_soilwater_fields f, const double* pca
   const int part = RO_FIELDS * nls, pitch = part + 1, stride = PC_ALL * nls;
   const int64_t ncols = (nc - c0) < RC_COLS ? (nc - c0) : RC_COLS;
   const double* in = pcache + c0 * stride + PC_LIQ * nls;
-  for (int idx = tid; idx < ncols * part; idx += RC_THREADS) {
-    const int cl = idx / part, r = idx % part;
-    t[cl * pitch + r] = in[(int64_t)cl * stride + r];
-  }
+  for (int cl = tid / 32; cl < ncols; cl += RC_THREADS / 32)
+    for (int r = tid % 32; r < part; r += 32) t[cl * pitch + r] = in[(int64_t)cl * stride + r];
   __syncthreads();
   for (int idx = tid; idx < RO_FIELDS * nls * RC_COLS; idx += RC_THREADS) {
     const int k = idx / (nls * RC_COLS), rem = idx % (nls * RC_COLS);
