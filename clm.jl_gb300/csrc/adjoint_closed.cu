@@ -41,6 +41,7 @@
 // the log could not hold) the substep loop runs on values here, keeping the same
 // checkpoints in the reserved per-slot storage, and is reversed here.
 #include "adjoint_richards.cuh"
+#include "adjoint_soil.cuh"
 #include "clmgb_device.cuh"
 #include "launch.h"
 #include "work_order.cuh"
@@ -48,18 +49,6 @@
 namespace clmgb {
 
 constexpr int CF_BLOCK = 64;
-
-// The factorisation of the column's band system: lu/x/piv point at the thread's own
-// storage (soil_temperature! run here) or at the column's soil_temperature! record.
-struct CfBand {
-  int n;
-  const double* lu;
-  const double* x;
-  const uint8_t* piv;
-  double lu_s[MAXROWS * 7];
-  double x_s[MAXROWS];
-  uint8_t piv_s[MAXROWS];
-};
 
 // The column's active state in per-thread storage, values only.
 struct CfState {
@@ -95,718 +84,6 @@ struct CfState {
   }
 };
 
-__device__ __forceinline__ bool same_bits(double a, double b) {
-  return __double_as_longlong(a) == __double_as_longlong(b);
-}
-
-// ---------------------------------------------------------------------------
-// Phase change of one level (snow or soil), reversed.  T0: the temperature the
-// band solve left, wice0/wliq0: ice and liquid water before the phase change,
-// fct: the level's fact.  In: the adjoints of the level's temperature, liquid
-// water and ice after the phase change.  Out (accumulated): the adjoints of T0,
-// wice0, wliq0, fct, dhsdT and the level's watsat, bsw, sucsat (supercooled water).
-// Columns with excess ice or snow without layers are flagged by the caller; their
-// branches are not taken here.
-// ---------------------------------------------------------------------------
-struct PcLevelIn {
-  int j, jtop;
-  double T0, wice0, wliq0, fct, dhsdT, fse, fh, dtime;
-  bool sc_type;
-  double ws, bs, suc, dz;
-};
-
-__device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& in, double Tpc_b, double liqpc_b,
-                                                        double icepc_b, double& T0_b, double& ice0_b,
-                                                        double& liq0_b, double& fct_b, double& dhsdT_b,
-                                                        double& ws_b, double& bs_b, double& suc_b) {
-  const int j = in.j, jtop = in.jtop;
-  const double T0 = in.T0, wice0 = in.wice0, wliq0 = in.wliq0, fct = in.fct, dhsdT = in.dhsdT;
-  const double fse = in.fse, fh = in.fh, dtime = in.dtime;
-  const double wmass0 = wice0 + wliq0 + 0.0;
-  // ---- the melt / freeze decision (:1990-2040) ----
-  int im = 0;
-  double tinc = 0.0;
-  bool sc_on = false;
-  double sc = 0.0, P = 0.0, r = 0.0, e = 0.0, q = 0.0, g = 0.0;
-  if (j <= 0) {
-    if (wice0 > 0.0 && T0 > TFRZ) {
-      im = 1;
-      tinc = TFRZ - T0;
-    } else if (wliq0 > 0.0 && T0 < TFRZ) {
-      im = 2;
-      tinc = TFRZ - T0;
-    }
-  } else {
-    double T = T0;
-    if (wice0 > 0.0 && T0 > TFRZ) {
-      im = 1;
-      tinc = TFRZ - T0;
-      T = TFRZ;
-    }
-    if (in.sc_type && T < TFRZ) {
-      sc_on = true;
-      q = HFUS * (TFRZ - T) / (GRAV * T);
-      g = GRAV * T;
-      const double smp = q * 1000.0;
-      r = smp / in.suc;
-      e = -1.0 / in.bs;
-      P = cm_pow(r, e);
-      sc = in.ws * P;
-      sc *= in.dz * 1000.0;
-    }
-    if (wliq0 > sc && T < TFRZ) {
-      im = 2;
-      tinc = TFRZ - T;
-    }
-  }
-  if (im == 0) {
-    T0_b += Tpc_b;
-    liq0_b += liqpc_b;
-    ice0_b += icepc_b;
-    return;
-  }
-  // ---- hm (:2060-2085) ----
-  double hm;
-  if (j == jtop) {
-    if (j > 0) hm = dhsdT * tinc - tinc / fct;
-    else hm = fse * (dhsdT * tinc - tinc / fct);
-    if (j == 1 && fh != 0.0) hm -= fh * dhsdT * tinc;
-  } else if (j == 1) {
-    hm = (1.0 - fse - fh) * dhsdT * tinc - tinc / fct;
-  } else {
-    if (j < 1) hm = -fse * tinc / fct;
-    else hm = -tinc / fct;
-  }
-  if ((im == 1 && hm < 0.0) || (im == 2 && hm > 0.0)) im = 0;
-  if (im == 0 || !(fabs(hm) > 0.0)) {
-    // the temperature was set to freezing (a constant); the water is unchanged
-    liq0_b += liqpc_b;
-    ice0_b += icepc_b;
-    return;
-  }
-  // ---- new ice and liquid water (:2090-2140) ----
-  const double xm = jl_div(hm * dtime, HFUS);
-  double ice = wice0, heatr = 0.0;
-  int kind = 0;   // 0 ice unchanged, 1 wice0 - xm, 2 constant, 3 wmass0, 4 wmass0 - sc
-  if (xm > 0.0) {
-    const double v = wice0 - xm;
-    ice = jl_max(0.0, v);
-    kind = same_bits(ice, 0.0) ? 2 : 1;
-    heatr = hm - jl_div(HFUS * (wice0 - ice), dtime);
-  } else if (xm < 0.0) {
-    if (j <= 0) {
-      const double a = wmass0, b = wice0 - xm;
-      ice = jl_min(a, b);
-      kind = same_bits(ice, a) ? 3 : 1;
-    } else {
-      if (wmass0 - 0.0 < sc) {
-        ice = 0.0;
-        kind = 2;
-      } else {
-        const double a = wmass0 - 0.0 - sc, b = wice0 - xm;
-        ice = jl_min(a, b);
-        kind = same_bits(ice, a) ? 4 : 1;
-      }
-    }
-    heatr = hm - jl_div(HFUS * (wice0 - ice), dtime);
-  }
-  const double liqv = wmass0 - ice - 0.0;
-  const double liq = jl_max(0.0, liqv);
-  const bool liq_pass = !same_bits(liq, 0.0);
-  // ---- reverse (derivative coefficients with reciprocals) ----
-  double heatr_b = 0.0, hm_b = 0.0, xm_b = 0.0, ice_b = icepc_b, wmass0_b = 0.0, wice0_b = 0.0, sc_b = 0.0;
-  double tinc_b = 0.0;
-  const double rf = 1.0 / fct;
-  if (fabs(heatr) > 0.0 && !(j <= 0 && liq * ice > 0.0)) {
-    // temperature correction (:2145-2165); the level starts from freezing
-    if (j == 1) {
-      const double k = (j == jtop) ? (1.0 - fh) : (1.0 - fse - fh);
-      const double rden = 1.0 / (1.0 - k * fct * dhsdT);
-      const double incr = fct * heatr * rden;
-      const double N_b = Tpc_b * rden, den_b = -Tpc_b * incr * rden;
-      fct_b += N_b * heatr - den_b * k * dhsdT;
-      heatr_b += N_b * fct;
-      dhsdT_b += -den_b * k * fct;
-    } else if (j == jtop) {      // top snow layer
-      if (fse > 0.0) {
-        const double rfse = 1.0 / fse;
-        const double rden = 1.0 / (1.0 - fct * dhsdT);
-        const double incr = fct * rfse * heatr * rden;
-        const double N_b = Tpc_b * rden, den_b = -Tpc_b * incr * rden;
-        fct_b += N_b * heatr * rfse - den_b * dhsdT;
-        heatr_b += N_b * fct * rfse;
-        dhsdT_b += -den_b * fct;
-      }
-    } else if (j > 0) {
-      fct_b += Tpc_b * heatr;
-      heatr_b += Tpc_b * fct;
-    } else if (fse > 0.0) {
-      const double rfse = 1.0 / fse;
-      fct_b += Tpc_b * heatr * rfse;
-      heatr_b += Tpc_b * fct * rfse;
-    }
-  }
-  if (liq_pass) {
-    wmass0_b += liqpc_b;
-    ice_b -= liqpc_b;
-  }
-  if (xm != 0.0) {
-    hm_b += heatr_b;
-    const double d_b = -heatr_b * HFUS * (1.0 / dtime);
-    wice0_b += d_b;
-    ice_b -= d_b;
-  }
-  switch (kind) {
-    case 0: wice0_b += ice_b; break;
-    case 1: wice0_b += ice_b; xm_b -= ice_b; break;
-    case 3: wmass0_b += ice_b; break;
-    case 4: wmass0_b += ice_b; sc_b -= ice_b; break;
-    default: break;
-  }
-  hm_b += xm_b * dtime * (1.0 / HFUS);
-  // hm
-  if (j == jtop) {
-    const double hb = (j > 0) ? hm_b : hm_b * fse;
-    dhsdT_b += hb * tinc;
-    tinc_b += hb * dhsdT - hb * rf;
-    fct_b += hb * tinc * rf * rf;
-    if (j == 1 && fh != 0.0) {
-      dhsdT_b -= hm_b * fh * tinc;
-      tinc_b -= hm_b * fh * dhsdT;
-    }
-  } else if (j == 1) {
-    const double k = 1.0 - fse - fh;
-    dhsdT_b += hm_b * k * tinc;
-    tinc_b += hm_b * k * dhsdT - hm_b * rf;
-    fct_b += hm_b * tinc * rf * rf;
-  } else {
-    const double a = (j < 1) ? fse : 1.0;     // hm = -a tinc / fct
-    tinc_b -= hm_b * a * rf;
-    fct_b += hm_b * a * tinc * rf * rf;
-  }
-  T0_b -= tinc_b;
-  // supercooled water sc = watsat (smp/sucsat)^(-1/bsw) dz 1000, smp = HFUS (TFRZ-T)/(GRAV T) 1000
-  if (sc_b != 0.0 && sc_on) {
-    const double sc0_b = sc_b * (in.dz * 1000.0);
-    ws_b += sc0_b * P;
-    const double P_b = sc0_b * in.ws;
-    const double rr = 1.0 / r, rsuc = 1.0 / in.suc, rg = 1.0 / g;
-    const double r_b = r != 0.0 ? P_b * e * P * rr : 0.0;
-    const double e_b = r > 0.0 ? P_b * P * cm_log(r) : 0.0;
-    bs_b += e_b * (-e) * (1.0 / in.bs);
-    const double smp_b = r_b * rsuc;
-    suc_b += r_b * (-r) * rsuc;
-    const double q_b = smp_b * 1000.0;
-    const double a_b = q_b * rg;
-    const double g_b = -q_b * q * rg;
-    T0_b += -a_b * HFUS + g_b * GRAV;
-  }
-  ice0_b += wice0_b + wmass0_b;
-  liq0_b += wmass0_b;
-}
-
-// ---------------------------------------------------------------------------
-// soil_temperature! reversed for column c.  The forward left in V the final state
-// and in B the band factors; tin, liq0, ice0, tg0, th0 are the step's inputs.
-// Tb, liqb, iceb, tgb, thb hold on entry the adjoints of the quantities after the
-// call and on return those of its inputs; forcb and wsb/bsb/sucb accumulate.
-// ---------------------------------------------------------------------------
-__device__ __noinline__ void soil_temperature_reverse(const Dims& D, const clmgb_soiltemp_fields& f,
-                                                      const clmgb_soilwater_fields& fw, int64_t c, double dtime,
-                                                      int snow_method, const double* fact, const double* tin,
-                                                      const double* liq0, const double* ice0, double tg0, double th0,
-                                                      double forc, const CfBand& B, double* Tb, double* liqb,
-                                                      double* iceb, double& tgb, double& thb, double& forcb,
-                                                      double* wsb, double* bsb, double* sucb) {
-  const int64_t ld = D.ldc, ldp = D.ldp;
-  const int nlevsno = D.nlevsno, nlevgrnd = D.nlevgrnd;
-  const int joff = nlevsno;
-  const int nw = nlevsno + nlevgrnd;
-  const int64_t snl = f.col_snl[c];
-  const int jtop = (int)snl + 1, jjtop = jtop + joff;
-  const int64_t l = f.col_landunit[c] - 1;
-  const int64_t it = f.col_itype[c];
-  const int64_t lit = f.lun_itype[l];
-  const bool is_special = (lit == ISTWET || lit == ISTICE);
-  const int64_t nbedrock = f.col_nbedrock[c];
-  const double fse = f.frac_sno_eff[c];
-  const double fh = f.frac_h2osfc[c];
-  const double omc = 1.0 - CNFAC;
-  const double LN_TKWAT = cm_log(TKWAT), LN_TKICE = cm_log(TKICE);
-
-  double zz[MAXL + 2], rdzp[MAXL + 2];     // rdzp[jj] = 1 / (z[jj+1] - z[jj])
-  for (int jj = jjtop; jj <= nw; jj++) zz[jj] = LVc(f.z, c, jj, ld);
-  for (int jj = jjtop; jj < nw; jj++) rdzp[jj] = 1.0 / (zz[jj + 1] - zz[jj]);
-
-  // ---- forward values with local partials ----
-  // layer conductivity thk and its partials in liquid water, ice and watsat
-  double thk[MAXL + 2], tl[MAXL + 2], ti[MAXL + 2], tw[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    double v = 0.0, dl = 0.0, di = 0.0, dw = 0.0;
-    if (j >= 1) {
-      if (!is_special) {
-        if (j > nbedrock) {
-          v = THK_BEDROCK;
-        } else {
-          const double liq = liq0[jj], ice = ice0[jj];
-          const double exi = LV(f.excess_ice, c, j, ld);
-          const double dzv = LVc(f.dz, c, jj, ld);
-          const double ws = LVc(fw.watsat, c, j, ld);
-          const double m = dzv * ws;
-          const double satw0 = (jl_div(liq, DENH2O) + jl_div(ice, DENICE) + jl_div(exi, DENICE)) / m;
-          const double satw = jl_min(1.0, satw0);
-          const bool spass = !same_bits(satw, 1.0);
-          if (satw > 1.0e-7) {
-            double dke, ddke;
-            if (tin[jj] >= TFRZ) {
-              const double L = cm_log10(satw) + 1.0;
-              dke = jl_max(0.0, L);
-              ddke = same_bits(dke, 0.0) ? 0.0 : 0.43429448190325182765 * (1.0 / satw);
-            } else {
-              dke = satw;
-              ddke = 1.0;
-            }
-            // derivative coefficients (reciprocals instead of divisions; TKWAT^a TKICE^b
-            // as one exponential)
-            const double rm = 1.0 / m, rdz = 1.0 / dzv;
-            const double a1 = liq * (1.0 / DENH2O) * rdz;
-            const double fl_denom = a1 + (ice + exi) * (1.0 / DENICE) * rdz;
-            const double rfd = 1.0 / fl_denom;
-            const double fl = a1 * rfd;
-            const double tkmg = LVc(f.tkmg, c, j, ld), tkdry = LVc(f.tkdry, c, j, ld);
-            const double dksat = tkmg * cm_exp(ws * (fl * LN_TKWAT + (1.0 - fl) * LN_TKICE));
-            v = dke * dksat + (1.0 - dke) * tkdry;
-            // d satw
-            const double sl = spass ? (1.0 / DENH2O) * rm : 0.0;
-            const double si = spass ? (1.0 / DENICE) * rm : 0.0;
-            const double sw = spass ? -(satw0 * rm) * dzv : 0.0;
-            // d dksat / d fl, d ws
-            const double kfl = dksat * (LN_TKWAT * ws - LN_TKICE * ws);
-            const double kws = dksat * (LN_TKWAT * fl + LN_TKICE * (1.0 - fl));
-            const double fll = (1.0 - fl) * rfd * (1.0 / DENH2O) * rdz;
-            const double fli = -fl * rfd * (1.0 / DENICE) * rdz;
-            const double cdke = (dksat - tkdry) * ddke;
-            dl = cdke * sl + dke * kfl * fll;
-            di = cdke * si + dke * kfl * fli;
-            dw = cdke * sw + dke * kws;
-          } else {
-            v = LVc(f.tkdry, c, j, ld);
-          }
-        }
-      } else if (lit == ISTICE) {
-        v = tin[jj] < TFRZ ? TKICE : TKWAT;
-      } else {
-        if (j > D.nlevsoi) v = THK_BEDROCK;
-        else v = tin[jj] < TFRZ ? TKICE : TKWAT;
-      }
-    } else {
-      const double denom = jl_max(fse, 1.0e-6) * jl_max(LVc(f.dz, c, jj, ld), 1.0e-6);
-      const double bwv = (ice0[jj] + liq0[jj]) / denom;
-      double dbw;
-      if (snow_method == CLMGB_SNOW_JORDAN1991) {
-        v = TKAIR + (7.75e-5 * bwv + 1.105e-6 * (bwv * bwv)) * (TKICE - TKAIR);
-        dbw = (7.75e-5 + 1.105e-6 * (bwv + bwv)) * (TKICE - TKAIR);
-      } else if (bwv <= 156.0) {
-        v = 0.023 + 0.234 * (bwv / 1000.0);
-        dbw = 0.234 / 1000.0;
-      } else {
-        v = 0.138 - 1.01 * (bwv / 1000.0) + 3.233 * ((bwv / 1000.0) * (bwv / 1000.0));
-        dbw = (-1.01 + 3.233 * (2.0 * (bwv / 1000.0))) / 1000.0;
-      }
-      dl = dbw / denom;
-      di = dbw / denom;
-    }
-    thk[jj] = v;
-    tl[jj] = dl;
-    ti[jj] = di;
-    tw[jj] = dw;
-  }
-  // tk_h2osfc from the soil-1 layer conductivity
-  double tkh, dtkh;
-  {
-    const double zh2osfc = 1.0e-3 * (0.5 * f.h2osfc[c]);
-    const double z1 = zz[1 + joff];
-    const double tk1 = thk[1 + joff];
-    const double den = TKWAT * z1 + tk1 * zh2osfc;
-    if (den > 0.0) {
-      tkh = TKWAT * tk1 * (z1 + zh2osfc) / den;
-      dtkh = (TKWAT * (z1 + zh2osfc) - tkh * zh2osfc) / den;
-    } else {
-      tkh = tk1;
-      dtkh = 1.0;
-    }
-  }
-  // interface conductivity and its partials in the two layers
-  double tkif[MAXL + 2], da[MAXL + 2], db[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    if (j <= nlevgrnd - 1) {
-      const double tkj = thk[jj], tkj1 = thk[jj + 1];
-      const double zj = zz[jj], zj1 = zz[jj + 1], zij1 = LVc(f.zi, c, jj + 1, ld);
-      const double A = zj1 - zj, Bz = zj1 - zij1, Cz = zij1 - zj;
-      const double rden = 1.0 / (tkj * Bz + tkj1 * Cz);
-      const double v = tkj * tkj1 * A * rden;
-      tkif[jj] = v;
-      da[jj] = (tkj1 * A - v * Bz) * rden;
-      db[jj] = (tkj * A - v * Cz) * rden;
-    } else {
-      tkif[jj] = 0.0;
-      da[jj] = 0.0;
-      db[jj] = 0.0;
-    }
-  }
-  // heat capacity: cv and the partials of fact in liquid water, ice and watsat
-  double cl[MAXL + 2], ci[MAXL + 2], cw[MAXL + 2];
-  double fn[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    const double dzv = LVc(f.dz, c, jj, ld);
-    double cv, dl = 0.0, di = 0.0, dw = 0.0;
-    if (j >= 1) {
-      if (!is_special) {
-        const double ws = LVc(fw.watsat, c, j, ld);
-        cv = LVc(f.csol, c, j, ld) * (1.0 - ws) * dzv + (ice0[jj] * CPICE + liq0[jj] * CPLIQ) +
-             LV(f.excess_ice, c, j, ld) * CPICE;
-        dl = CPLIQ;
-        di = CPICE;
-        dw = -LVc(f.csol, c, j, ld) * dzv;
-      } else {
-        cv = ice0[jj] * CPICE + liq0[jj] * CPLIQ;
-        dl = CPLIQ;
-        di = CPICE;
-      }
-      if (j > nbedrock) {
-        cv = CSOL_BEDROCK * dzv;
-        dl = di = dw = 0.0;
-      }
-      if (j == 1 && f.h2osno_no_layers[c] > 0.0) cv += CPICE * f.h2osno_no_layers[c];
-    } else {
-      if (fse > 0.0) {
-        const double v = (CPLIQ * liq0[jj] + CPICE * ice0[jj]) / fse;
-        cv = jl_max(THIN_SFCLAYER, v);
-        if (!same_bits(cv, THIN_SFCLAYER)) {
-          dl = CPLIQ / fse;
-          di = CPICE / fse;
-        }
-      } else {
-        cv = THIN_SFCLAYER;
-      }
-    }
-    const double dfdcv = -fact[jj] / cv;
-    cl[jj] = dfdcv * dl;
-    ci[jj] = dfdcv * di;
-    cw[jj] = dfdcv * dw;
-    if (j <= nlevgrnd - 1) fn[jj] = tkif[jj] * (tin[jj + 1] - tin[jj]) * rdzp[jj];
-    else fn[jj] = f.eflx_bot[c];
-  }
-  // ground heat flux sums and their derivative weights
-  const double eg = f.emg[c];
-  const double htvp = f.htvp[c];
-  double dhsdT = 0.0, hs_soil = 0.0, hs_h2osfc = 0.0, hs_top = 0.0;
-  double w_set = 0.0, wb_set = 0.0, w_act = 0.0, wb_act = 0.0;
-  double sabg_col[MAXSNO + 2];
-  for (int k = 0; k <= nlevsno + 1; k++) sabg_col[k] = 0.0;
-  {
-    const double dlwrad_emit = 4.0 * eg * SB * (tg0 * tg0 * tg0);
-    const double lwe_snow = eg * SB * jl_pow4(tin[jjtop]);
-    const double lwe_soil = eg * SB * jl_pow4(tin[1 + joff]);
-    const double lwe_h2osfc = eg * SB * jl_pow4(th0);
-    for (int64_t p1 = f.col_patchi[c]; p1 <= f.col_patchf[c]; p1++) {
-      const int64_t p = p1 - 1;
-      if (f.patch_column[p] != c + 1 + D.c0) continue;
-      double dh_p = 0.0, hsoil_p = 0.0, hh_p = 0.0;
-      const bool act = f.mask_nolakep[p] != 0;
-      const double cb = (1.0 - (double)f.frac_veg_nosno[p]) * eg;
-      const double base = f.dlrad[p] + cb * forc;
-      const double wt = f.patch_wtcol[p];
-      if (act && !f.lun_urbpoi[f.patch_landunit[p] - 1]) {
-        const double dg = -f.cgrnd[p] - dlwrad_emit;
-        const double gsoil = f.sabg_soil[p] + base - lwe_soil - (f.eflx_sh_soil[p] + f.qflx_ev_soil[p] * htvp);
-        const double gh2o = f.sabg_soil[p] + base - lwe_h2osfc - (f.eflx_sh_h2osfc[p] + f.qflx_ev_h2osfc[p] * htvp);
-        if (wt != 0.0) {
-          dh_p = dg * wt;
-          hsoil_p = gsoil * wt;
-          hh_p = gh2o * wt;
-          w_set += wt;
-          wb_set += wt * cb;
-        }
-      }
-      dhsdT += dh_p; hs_soil += hsoil_p; hs_h2osfc += hh_p;
-      if (act) {
-        const double sab = LVc(f.sabg_lyr, p, jtop + joff, ldp);
-        const double gsnow = sab + base - lwe_snow - (f.eflx_sh_snow[p] + f.qflx_ev_snow[p] * htvp);
-        hs_top += gsnow * wt;
-        w_act += wt;
-        wb_act += wt * cb;
-        for (int j = jtop; j <= 1; j++) sabg_col[j + nlevsno] += LVc(f.sabg_lyr, p, j + joff, ldp) * wt;
-      }
-    }
-  }
-  double ch, dz_h2osfc;
-  if (f.h2osfc[c] > THIN_SFCLAYER && fh > THIN_SFCLAYER) {
-    ch = jl_max(THIN_SFCLAYER, CPLIQ * f.h2osfc[c] / fh);
-    dz_h2osfc = jl_max(THIN_SFCLAYER, 1.0e-3 * f.h2osfc[c] / fh);
-  } else {
-    ch = THIN_SFCLAYER;
-    dz_h2osfc = THIN_SFCLAYER;
-  }
-  const int n = B.n;
-  const int rsw = -(int)snl;
-
-  // ---- reverse: t_grnd ----
-  double Tpc_b[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) Tpc_b[jj] = Tb[jj];
-  double thpc_b = thb;                          // t_h2osfc after the call
-  if (snl < 0) {
-    Tpc_b[jjtop] += fse * tgb;
-    Tpc_b[1 + joff] += (fh != 0.0 ? (1.0 - fse - fh) : (1.0 - fse)) * tgb;
-    if (fh != 0.0) thpc_b += fh * tgb;
-  } else {
-    Tpc_b[1 + joff] += (fh != 0.0 ? (1.0 - fh) : 1.0) * tgb;
-    if (fh != 0.0) thpc_b += fh * tgb;
-  }
-  // ---- reverse: phase change ----
-  double ts_b[MAXL + 2], fct_b[MAXL + 2], liq_in_b[MAXL + 2], ice_in_b[MAXL + 2];
-  double dhsdT_b = 0.0;
-  const bool sc_type = (lit == ISTSOIL || lit == ISTCROP || it == ICOL_ROAD_PERV);
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    ts_b[jj] = 0.0;
-    fct_b[jj] = 0.0;
-    liq_in_b[jj] = 0.0;
-    ice_in_b[jj] = 0.0;
-    PcLevelIn in;
-    in.j = j;
-    in.jtop = jtop;
-    in.T0 = B.x[j <= 0 ? j - jtop : rsw + j];
-    in.wice0 = ice0[jj];
-    in.wliq0 = liq0[jj];
-    in.fct = fact[jj];
-    in.dhsdT = dhsdT;
-    in.fse = fse;
-    in.fh = fh;
-    in.dtime = dtime;
-    in.sc_type = sc_type;
-    in.ws = j >= 1 ? LVc(fw.watsat, c, j, ld) : 0.0;
-    in.bs = j >= 1 ? LVc(fw.bsw, c, j, ld) : 0.0;
-    in.suc = j >= 1 ? LVc(fw.sucsat, c, j, ld) : 0.0;
-    in.dz = LVc(f.dz, c, jj, ld);
-    double wsd = 0.0, bsd = 0.0, sud = 0.0;
-    phase_change_level_reverse(in, Tpc_b[jj], liqb[jj], iceb[jj], ts_b[jj], ice_in_b[jj], liq_in_b[jj], fct_b[jj],
-                               dhsdT_b, wsd, bsd, sud);
-    if (j >= 1) {
-      wsb[j] += wsd;
-      bsb[j] += bsd;
-      sucb[j] += sud;
-    }
-  }
-  // ---- reverse: extraction and the band solve ----
-  double w[MAXROWS];
-  for (int r = 0; r < n; r++) w[r] = 0.0;
-  for (int j = jtop; j <= 0; j++) w[j - jtop] += ts_b[j + joff];
-  for (int j = 1; j <= nlevgrnd; j++) w[rsw + j] += ts_b[j + joff];
-  if (fh == 0.0) w[rsw + 1] += thpc_b;   // t_h2osfc took the soil-1 temperature
-  else w[rsw] += thpc_b;
-  band_lu_transpose_solve<2, 2>(B.lu, B.piv, w, n);    // w = lambda
-  // Abar[r][col] = -lambda_r x_col
-#define ABAR(r, d) ((((r) - 2 + (d)) >= 0 && ((r) - 2 + (d)) < n) ? -w[r] * B.x[(r) - 2 + (d)] : 0.0)
-  // ---- reverse: assembly ----
-  double tin_b[MAXL + 2], tkif_b[MAXL + 2], fn_b[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) {
-    tin_b[jj] = 0.0;
-    tkif_b[jj] = 0.0;
-    fn_b[jj] = 0.0;
-  }
-  double hs_top_b = 0.0, hs_soil_b = 0.0, hs_h2osfc_b = 0.0, tkh_b = 0.0, th_b = 0.0;
-  for (int j = jtop; j <= 0; j++) {
-    const int jj = j + joff;
-    const int r = j - jtop;
-    const double fc = fact[jj];
-    const double rp = rdzp[jj];
-    const double lam = w[r];
-    tin_b[jj] += lam;
-    if (j == jtop) {
-      const double inner = hs_top - dhsdT * tin[jj] + CNFAC * fn[jj];
-      fct_b[jj] += lam * inner;
-      const double ib = lam * fc;
-      hs_top_b += ib;
-      dhsdT_b -= ib * tin[jj];
-      tin_b[jj] -= ib * dhsdT;
-      fn_b[jj] += ib * CNFAC;
-      const double g2 = ABAR(r, 2);
-      fct_b[jj] += g2 * (omc * tkif[jj] * rp - dhsdT);
-      tkif_b[jj] += g2 * omc * fc * rp;
-      dhsdT_b -= g2 * fc;
-    } else {
-      fct_b[jj] += lam * (CNFAC * (fn[jj] - fn[jj - 1]) + sabg_col[jj]);
-      fn_b[jj] += lam * CNFAC * fc;
-      fn_b[jj - 1] -= lam * CNFAC * fc;
-      const double rmn = rdzp[jj - 1];
-      const double g1 = ABAR(r, 1), g2 = ABAR(r, 2);
-      fct_b[jj] += -g1 * omc * tkif[jj - 1] * rmn + g2 * omc * (tkif[jj] * rp + tkif[jj - 1] * rmn);
-      tkif_b[jj - 1] += -g1 * omc * fc * rmn + g2 * omc * fc * rmn;
-      tkif_b[jj] += g2 * omc * fc * rp;
-    }
-    const double g = (j != 0) ? ABAR(r, 3) : ABAR(r, 4);
-    fct_b[jj] += -g * omc * tkif[jj] * rp;
-    tkif_b[jj] += -g * omc * fc * rp;
-  }
-  {   // surface-water row
-    const double rdh = 1.0 / (0.5 * dz_h2osfc + zz[1 + joff]);
-    const double dtc = dtime / ch;
-    const double t1 = tin[1 + joff];
-    const double fnh = tkh * (t1 - th0) * rdh;
-    const double lam = w[rsw];
-    th_b += lam;
-    const double ib = lam * dtc;
-    hs_h2osfc_b += ib;
-    dhsdT_b -= ib * th0;
-    th_b -= ib * dhsdT;
-    const double fnh_b = ib * CNFAC;
-    const double g2 = ABAR(rsw, 2), g3 = ABAR(rsw, 3);
-    tkh_b += g2 * omc * dtc * rdh - g3 * omc * dtc * rdh;
-    dhsdT_b -= g2 * dtc;
-    tkh_b += fnh_b * (t1 - th0) * rdh;
-    const double d_b = fnh_b * tkh * rdh;
-    tin_b[1 + joff] += d_b;
-    th_b -= d_b;
-    (void)fnh;
-  }
-  for (int j = 1; j <= nlevgrnd; j++) {
-    const int jj = j + joff;
-    const int r = rsw + j;
-    const double fc = fact[jj];
-    const double t0 = tin[jj];
-    const double lam = w[r];
-    tin_b[jj] += lam;
-    if (j == jtop) {
-      const double rp = rdzp[jj];
-      const double inner = hs_top - dhsdT * t0 + CNFAC * fn[jj];
-      fct_b[jj] += lam * inner;
-      const double ib = lam * fc;
-      hs_top_b += ib;
-      dhsdT_b -= ib * t0;
-      tin_b[jj] -= ib * dhsdT;
-      fn_b[jj] += ib * CNFAC;
-      const double g2 = ABAR(r, 2), g3 = ABAR(r, 3);
-      fct_b[jj] += g2 * (omc * tkif[jj] * rp - dhsdT) - g3 * omc * tkif[jj] * rp;
-      tkif_b[jj] += g2 * omc * fc * rp - g3 * omc * fc * rp;
-      dhsdT_b -= g2 * fc;
-    } else if (j == 1) {
-      const double rmn = rdzp[jj - 1];
-      const double rp = rdzp[jj];
-      const double inner = (1.0 - fse) * (hs_soil - dhsdT * t0) + CNFAC * (fn[jj] - fse * fn[jj - 1]);
-      fct_b[jj] += lam * (inner + fse * sabg_col[j + nlevsno]);
-      const double ib = lam * fc;
-      const double u = ib * (1.0 - fse);
-      hs_soil_b += u;
-      dhsdT_b -= u * t0;
-      tin_b[jj] -= u * dhsdT;
-      fn_b[jj] += ib * CNFAC;
-      fn_b[jj - 1] -= ib * CNFAC * fse;
-      const double g0 = ABAR(r, 0), g2 = ABAR(r, 2), g3 = ABAR(r, 3);
-      fct_b[jj] += -g3 * omc * tkif[jj] * rp +
-                   g2 * (omc * (tkif[jj] * rp + fse * tkif[jj - 1] * rmn) - (1.0 - fse) * dhsdT) -
-                   g0 * fse * omc * tkif[jj - 1] * rmn;
-      tkif_b[jj] += -g3 * omc * fc * rp + g2 * omc * fc * rp;
-      tkif_b[jj - 1] += g2 * omc * fc * fse * rmn - g0 * fse * omc * fc * rmn;
-      dhsdT_b -= g2 * (1.0 - fse) * fc;
-    } else if (j <= nlevgrnd - 1) {
-      const double rmn = rdzp[jj - 1];
-      const double rp = rdzp[jj];
-      fct_b[jj] += lam * CNFAC * (fn[jj] - fn[jj - 1]);
-      fn_b[jj] += lam * CNFAC * fc;
-      fn_b[jj - 1] -= lam * CNFAC * fc;
-      const double g1 = ABAR(r, 1), g2 = ABAR(r, 2), g3 = ABAR(r, 3);
-      fct_b[jj] += -g3 * omc * tkif[jj] * rp + g2 * omc * (tkif[jj] * rp + tkif[jj - 1] * rmn) -
-                   g1 * omc * tkif[jj - 1] * rmn;
-      tkif_b[jj] += -g3 * omc * fc * rp + g2 * omc * fc * rp;
-      tkif_b[jj - 1] += g2 * omc * fc * rmn - g1 * omc * fc * rmn;
-    } else {
-      const double rmn = rdzp[jj - 1];
-      fct_b[jj] += lam * (-CNFAC * fn[jj - 1] + fn[jj]);
-      fn_b[jj - 1] -= lam * CNFAC * fc;
-      const double g1 = ABAR(r, 1), g2 = ABAR(r, 2);
-      fct_b[jj] += g2 * omc * tkif[jj - 1] * rmn - g1 * omc * tkif[jj - 1] * rmn;
-      tkif_b[jj - 1] += g2 * omc * fc * rmn - g1 * omc * fc * rmn;
-    }
-  }
-  if (fh != 0.0) {   // surface-water corrections to soil layer 1
-    const int jj = 1 + joff;
-    const int r = rsw + 1;
-    const double fc = fact[jj];
-    const double rdh = 1.0 / (0.5 * dz_h2osfc + zz[1 + joff]);
-    const double fnh = tkh * (tin[jj] - th0) * rdh;
-    const double lam = w[r];
-    // x[r] -= fh fc ((hs_soil - dhsdT t1) + CNFAC fnh)
-    const double ib = -lam * fh;
-    fct_b[jj] += ib * ((hs_soil - dhsdT * tin[jj]) + CNFAC * fnh);
-    hs_soil_b += ib * fc;
-    dhsdT_b -= ib * fc * tin[jj];
-    tin_b[jj] -= ib * fc * dhsdT;
-    const double fnh_b = ib * fc * CNFAC;
-    tkh_b += fnh_b * (tin[jj] - th0) * rdh;
-    tin_b[jj] += fnh_b * tkh * rdh;
-    th_b -= fnh_b * tkh * rdh;
-    // ab[r][2] += fh (omc fc tkh / dzm + fc dhsdT); ab[r][1] = -fh omc fc tkh / dzm
-    const double g2 = ABAR(r, 2), g1 = ABAR(r, 1);
-    fct_b[jj] += g2 * fh * (omc * tkh * rdh + dhsdT) - g1 * fh * omc * tkh * rdh;
-    tkh_b += g2 * fh * omc * fc * rdh - g1 * fh * omc * fc * rdh;
-    dhsdT_b += g2 * fh * fc;
-  }
-#undef ABAR
-  // ---- reverse: fn ----
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    if (j <= nlevgrnd - 1 && fn_b[jj] != 0.0) {
-      const double rz = rdzp[jj];
-      tkif_b[jj] += fn_b[jj] * (tin[jj + 1] - tin[jj]) * rz;
-      const double d_b = fn_b[jj] * tkif[jj] * rz;
-      tin_b[jj + 1] += d_b;
-      tin_b[jj] -= d_b;
-    }
-  }
-  // ---- reverse: ground heat flux sums ----
-  const double e4 = eg * SB * 4.0;
-  tgb = dhsdT_b * (-w_set) * (4.0 * eg * SB) * (3.0 * (tg0 * tg0));
-  forcb += (hs_soil_b + hs_h2osfc_b) * wb_set + hs_top_b * wb_act;
-  tin_b[1 + joff] += hs_soil_b * (-w_set) * e4 * (tin[1 + joff] * tin[1 + joff] * tin[1 + joff]);
-  th_b += hs_h2osfc_b * (-w_set) * e4 * (th0 * th0 * th0);
-  tin_b[jjtop] += hs_top_b * (-w_act) * e4 * (tin[jjtop] * tin[jjtop] * tin[jjtop]);
-  // ---- reverse: fact (through cv) ----
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    liq_in_b[jj] += fct_b[jj] * cl[jj];
-    ice_in_b[jj] += fct_b[jj] * ci[jj];
-    if (j >= 1) wsb[j] += fct_b[jj] * cw[jj];
-  }
-  // ---- reverse: interface conductivity, tk_h2osfc, layer conductivity ----
-  double thk_b[MAXL + 2];
-  for (int jj = jjtop; jj <= nw; jj++) thk_b[jj] = 0.0;
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    if (j <= nlevgrnd - 1) {
-      thk_b[jj] += tkif_b[jj] * da[jj];
-      thk_b[jj + 1] += tkif_b[jj] * db[jj];
-    }
-  }
-  thk_b[1 + joff] += tkh_b * dtkh;
-  for (int jj = jjtop; jj <= nw; jj++) {
-    const int j = jj - nlevsno;
-    liq_in_b[jj] += thk_b[jj] * tl[jj];
-    ice_in_b[jj] += thk_b[jj] * ti[jj];
-    if (j >= 1) wsb[j] += thk_b[jj] * tw[jj];
-  }
-  // ---- adjoints of the inputs ----
-  for (int jj = jjtop; jj <= nw; jj++) {
-    Tb[jj] = tin_b[jj];
-    liqb[jj] = liq_in_b[jj];
-    iceb[jj] = ice_in_b[jj];
-  }
-  thb = th_b;
-}
-
 // ---------------------------------------------------------------------------
 // The kernel: one thread per column, columns handed out by a work counter.
 // ---------------------------------------------------------------------------
@@ -840,6 +117,7 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
     if (k >= nc) break;
     const int64_t c = order ? (int64_t)order[k] : k;
     const bool do_t = ft.mask_nolakec[c] != 0, do_w = fw.mask_hydrology[c] != 0;
+    if (step_reversed_here(D, ft, fw, lg, c)) continue;     // k_richards_reverse and k_soil_reverse have
     if (!do_t && !do_w) {     // the step leaves the column alone: identity
       if (col_status) col_status[c] = 0;
       continue;
@@ -915,24 +193,19 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
     bool rich = false;
     int nacc = 0;
     const double* logc = nullptr;     // this column's log region, when it holds the solve
-    // k_richards_reverse has reversed the solve: adj holds the adjoints before it
-    const bool reversed = do_w && richards_reversed_here(D, ft, fw, lg, c);
-    const int32_t cnt = do_w && lg.rec ? lg.count[c] : -1;
     if (do_w) {
-      if (!reversed) {
-        water_fractions_col(D, fw, c, V);
-        rich = mf_begin(L, D, fw, cfg, dtime, c, V);
-      }
-      if (!reversed && !rich) {
+      water_fractions_col(D, fw, c, V);
+      rich = mf_begin(L, D, fw, cfg, dtime, c, V);
+      if (!rich) {
         st |= L.status;
       } else {
-        if (reversed || (cnt >= 0 && cnt <= lg.cap)) {
+        const int32_t cnt = lg.rec ? lg.count[c] : -1;
+        if (cnt >= 0 && cnt <= lg.cap) {
           logc = lg.rec + c * lg.stride;
           nacc = cnt;
           const double* fin = logc + (int64_t)lg.cap * SUB_REC;
           uint32_t rs = (uint32_t)fin[3 * MAXSOI + 2];
-          const int nl = (int)fw.col_nbedrock[c];
-          for (int j = 1; j <= nl; j++) {
+          for (int j = 1; j <= L.nlayers; j++) {
             V.liq[joff + j] = fin[j - 1];
             LV(fw.smp_l, c, j, ld) = fin[MAXSOI + j - 1];
             LV(fw.hk_l, c, j, ld) = fin[2 * MAXSOI + j - 1];
@@ -967,7 +240,7 @@ k_column_step_vjp_cf(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwat
       LV(ft.h2osoi_ice, c, jj, ld) = V.ice[jj];
       if (do_t) LV(ft.fact, c, jj, ld) = V.fact[jj];
     }
-    if (do_w && !reversed)
+    if (do_w)
       for (int j = 1; j <= nlevsoi; j++) LV(fw.icefrac, c, j, ld) = V.icefrac[j];
     ft.t_grnd[c] = V.tg;
     ft.t_h2osfc[c] = V.th;
@@ -1099,8 +372,14 @@ cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soi
     if ((e = launch_order(nc, VjpKey{ft, fw, lg}, qs.bins, qs.order, s)) != cudaSuccess) return e;
     order = qs.order;
   }
-  if (lg.rec && lg.st && (e = launch_richards_reverse(D, nc, ft, fw, cfg, dtime, adj, lg, order, s)) != cudaSuccess)
-    return e;
+  // The logged columns.  A launch each before the others' kernel, which writes nothing that
+  // they read (their columns are its `continue`).
+  if (lg.rec && lg.st) {
+    if ((e = launch_richards_reverse(D, nc, ft, fw, cfg, dtime, adj, lg, order, s)) != cudaSuccess) return e;
+    if ((e = launch_soil_reverse(D, nc, ft, fw, dtime, snow_method, t_ssbef, t_h2osfc_bef, adj, lg, order, col_status,
+                                 dev_status, s)) != cudaSuccess)
+      return e;
+  }
   int64_t blocks = grid_blocks;
   const int64_t max_blocks = tp.slots / CF_BLOCK;
   if (blocks > max_blocks) blocks = max_blocks;

@@ -209,6 +209,10 @@ cudaError_t launch_richards_reverse(const Dims& D, int64_t nc, const clmgb_soilt
                                     const clmgb_soilwater_fields& fw, const clmgb_swm_config& cfg, double dtime,
                                     const clmgb_step_adjoint& adj, const SubstepLogView& lg, const uint32_t* order,
                                     cudaStream_t s);
+cudaError_t launch_soil_reverse(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,
+                                const clmgb_soilwater_fields& fw, double dtime, int snow_method, double* t_ssbef,
+                                double* t_h2osfc_bef, const clmgb_step_adjoint& adj, const SubstepLogView& lg,
+                                const uint32_t* order, uint32_t* col_status, uint32_t* dev_status, cudaStream_t s);
 cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& ft,
                                       const clmgb_soilwater_fields& fw, const clmgb_swm_config& cfg, double dtime,
                                       int snow_method, double* t_ssbef, double* t_h2osfc_bef,
