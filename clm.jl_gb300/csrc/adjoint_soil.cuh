@@ -54,21 +54,21 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
   bool sc_on = false;
   double sc = 0.0, P = 0.0, r = 0.0, e = 0.0, q = 0.0, g = 0.0;
   if (j <= 0) {
-    if (wice0 > 0.0 && T0 > TFRZ) {
+    if (pos(wice0) && above(T0, TFRZ)) {
       im = 1;
       tinc = TFRZ - T0;
-    } else if (wliq0 > 0.0 && T0 < TFRZ) {
+    } else if (pos(wliq0) && below(T0, TFRZ)) {
       im = 2;
       tinc = TFRZ - T0;
     }
   } else {
     double T = T0;
-    if (wice0 > 0.0 && T0 > TFRZ) {
+    if (pos(wice0) && above(T0, TFRZ)) {
       im = 1;
       tinc = TFRZ - T0;
       T = TFRZ;
     }
-    if (in.sc_type && T < TFRZ) {
+    if (in.sc_type && below(T, TFRZ)) {
       sc_on = true;
       q = jl_div(HFUS * (TFRZ - T), GRAV * T);
       g = GRAV * T;
@@ -79,7 +79,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
       sc = in.ws * P;
       sc *= in.dz * 1000.0;
     }
-    if (wliq0 > sc && T < TFRZ) {
+    if (below(T, TFRZ) && wliq0 > sc) {
       im = 2;
       tinc = TFRZ - T;
     }
@@ -95,15 +95,15 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
   if (j == jtop) {
     if (j > 0) hm = dhsdT * tinc - jl_div(tinc, fct);
     else hm = fse * (dhsdT * tinc - jl_div(tinc, fct));
-    if (j == 1 && fh != 0.0) hm -= fh * dhsdT * tinc;
+    if (j == 1 && !zero_bits(fh)) hm -= fh * dhsdT * tinc;
   } else if (j == 1) {
     hm = (1.0 - fse - fh) * dhsdT * tinc - jl_div(tinc, fct);
   } else {
     if (j < 1) hm = jl_div(-fse * tinc, fct);
     else hm = jl_div(-tinc, fct);
   }
-  if ((im == 1 && hm < 0.0) || (im == 2 && hm > 0.0)) im = 0;
-  if (im == 0 || !(fabs(hm) > 0.0)) {
+  if ((im == 1 && negv(hm)) || (im == 2 && pos(hm))) im = 0;
+  if (im == 0 || !(pos(hm) || negv(hm))) {
     // the temperature was set to freezing (a constant); the water is unchanged
     liq0_b += liqpc_b;
     ice0_b += icepc_b;
@@ -113,12 +113,12 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
   const double xm = jl_div(hm * dtime, HFUS);
   double ice = wice0, heatr = 0.0;
   int kind = 0;   // 0 ice unchanged, 1 wice0 - xm, 2 constant, 3 wmass0, 4 wmass0 - sc
-  if (xm > 0.0) {
+  if (pos(xm)) {
     const double v = wice0 - xm;
     ice = jl_max(0.0, v);
     kind = same_bits(ice, 0.0) ? 2 : 1;
     heatr = hm - jl_div(HFUS * (wice0 - ice), dtime);
-  } else if (xm < 0.0) {
+  } else if (negv(xm)) {
     if (j <= 0) {
       const double a = wmass0, b = wice0 - xm;
       ice = jl_min(a, b);
@@ -142,7 +142,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
   double heatr_b = 0.0, hm_b = 0.0, xm_b = 0.0, ice_b = icepc_b, wmass0_b = 0.0, wice0_b = 0.0, sc_b = 0.0;
   double tinc_b = 0.0;
   const double rf = jl_div(1.0, fct);
-  if (fabs(heatr) > 0.0 && !(j <= 0 && liq * ice > 0.0)) {
+  if ((pos(heatr) || negv(heatr)) && !(j <= 0 && pos(liq * ice))) {
     // temperature correction (:2145-2165); the level starts from freezing
     if (j == 1) {
       const double k = (j == jtop) ? (1.0 - fh) : (1.0 - fse - fh);
@@ -153,7 +153,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
       heatr_b += N_b * fct;
       dhsdT_b += -den_b * k * fct;
     } else if (j == jtop) {      // top snow layer
-      if (fse > 0.0) {
+      if (pos(fse)) {
         const double rfse = jl_div(1.0, fse);
         const double rden = jl_div(1.0, 1.0 - fct * dhsdT);
         const double incr = fct * rfse * heatr * rden;
@@ -165,7 +165,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
     } else if (j > 0) {
       fct_b += Tpc_b * heatr;
       heatr_b += Tpc_b * fct;
-    } else if (fse > 0.0) {
+    } else if (pos(fse)) {
       const double rfse = jl_div(1.0, fse);
       fct_b += Tpc_b * heatr * rfse;
       heatr_b += Tpc_b * fct * rfse;
@@ -175,7 +175,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
     wmass0_b += liqpc_b;
     ice_b -= liqpc_b;
   }
-  if (xm != 0.0) {
+  if (!zero_bits(xm)) {
     hm_b += heatr_b;
     const double d_b = -heatr_b * HFUS * jl_div(1.0, dtime);
     wice0_b += d_b;
@@ -195,7 +195,7 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
     dhsdT_b += hb * tinc;
     tinc_b += hb * dhsdT - hb * rf;
     fct_b += hb * tinc * rf * rf;
-    if (j == 1 && fh != 0.0) {
+    if (j == 1 && !zero_bits(fh)) {
       dhsdT_b -= hm_b * fh * tinc;
       tinc_b -= hm_b * fh * dhsdT;
     }
@@ -211,13 +211,13 @@ static __device__ __noinline__ void phase_change_level_reverse(const PcLevelIn& 
   }
   T0_b -= tinc_b;
   // supercooled water sc = watsat (smp/sucsat)^(-1/bsw) dz 1000, smp = HFUS (TFRZ-T)/(GRAV T) 1000
-  if (sc_b != 0.0 && sc_on) {
+  if (sc_on && !zero_bits(sc_b)) {
     const double sc0_b = sc_b * (in.dz * 1000.0);
     ws_b += sc0_b * P;
     const double P_b = sc0_b * in.ws;
     const double rr = jl_div(1.0, r), rsuc = jl_div(1.0, in.suc), rg = jl_div(1.0, g);
-    const double r_b = r != 0.0 ? P_b * e * P * rr : 0.0;
-    const double e_b = r > 0.0 ? P_b * P * cm_log(r) : 0.0;
+    const double r_b = !zero_bits(r) ? P_b * e * P * rr : 0.0;
+    const double e_b = pos(r) ? P_b * P * cm_log(r) : 0.0;
     bs_b += e_b * (-e) * jl_div(1.0, in.bs);
     const double smp_b = r_b * rsuc;
     suc_b += r_b * (-r) * rsuc;
@@ -281,7 +281,7 @@ __device__ __forceinline__ void st_sums(StCol& C, const Dims& D, const clmgb_soi
       const double dg = -f.cgrnd[p] - dlwrad_emit;
       const double gsoil = f.sabg_soil[p] + base - lwe_soil - (f.eflx_sh_soil[p] + f.qflx_ev_soil[p] * htvp);
       const double gh2o = f.sabg_soil[p] + base - lwe_h2osfc - (f.eflx_sh_h2osfc[p] + f.qflx_ev_h2osfc[p] * htvp);
-      if (wt != 0.0) {
+      if (!zero_bits(wt)) {
         dh_p = dg * wt;
         hsoil_p = gsoil * wt;
         hh_p = gh2o * wt;
@@ -301,7 +301,7 @@ __device__ __forceinline__ void st_sums(StCol& C, const Dims& D, const clmgb_soi
     }
   }
   double ch, dz_h2osfc;
-  if (f.h2osfc[c] > THIN_SFCLAYER && C.fh > THIN_SFCLAYER) {
+  if (above(f.h2osfc[c], THIN_SFCLAYER) && above(C.fh, THIN_SFCLAYER)) {
     ch = jl_max(THIN_SFCLAYER, jl_div(CPLIQ * f.h2osfc[c], C.fh));
     dz_h2osfc = jl_max(THIN_SFCLAYER, jl_div(1.0e-3 * f.h2osfc[c], C.fh));
   } else {
@@ -331,11 +331,11 @@ __device__ __forceinline__ StLayer st_layer(const StCol& C, const Dims& D, const
                                          double ice) {
   const int64_t ld = D.ldc;
   const int j = jj - D.nlevsno;
-  const double LN_TKWAT = cm_log(TKWAT), LN_TKICE = cm_log(TKICE);
+  constexpr double LN_TKWAT = -0.56211891815354124, LN_TKICE = 0.82855181756614826;   // of 0.57 and 2.29
   StLayer r = {0.0, 0.0, 0.0, 0.0};
   if (j >= 1) {
     if (C.is_special) {
-      if (C.lit == ISTICE || j <= D.nlevsoi) r.v = tin < TFRZ ? TKICE : TKWAT;
+      if (C.lit == ISTICE || j <= D.nlevsoi) r.v = below(tin, TFRZ) ? TKICE : TKWAT;
       else r.v = THK_BEDROCK;
       return r;
     }
@@ -351,12 +351,12 @@ __device__ __forceinline__ StLayer st_layer(const StCol& C, const Dims& D, const
     const double satw = jl_min(1.0, satw0);
     const bool spass = !same_bits(satw, 1.0);
     const double tkdry = LVc(f.tkdry, c, j, ld);
-    if (!(satw > 1.0e-7)) {
+    if (!above(satw, 1.0e-7)) {
       r.v = tkdry;
       return r;
     }
     double dke, ddke;
-    if (tin >= TFRZ) {
+    if (at_least(tin, TFRZ)) {
       const double L = cm_log10(satw) + 1.0;
       dke = jl_max(0.0, L);
       ddke = same_bits(dke, 0.0) ? 0.0 : 0.43429448190325182765 * jl_div(1.0, satw);
@@ -367,23 +367,18 @@ __device__ __forceinline__ StLayer st_layer(const StCol& C, const Dims& D, const
     // TKWAT^a TKICE^b as one exponential
     const double rm = jl_div(1.0, m), rdz = jl_div(1.0, dzv);
     const double a1 = liq * (1.0 / DENH2O) * rdz;
-    const double fl_denom = a1 + (ice + exi) * (1.0 / DENICE) * rdz;
+    const double fl_denom = rv_fma((ice + exi) * (1.0 / DENICE), rdz, a1);
     const double rfd = jl_div(1.0, fl_denom);
     const double fl = a1 * rfd;
     const double tkmg = LVc(f.tkmg, c, j, ld);
-    const double dksat = tkmg * cm_exp(ws * (fl * LN_TKWAT + (1.0 - fl) * LN_TKICE));
-    r.v = dke * dksat + (1.0 - dke) * tkdry;
-    const double sl = spass ? (1.0 / DENH2O) * rm : 0.0;
-    const double si = spass ? (1.0 / DENICE) * rm : 0.0;
-    const double sw = spass ? -(satw0 * rm) * dzv : 0.0;
-    const double kfl = dksat * (LN_TKWAT * ws - LN_TKICE * ws);
-    const double kws = dksat * (LN_TKWAT * fl + LN_TKICE * (1.0 - fl));
-    const double fll = (1.0 - fl) * rfd * (1.0 / DENH2O) * rdz;
-    const double fli = -fl * rfd * (1.0 / DENICE) * rdz;
-    const double cdke = (dksat - tkdry) * ddke;
-    r.dl = cdke * sl + dke * kfl * fll;
-    r.di = cdke * si + dke * kfl * fli;
-    r.dw = cdke * sw + dke * kws;
+    const double mix = rv_fma(fl, LN_TKWAT - LN_TKICE, LN_TKICE);
+    const double dksat = tkmg * cm_exp(ws * mix);
+    r.v = rv_fma(dke, dksat - tkdry, tkdry);
+    const double dk = dke * dksat, q = rfd * rdz, kfl = dk * (ws * (LN_TKWAT - LN_TKICE)) * q;
+    const double cdke = spass ? (dksat - tkdry) * ddke * rm : 0.0;
+    r.dl = rv_fma(kfl, (1.0 - fl) * (1.0 / DENH2O), cdke * (1.0 / DENH2O));
+    r.di = rv_fma(kfl, -fl * (1.0 / DENICE), cdke * (1.0 / DENICE));
+    r.dw = rv_fma(dk, mix, -cdke * (satw0 * dzv));
     return r;
   }
   const double denom = jl_max(C.fse, 1.0e-6) * jl_max(LVc(f.dz, c, jj, ld), 1.0e-6);
@@ -410,7 +405,7 @@ __device__ __forceinline__ void st_tkh(const Dims& D, const clmgb_soiltemp_field
   const double zh2osfc = 1.0e-3 * (0.5 * f.h2osfc[c]);
   const double z1 = LVc(f.z, c, 1 + D.nlevsno, D.ldc);
   const double den = TKWAT * z1 + tk1 * zh2osfc;
-  if (den > 0.0) {
+  if (pos(den)) {
     tkh = jl_div(TKWAT * tk1 * (z1 + zh2osfc), den);
     dtkh = jl_div(TKWAT * (z1 + zh2osfc) - tkh * zh2osfc, den);
   } else {
@@ -465,8 +460,8 @@ __device__ __forceinline__ StCap st_capacity(const StCol& C, const Dims& D, cons
       cv = CSOL_BEDROCK * dzv;
       dl = di = dw = 0.0;
     }
-    if (j == 1 && f.h2osno_no_layers[c] > 0.0) cv += CPICE * f.h2osno_no_layers[c];
-  } else if (C.fse > 0.0) {
+    if (j == 1 && pos(f.h2osno_no_layers[c])) cv += CPICE * f.h2osno_no_layers[c];
+  } else if (pos(C.fse)) {
     const double v = jl_div(CPLIQ * liq + CPICE * ice, C.fse);
     cv = jl_max(THIN_SFCLAYER, v);
     if (!same_bits(cv, THIN_SFCLAYER)) {
@@ -485,12 +480,12 @@ __device__ __forceinline__ double st_tgrnd_level(const StCol& C, int j, double t
   if (C.snl < 0) {
     double b = 0.0;
     if (j == C.jtop) b += C.fse * tgb;
-    if (j == 1) b += (C.fh != 0.0 ? (1.0 - C.fse - C.fh) : (1.0 - C.fse)) * tgb;
+    if (j == 1) b += (!zero_bits(C.fh) ? (1.0 - C.fse - C.fh) : (1.0 - C.fse)) * tgb;
     return b;
   }
-  return j == 1 ? (C.fh != 0.0 ? (1.0 - C.fh) : 1.0) * tgb : 0.0;
+  return j == 1 ? (!zero_bits(C.fh) ? (1.0 - C.fh) : 1.0) * tgb : 0.0;
 }
-__device__ __forceinline__ double st_tgrnd_h2osfc(const StCol& C, double tgb) { return C.fh != 0.0 ? C.fh * tgb : 0.0; }
+__device__ __forceinline__ double st_tgrnd_h2osfc(const StCol& C, double tgb) { return !zero_bits(C.fh) ? C.fh * tgb : 0.0; }
 
 // ---- phase change of a level in reverse ----
 struct StPc {
@@ -540,7 +535,7 @@ __device__ __forceinline__ StRow st_row(const StCol& C, int nlevgrnd, const StRo
   const double sp = omc * a.tk * a.rp, sm = omc * a.tkp * a.rmn;      // d entry / d fact
   const double ib = a.lam * a.fc, cb = ib * CNFAC;
   if (a.j == C.jtop) {
-    r.f = a.lam * (C.hs_top - C.dhsdT * a.t + CNFAC * a.fn) + a.g2 * (sp - C.dhsdT);
+    r.f = rv_fma(a.lam, rv_fma(-C.dhsdT, a.t, C.hs_top) + CNFAC * a.fn, a.g2 * (sp - C.dhsdT));
     r.hst = ib;
     r.dh = -ib * a.t - a.g2 * a.fc;
     r.t -= ib * C.dhsdT;
@@ -568,7 +563,7 @@ __device__ __forceinline__ StRow st_row(const StCol& C, int nlevgrnd, const StRo
     r.k = (a.g2 - a.g3) * ip;
     r.kp = (a.g2 - a.g0) * C.fse * im;
   } else if (a.j <= nlevgrnd - 1) {
-    r.f = a.lam * CNFAC * (a.fn - a.fnp) - a.g3 * sp + a.g2 * (sp + sm) - a.g1 * sm;
+    r.f = rv_fma(a.lam * CNFAC, a.fn - a.fnp, rv_fma(a.g2 - a.g3, sp, (a.g2 - a.g1) * sm));
     r.n = cb;
     r.np = -cb;
     r.k = (a.g2 - a.g3) * ip;
@@ -598,7 +593,7 @@ __device__ __forceinline__ StSurf st_surface(const StCol& C, double tkh, double 
   const double d_b = fnh_b * tkh * C.rdh;
   r.t1 = d_b;
   r.th -= d_b;
-  if (C.fh != 0.0) {
+  if (!zero_bits(C.fh)) {
     const double fnh = tkh * dT * C.rdh, jb = -lam1 * C.fh, jf = jb * fact;
     r.f1 = jb * ((C.hs_soil - C.dhsdT * t1) + CNFAC * fnh) + g2 * C.fh * (omc * tkh * C.rdh + C.dhsdT) -
            g1 * C.fh * omc * tkh * C.rdh;
@@ -656,7 +651,7 @@ static __device__ __noinline__ void soil_temperature_reverse(const Dims& D, cons
     w[row_of(jj)] = pc[jj].t;
   }
   const double thpc = thb + st_tgrnd_h2osfc(C, tgb);
-  if (C.fh == 0.0) {                    // t_h2osfc took the soil-1 temperature
+  if (zero_bits(C.fh)) {                    // t_h2osfc took the soil-1 temperature
     w[rsw + 1] += thpc;
     w[rsw] = 0.0;
   } else {

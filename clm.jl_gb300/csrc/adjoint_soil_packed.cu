@@ -3,18 +3,21 @@
 //
 // On a thread per column (k_column_step_vjp_cf) it is a chain through some 40 arrays of
 // levels in local memory, 20 KB a thread; here a block takes SV_COLS columns of the work
-// order, a half-warp per level, and a level's values stay in registers:
+// order, 8 lanes per level, and a level's values stay in registers:
 //
 //   sums, layer conductivity | interface, phase change | transposed band solve | rows | sums
 //   of the rows' parts
 //
 // with neighbours' values through shared memory and a block barrier between the stages (the
 // functions and their order are soil_temperature_reverse's, adjoint_soil.cuh: the same bits).
-// The band solve runs on a half-warp, a column per lane, its right-hand side, factors and
-// pivots staged in shared memory by all threads.
+// The band solve runs a column per lane, its right-hand side, factors and pivots staged in
+// shared memory by all threads.
 //
-// (sums, conductivities and phase change are bound by FP64 instructions, the band solve by
-// its chain.)
+// Measured, 16,384 columns: 1,100 us on a thread per column, 470 us here.  What bounds it: the
+// stages in turn, the band solve's chain and the barriers (26 of 45 stall cycles an issue,
+// FP64 unit 35 % busy with two blocks to an SM).  Hence four blocks of 8 columns to an SM at
+// 48 registers, spills included (two at 96: 570 us, three 503; 16 columns a block 604, 4
+// columns 522).
 #include "adjoint_soil.cuh"
 #include "clmgb_device.cuh"
 #include "launch.h"
@@ -43,7 +46,7 @@ constexpr int SV_ROWS = SV_THREADS / SV_COLS + 2;
 constexpr size_t SV_SMEM = sizeof(double) * SV_COLS * ((size_t)SV_ARRAYS * SV_ROWS + SS_COUNT + 7 * MAXROWS) +
                            (size_t)SV_COLS * MAXROWS;
 
-__global__ void __launch_bounds__(SV_THREADS, 2)
+__global__ void __launch_bounds__(SV_THREADS, 4)
 k_soil_reverse(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fields fw, double dtime,
                int snow_method, double* t_ssbef, double* t_h2osfc_bef, clmgb_step_adjoint adj,
                SubstepLogView lg, const uint32_t* __restrict__ order, uint32_t* col_status, uint32_t* dev_status) {
@@ -90,34 +93,41 @@ k_soil_reverse(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fie
   }
   at(SV_T, jj) = tin;
   if (in && do_t && t_ssbef)
-    for (int q = jj; q <= nlev; q += SV_THREADS / SV_COLS) LV(t_ssbef, c, q, ld) = LV(ft.t_soisno, c, q, ld);
+    if (jj <= nlev) LV(t_ssbef, c, jj, ld) = LV(ft.t_soisno, c, jj, ld);
   for (int r = jj - 1; full && r < n; r += SV_THREADS / SV_COLS) {
     for (int d = 0; d < 7; d++) lu[(r * 7 + d) * SV_COLS] = rec[ST_LU + r * 7 + d];
     piv[r * SV_COLS] = reinterpret_cast<const uint8_t*>(rec + ST_PIV)[r];
     at(SV_X, r) = rec[ST_X + r];
   }
+  // (loads ahead of the barrier, stores behind it: the state's old values are read by then)
+  double tout = 0.0, liq1 = liq0, ice1 = ice0, smp = 0.0, hk = 0.0;
+  const bool solved = do_w && on && j >= 1 && j <= (int)C.nbedrock;
+  if (do_t && jj >= C.jjtop && jj <= nlev) tout = rec[ST_T + jj - 1];
+  if (on && do_t) {
+    liq1 = rec[ST_LIQ + jj - 1];
+    ice1 = rec[ST_ICE + jj - 1];
+  }
+  const double* const fin = lg.rec + c * lg.stride + (int64_t)lg.cap * SUB_REC;
+  if (solved) {
+    liq1 = fin[j - 1];
+    smp = fin[MAXSOI + j - 1];
+    hk = fin[2 * MAXSOI + j - 1];
+  }
   __syncthreads();
-  if (in && jj >= C.jjtop && do_t)
-    for (int q = jj; q <= nlev; q += SV_THREADS / SV_COLS) LV(ft.t_soisno, c, q, ld) = rec[ST_T + q - 1];
+  if (do_t && jj >= C.jjtop && jj <= nlev) LV(ft.t_soisno, c, jj, ld) = tout;
   if (on) {
-    if (do_t) {
-      LV(ft.h2osoi_liq, c, jj, ld) = rec[ST_LIQ + jj - 1];
-      LV(ft.h2osoi_ice, c, jj, ld) = rec[ST_ICE + jj - 1];
-      LV(ft.fact, c, jj, ld) = fact;
-    }
-    if (do_w) {
-      const double* fin = lg.rec + c * lg.stride + (int64_t)lg.cap * SUB_REC;
-      if (j >= 1 && j <= (int)C.nbedrock) {
-        LV(ft.h2osoi_liq, c, jj, ld) = fin[j - 1];
-        LV(fw.smp_l, c, j, ld) = fin[MAXSOI + j - 1];
-        LV(fw.hk_l, c, j, ld) = fin[2 * MAXSOI + j - 1];
-      }
-      if (j == 1) {
-        fw.qcharge[c] = fin[3 * MAXSOI];
-        fw.num_substeps[c] = fin[3 * MAXSOI + 1];
-        st |= (uint32_t)fin[3 * MAXSOI + 2];
-      }
-    }
+    LV(ft.h2osoi_liq, c, jj, ld) = liq1;
+    LV(ft.h2osoi_ice, c, jj, ld) = ice1;
+    if (do_t) LV(ft.fact, c, jj, ld) = fact;
+  }
+  if (solved) {
+    LV(fw.smp_l, c, j, ld) = smp;
+    LV(fw.hk_l, c, j, ld) = hk;
+  }
+  if (do_w && j == 1) {
+    fw.qcharge[c] = fin[3 * MAXSOI];
+    fw.num_substeps[c] = fin[3 * MAXSOI + 1];
+    st |= (uint32_t)fin[3 * MAXSOI + 2];
   }
   if (in && j == 1) {
     st |= s1;
@@ -192,15 +202,20 @@ k_soil_reverse(Dims D, int64_t nc, clmgb_soiltemp_fields ft, clmgb_soilwater_fie
   // ---- A^T lambda = w, band_lu_transpose_solve on a column per lane ----
   if (warp == 0 && lane < SV_COLS && full) {
     auto ab = [&](int row, int col) -> double { return lu[(row * 7 + col - row + 2) * SV_COLS]; };
+    // U^T: a row's sum loses each product as soon as lambda is known, the next row's first
+    double s0 = at(SV_W, 0), s1 = at(SV_W, 1), s2 = at(SV_W, 2), s3 = at(SV_W, 3);
     for (int p = 0; p < n; p++) {
-      double s = at(SV_W, p);
-      for (int q = max(0, p - 4); q < p; q++) s = s - ab(q, p) * at(SV_W, q);
-      at(SV_W, p) = div_chain(s, ab(p, p));
+      const double x = div_chain(s0, ab(p, p)), s4 = p + 4 < n ? at(SV_W, p + 4) : 0.0;
+      at(SV_W, p) = x;
+      s0 = p + 1 < n ? less_product(s1, ab(p, p + 1), x) : 0.0;
+      s1 = p + 2 < n ? less_product(s2, ab(p, p + 2), x) : 0.0;
+      s2 = p + 3 < n ? less_product(s3, ab(p, p + 3), x) : 0.0;
+      s3 = p + 4 < n ? less_product(s4, ab(p, p + 4), x) : 0.0;
     }
     for (int p = n - 2; p >= 0; p--) {
       double s = at(SV_W, p);
       const int last = min(n - 1, p + 2);
-      for (int q = p + 1; q <= last; q++) s = s - ab(q, p) * at(SV_W, q);
+      for (int q = p + 1; q <= last; q++) s = less_product(s, ab(q, p), at(SV_W, q));
       const int x = p + (int)piv[p * SV_COLS];
       at(SV_W, p) = s;
       if (x != p) {

@@ -373,6 +373,12 @@ __device__ __forceinline__ void band_lu_factor_solve(double* ab, double* x, uint
 #undef AB
 }
 
+// s - e w, without the two FP64 instructions where e is one of the band's many zeros
+__device__ __forceinline__ double less_product(double s, double e, double w) {
+  if (zero_bits(e) && finite_bits(w)) return s;
+  return s - e * w;
+}
+
 // A^T w = b from the factors of band_lu_factor_solve (LAPACK gbtrs 'T' order):
 // U^T y = b by forward substitution, then for k = n-2..0: y_k -= sum_i f_ik y_i and
 // the row exchange of step k.  w holds b on entry.
@@ -382,13 +388,13 @@ __device__ __forceinline__ void band_lu_transpose_solve(const double* ab, const 
 #define AB(r, col) ab[(r) * W + ((col) - (r) + KL)]
   for (int i = 0; i < n; i++) {
     double s = w[i];
-    for (int j = max(0, i - KL - KU); j < i; j++) s = s - AB(j, i) * w[j];
+    for (int j = max(0, i - KL - KU); j < i; j++) s = less_product(s, AB(j, i), w[j]);
     w[i] = jl_div(s, AB(i, i));
   }
   for (int k = n - 2; k >= 0; k--) {
     double s = w[k];
     const int ilast = min(n - 1, k + KL);
-    for (int i = k + 1; i <= ilast; i++) s = s - AB(i, k) * w[i];
+    for (int i = k + 1; i <= ilast; i++) s = less_product(s, AB(i, k), w[i]);
     w[k] = s;
     const int p = k + (int)piv[k];
     if (p != k) {
