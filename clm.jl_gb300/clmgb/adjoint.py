@@ -26,6 +26,7 @@ the water (liquid + ice, mm) of the top 10 cm of soil.
 import numpy as np
 
 from . import abi, api
+from .state import copy_arrays
 
 PARAMS = ("watsat", "bsw", "sucsat", "hksat")
 
@@ -77,9 +78,12 @@ def copy_state_(dst, src, full=False):
     column step writes them, so two states of one trajectory hold the same values
     there (the states the reverse passes copy between all descend from one state)."""
     from .hoststep import STATIC
-    for k, v in src.arrays.items():
-        if full or k not in STATIC:
-            dst.arrays[k].copy_(v)
+    pairs = [(dst.arrays[k], v) for k, v in src.arrays.items() if full or k not in STATIC]
+    if src.on_device and dst.on_device:
+        copy_arrays(pairs)
+    else:
+        for d, v in pairs:
+            d.copy_(v)
 
 
 class Trajectory:

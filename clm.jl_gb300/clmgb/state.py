@@ -42,6 +42,27 @@ def pointer_struct(cls, fields, arrays):
     return cls.from_buffer_copy(array.array("Q", words))
 
 
+def copy_arrays(pairs):
+    """dst <- src for (dst, src) pairs of device tensors on the current stream: contiguous
+    ones of the same type, shape and device together in one launch, the others by torch."""
+    import torch
+    from . import _lib
+    dst, src, size = array.array("Q"), array.array("Q"), array.array("q")
+    here = torch.device("cuda", torch.cuda.current_device()) if torch.cuda.is_initialized() else None
+    for d, s in pairs:
+        if (d.device == here and s.device == here and d.is_contiguous() and s.is_contiguous() and
+                d.dtype == s.dtype and d.shape == s.shape):
+            dst.append(d.data_ptr())
+            src.append(s.data_ptr())
+            size.append(s.nbytes)
+        else:
+            d.copy_(s)
+    if dst:
+        p = [C.c_void_p(a.buffer_info()[0]) for a in (dst, src, size)]
+        _lib.check(_lib.load().clmgb_copy_arrays(len(dst), *p, C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                   "copy_arrays")
+
+
 class ColumnState:
     """All fields of the soil/snow column solve for `nc` columns."""
 
@@ -76,7 +97,9 @@ class ColumnState:
 
     def copy(self):
         if self.on_device:
-            arrs = {k: v.clone() for k, v in self.arrays.items()}
+            import torch
+            arrs = {k: torch.empty_like(v) for k, v in self.arrays.items()}
+            copy_arrays((arrs[k], v) for k, v in self.arrays.items())
         else:
             arrs = {k: v.copy() for k, v in self.arrays.items()}
         return ColumnState(self.vp, self.nc, self.np, self.nl, arrs)

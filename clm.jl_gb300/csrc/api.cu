@@ -903,6 +903,16 @@ int32_t clmgb_get_option(clmgb_handle h, int32_t key, int64_t* value) {
   }
 }
 
+int32_t clmgb_copy_arrays(int32_t n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream) {
+  if (n < 0) return CLMGB_ERR_DIMS;
+  if (n && (!dst || !src || !bytes)) return CLMGB_ERR_NULL_ARG;
+  for (int32_t i = 0; i < n; i++) {
+    if (bytes[i] < 0) return CLMGB_ERR_DIMS;
+    if (bytes[i] && (!dst[i] || !src[i])) return CLMGB_ERR_NULL_ARG;
+  }
+  return clmgb::launch_copy_arrays(n, dst, src, bytes, (cudaStream_t)stream) == cudaSuccess ? CLMGB_OK : CLMGB_ERR_CUDA;
+}
+
 int32_t clmgb_math_eval(clmgb_handle h, int32_t op, int64_t n, const double* x, const double* y, double* out,
                         void* stream) {
   if (!handle_ok(h)) return CLMGB_ERR_HANDLE;

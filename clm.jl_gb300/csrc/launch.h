@@ -232,6 +232,10 @@ cudaError_t launch_tridiagonal_adjoint(int64_t ncols, int64_t ldc, int nlevs, co
                                        double* cbar, double* rbar, const int64_t* jtop, const uint8_t* mask,
                                        cudaStream_t s);
 
+// Copies n arrays in as few launches as their table allows (COPY_MAX arrays each).
+constexpr int COPY_MAX = 128;
+cudaError_t launch_copy_arrays(int n, void* const* dst, const void* const* src, const int64_t* bytes, cudaStream_t s);
+
 cudaError_t launch_mlp_linear(int64_t M, int N, int K, const void* X, int64_t ldx, const void* W, const float* b,
                               int act, float* Z, int64_t ldz, void* Y, int64_t ldy, cudaStream_t s);
 cudaError_t launch_mlp_linear_dw(int64_t M, int N, int K, const void* dZ, int64_t lddz, const void* X, int64_t ldx,

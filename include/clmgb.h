@@ -771,6 +771,10 @@ int32_t clmgb_get_option(clmgb_handle h, int32_t key, int64_t* value);
 int32_t clmgb_math_eval(clmgb_handle h, int32_t op, int64_t n, const double* x, const double* y,
                         double* out, void* stream);
 
+/* dst[i] <- src[i], bytes[i] bytes each, for n pairs of device arrays that do not overlap (equal
+ * pointers are left alone), in one launch per 128 arrays.  dst, src and bytes are host arrays. */
+int32_t clmgb_copy_arrays(int32_t n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream);
+
 /* ---- drop-in entry points ---- */
 
 /* soil_temperature! (soil_temperature.jl:358) for non-urban, non-lake columns.
