@@ -373,9 +373,13 @@ __device__ __forceinline__ void band_lu_factor_solve(double* ab, double* x, uint
 #undef AB
 }
 
-// s - e w, without the two FP64 instructions where e is one of the band's many zeros
+// whether s - e w is s for a zero e: w finite and s not -0 (which a product of -0 turns to +0)
+__device__ __forceinline__ bool keeps(double s, double w) {
+  return finite_bits(w) && dbits(s) != (long long)0x8000000000000000ULL;
+}
+// s - e w, without the two FP64 instructions where e is one of a band's many zeros
 __device__ __forceinline__ double less_product(double s, double e, double w) {
-  if (zero_bits(e) && finite_bits(w)) return s;
+  if (zero_bits(e) && keeps(s, w)) return s;
   return s - e * w;
 }
 
