@@ -30,10 +30,13 @@
 //
 // Measured per call (scale workload, steps 5-24, ms), against the kernel with one column
 // per lane and a warp-per-column finish it replaced: 61 columns 1.88 -> 0.29, 1,024 4.06
-// -> 0.49, 16,384 6.27 -> 1.06, 65,536 6.90 -> 1.86, 262,144 9.94 -> 4.46.  What bounds
-// it: at few columns the longest column's attempts, one after another (8 us each); at
-// many the latency of the divisions and powers at 2.5 warps per sub-partition (ncu at
-// 65,536 columns: FP64 unit 47 % busy, issue slots 32 %).
+// -> 0.46, 16,384 6.27 -> 0.97, 65,536 6.90 -> 1.7, 262,144 9.94 -> 4.3.  What bounds
+// it: at few columns the longest column's attempts, one after another (8 us each, half of it
+// the forward sweep and the back substitution); at many the FP64 unit and the latency of the
+// divisions and powers at 2.4 warps per sub-partition (ncu at 262,144 columns: FP64 unit 54 %
+// busy, issue slots 35 %).  Not warps: with three level arrays in the L2-resident records and
+// 15 or 18 warps per SM the solve took 4.5 and 4.33 ms for 4.30.  Not divisions: exact
+// quotients from kept 64-bit reciprocals, half the instructions, took 4.30.
 #include "clmgb_device.cuh"
 #include "launch.h"
 
@@ -43,6 +46,12 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int KS = 16, SLD = KS + 1;
+// Columns per warp up to which an attempt's quotients and powers are formed in line (FEW): the
+// warp waits for its own chain, and independent ones overlap.  ms a call in line / through the
+// shared functions, scale workload: 61 columns 0.249 / 0.268, 1,024 0.459 / 0.486, 8,000 (6 a
+// warp) 0.796 / 0.838, 12,000 (8) 0.818 / 0.832, 24,000 (16) 1.094 / 1.057, 262,144 5.1 / 4.3:
+// warps in different phases no longer find the code in the instruction cache.
+constexpr int FEW_SLOTS = 8;
 constexpr int PWARPS = 5, PBLOCK = 32 * PWARPS;   // 2 blocks, 10 warps, of 20 levels on an SM
 
 // level arrays: the flux derivatives dqodw1, dqodw2 and the net flux (kept from a
@@ -68,7 +77,31 @@ __host__ __device__ constexpr int64_t warp_bytes(int nls, bool expensive) {
   return level_doubles(nls, expensive) * 8 + (int64_t)((sizeof(SlotArea) + 15) / 16 * 16);
 }
 
-template <bool LOG, bool EXPENSIVE>
+// A quotient of a group: with FEW in line and without a branch, so that independent ones
+// overlap (ok turns false where the group has to be formed again by jl_div); else jl_div.
+template <bool FEW>
+__device__ __forceinline__ double quotient(double x, double y, bool& ok) {
+  if (!FEW) return jl_div(x, y);
+  bool o;
+  const double q = cm_div_fx(x, y, &o);
+  ok = ok & o;
+  return q;
+}
+// both powers of an item: with FEW in line, beside each other
+template <bool FEW>
+__device__ __forceinline__ void power_pair(double x1, double y1, double x2, double y2, double& p1, double& p2) {
+  if (FEW) {
+    const bool o1 = cm_pow_fx(x1, y1, &p1), o2 = cm_pow_fx(x2, y2, &p2);
+    if (!o1) p1 = cm_pow_dd_call_(x1, y1);
+    if (!o2) p2 = cm_pow_dd_call_(x2, y2);
+  } else {
+    p1 = cm_pow(x1, y1);
+    p2 = cm_pow(x2, y2);
+  }
+}
+
+// FEW: for warps of few columns, whose attempts wait for their own quotients and powers
+template <bool LOG, bool EXPENSIVE, bool FEW>
 __global__ void __launch_bounds__(PBLOCK, 2)
 k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_config cfg, double dtime,
                        uint32_t* col_status, int or_status, uint32_t* dev_status, unsigned long long* queue,
@@ -151,8 +184,10 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
       if (dn) {
         if (!finite_bits(liq)) SA.bad[it.s] = 1;
       } else {
-        const double vwc = jl_div(jl_max(liq, 1.0e-6), dzw);
-        double s = jl_div(vwc, ws);
+        const double lm = jl_max(liq, 1.0e-6);
+        bool ok = true;
+        double s = quotient<FEW>(quotient<FEW>(lm, dzw, ok), ws, ok);
+        if (FEW && !ok) s = jl_div(jl_div(lm, dzw), ws);
         s = jl_min(s, 1.0);
         A(LA_A, it.j, it.s) = jl_max(0.01, s);
       }
@@ -278,12 +313,20 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
           s1 = jl_min(s1, 1.0);
           s1 = jl_max(0.01, s1);
           const double e = 2.0 * b + 3.0;
-          const double hkv = imp * ks * cm_pow(s1, e);
-          const double smpv = -suc * cm_pow(sj, -b);
+          double p1, p2;
+          power_pair<FEW>(s1, e, sj, -b, p1, p2);
+          const double hkv = imp * ks * p1;
+          const double smpv = -suc * p2;
           A(LA_B, j, s) = hkv;
-          A(LA_C, j, s) = jl_div(e * hkv, s1);
           A(LA_R, j, s) = smpv;
-          A(LA_FN, j, s) = jl_div(jl_div(-b * smpv, sj), ws);
+          bool ok = true;
+          double dhk = quotient<FEW>(e * hkv, s1, ok), dsmp = quotient<FEW>(quotient<FEW>(-b * smpv, sj, ok), ws, ok);
+          if (FEW && !ok) {
+            dhk = jl_div(e * hkv, s1);
+            dsmp = jl_div(jl_div(-b * smpv, sj), ws);
+          }
+          A(LA_C, j, s) = dhk;
+          A(LA_FN, j, s) = dsmp;
           rec[PC_SMP * nls] = smpv;
           rec[PC_HK * nls] = hkv;
         }
@@ -302,13 +345,20 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
           double qo = 0.0, d1 = 0.0, d2 = 0.0;
           if (j < it.nl) {
             const double hd = half_of(dhkdw);
-            const double dhkds1 = jl_div(hd, ws);
-            const double dhkds2 = jl_div(hd, rec[PC_WS * nls + 1]);
+            const double wsn = rec[PC_WS * nls + 1], den = rec[PC_DEN * nls];
             const double num = A(LA_R, j + 1, s) - smp;
-            const double den = rec[PC_DEN * nls];
-            qo = jl_div(-hk * num, den) + hk;
-            d1 = jl_div(hk * dsmpdw - dhkds1 * num, den) + dhkds1;
-            d2 = jl_div(-hk * A(LA_FN, j + 1, s) - dhkds2 * num, den) + dhkds2;
+            bool ok = true;
+            double dhkds1 = quotient<FEW>(hd, ws, ok), dhkds2 = quotient<FEW>(hd, wsn, ok);
+            qo = quotient<FEW>(-hk * num, den, ok) + hk;
+            d1 = quotient<FEW>(hk * dsmpdw - dhkds1 * num, den, ok) + dhkds1;
+            d2 = quotient<FEW>(-hk * A(LA_FN, j + 1, s) - dhkds2 * num, den, ok) + dhkds2;
+            if (FEW && !ok) {
+              dhkds1 = jl_div(hd, ws);
+              dhkds2 = jl_div(hd, wsn);
+              qo = jl_div(-hk * num, den) + hk;
+              d1 = jl_div(hk * dsmpdw - dhkds1 * num, den) + dhkds1;
+              d2 = jl_div(-hk * A(LA_FN, j + 1, s) - dhkds2 * num, den) + dhkds2;
+            }
           } else {
             if (lower_bc == CLMGB_BC_WATERTABLE) {
               int jwt = nls;
@@ -455,7 +505,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
                                                     A(LA_D2, j, si) * A(LA_R, j + 1, si);
           fnet0 = qin_test - qout_test - pcache[cc * (int64_t)stride + PC_ROOT * nls + (j - 1)];
         } else {
-          fnet0 = jl_div(dw, A(LA_DT, j, si));
+          fnet0 = FEW ? div_chain(dw, A(LA_DT, j, si)) : jl_div(dw, A(LA_DT, j, si));
         }
         const long long ev = dbits(half_of(fabs(fnet1 - fnet0) * SA.dt[si])) & 0x7fffffffffffffffLL;
         fn = ev > 0x7ff0000000000000LL;
@@ -519,8 +569,8 @@ cudaError_t launch_moisture_form_packed(const Dims& D, int64_t nc, const clmgb_s
                                         int max_blocks, const QueueScratch& qs, cudaStream_t s) {
   const bool expensive = cfg.flux_calculation == 42;
   const size_t smem = (size_t)PWARPS * (size_t)warp_bytes(D.nlevsoi, expensive);
-  auto kern = log ? (expensive ? k_moisture_form_packed<true, true> : k_moisture_form_packed<true, false>)
-                  : (expensive ? k_moisture_form_packed<false, true> : k_moisture_form_packed<false, false>);
+  auto kern = log ? (expensive ? k_moisture_form_packed<true, true, false> : k_moisture_form_packed<true, false, false>)
+                  : (expensive ? k_moisture_form_packed<false, true, false> : k_moisture_form_packed<false, false, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int dev = 0, nsm = 0, nb = 0;
@@ -535,6 +585,10 @@ cudaError_t launch_moisture_form_packed(const Dims& D, int64_t nc, const clmgb_s
   int64_t kslots = (nc + grid * PWARPS - 1) / (grid * PWARPS);
   if (kslots > KS) kslots = KS;
   if (kslots < 1) kslots = 1;
+  if (!expensive && kslots <= FEW_SLOTS) {
+    kern = log ? k_moisture_form_packed<true, false, true> : k_moisture_form_packed<false, false, true>;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+  }
   kern<<<(unsigned)grid, PBLOCK, smem, s>>>(D, nc, f, cfg, dtime, col_status, or_status, dev_status, queue, order,
                                             nlisted, dt_init, log ? *log : SubstepLogView{nullptr, nullptr, 0, 0},
                                             (int)kslots, qs);
