@@ -90,7 +90,7 @@ def richards_launch_count(h, nc):
     """This library's kernels in one clmgb_soil_water call under the handle's schedule."""
     from clmgb import abi
     if h.get_option(abi.OPT_STEP_SCHEDULE) == abi.SCHEDULE_QUEUE and h.get_option(abi.OPT_RESERVED_COLUMNS) >= nc:
-        order = 3 if h.get_option(abi.OPT_QUEUE_ORDER) == 1 else 0
+        order = (1 if nc <= 4096 else 2) if h.get_option(abi.OPT_QUEUE_ORDER) == 1 else 0
         packed = h.get_option(abi.OPT_QUEUE_PACKED_REFRESH) == 1
         return 1 + order + 1 + (1 if packed else 0)
     return 1
@@ -710,8 +710,8 @@ def run_ours(args):
                 "note": "HBM is not the bound: the kernel runs thousands of FP64 operations per 2 KB of traffic. "
                         "fp64 is its FP64-pipe work in DFMA-equivalents (clmgb/flops_model.py, levels counted by "
                         "the kernel) over its time and the DFMA rate the probe measures on this device; its "
-                        "divisions run on the integer pipes (fp64.integer_pipe_divisions_per_launch), and with "
-                        "them off the FP64 pipe the kernel is bound by latency at 7-10 warps per SM; ncu "
+                        "divisions and powers run on the integer pipes (fp64.integer_pipe_divisions_per_launch), "
+                        "and the kernel is bound by the FP64 unit and their latency at 10 warps per SM; ncu "
                         "summaries in profiles/"}
 
     # end to end with the state in pinned host memory (clmgb.hoststep): each step moves
@@ -764,8 +764,9 @@ def run_ours(args):
 
     # this library's kernels per timed step: forcing, soil temperature, water fractions,
     # then the Richards call (work queue with reserved scratch: the impedance / column
-    # record pass, the three longest-first ordering kernels, the solve, and with the
-    # packed refresh the post-pass that writes the columns' outputs from their records)
+    # record pass, the longest-first ordering (one kernel up to 4,096 columns, else two), the
+    # solve, and with the packed solve the post-pass that writes the columns' outputs from
+    # their records)
     richards_launches = richards_launch_count(h, nc)
     launches_per_step = 3 + richards_launches
     if rank == 0:

@@ -10,7 +10,7 @@ after every accepted substep, plus that substep's water update):
     recurrence bet 2 and dwat 2, with the divisions gam = cmx/bet and dwat = ../bet;
     back substitution 2; error estimate fnet0 = dwat/dt_dz (a division) and 3 more:
     15 add/mul + 3 divisions per level
-  refresh (mfp_refresh, kernels.cu; :1280-1378, :1466-1470)
+  refresh (k_moisture_form_packed, richards_packed.cu; :1280-1378, :1466-1470)
     saturation: 2 divisions; hydraulic properties: 9 add/mul, 3 divisions and the two
     pow of s^(2b+3) and s^(-b); fluxes and derivatives: 13 add/mul and 5 divisions; net
     flux 2; the accepted substep's water update 3:
@@ -20,7 +20,7 @@ An add, subtract or multiply is one FP64 pipe instruction, as a DFMA is.  A pow
 (clm_math.h: fixed point on the integer pipes, with an FP64 fallback where its rounding
 test does not decide) is charged its time: the ratio of the DFMA rate to its rate, both
 measured on the device by the probe (clm.jl_gb300/probe/fp64_probe.cu).  The divisions run on the
-integer pipes (jl_div: cm_div's 64-bit reciprocal and 2/1 division), not on the FP64
+integer pipes (jl_div: cm_div's long division), not on the FP64
 pipe, so they add nothing to the FP64 work; they are counted separately.  The kernel
 counts the levels of its attempts and refreshes itself (CLMGB_OPT_COUNT_WORK), so
 
