@@ -365,6 +365,12 @@ cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soi
                                       const clmgb_step_adjoint& adj, const AdjTape& tp, const SubstepLogView& lg,
                                       const QueueScratch& qs, unsigned long long* queue, int grid_blocks,
                                       uint32_t* col_status, uint32_t* dev_status, cudaStream_t s) {
+  int64_t blocks = grid_blocks;
+  const int64_t max_blocks = tp.slots / CF_BLOCK;
+  if (blocks > max_blocks) blocks = max_blocks;
+  const int64_t need = (nc + CF_BLOCK - 1) / CF_BLOCK;
+  if (blocks > need) blocks = need;
+  if (blocks < 1) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
   const uint32_t* order = nullptr;
@@ -380,12 +386,6 @@ cudaError_t launch_column_step_vjp_cf(const Dims& D, int64_t nc, const clmgb_soi
                                  dev_status, s)) != cudaSuccess)
       return e;
   }
-  int64_t blocks = grid_blocks;
-  const int64_t max_blocks = tp.slots / CF_BLOCK;
-  if (blocks > max_blocks) blocks = max_blocks;
-  const int64_t need = (nc + CF_BLOCK - 1) / CF_BLOCK;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) return cudaErrorInvalidValue;
   CfSub S{tp.sub, (int)tp.maxsub, tp.slots};
   k_column_step_vjp_cf<<<(unsigned int)blocks, CF_BLOCK, 0, s>>>(D, nc, ft, fw, cfg, dtime, snow_method, t_ssbef,
                                                                  t_h2osfc_bef, adj, S, lg, queue, order,
