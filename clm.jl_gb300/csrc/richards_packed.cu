@@ -1,7 +1,7 @@
 // richards_packed.cu — the work-queue Richards solve (soilwm_moisture_form_solve!,
 // soil_water_movement.jl:1250-1489) with a warp's columns spread over its lanes.
 //
-// A warp owns up to KS = 16 columns at a time, its slots, and advances all of them by
+// A warp owns up to KS = 8 columns at a time, its slots, and advances all of them by
 // one substep attempt per loop trip; a slot whose column finishes takes the next column
 // of the queue.  On GB300 an FP64 instruction holds its sub-partition's FP64 unit for
 // about 65 cycles whatever the number of active lanes, so the work is laid out for few
@@ -11,17 +11,17 @@
 //     a time: the water update and the saturations, the hydraulic properties, the fluxes
 //     and their derivatives, the net fluxes (mf_refresh, after an accepted substep), the
 //     matrix entries and the error estimate (mf_attempt);
-//   * the forward sweep uses both half-warps: lane s < 16 carries column s's pivot
+//   * the forward sweep uses both half-warps: lane s carries column s's pivot
 //     (gam_j = c_{j-1}/bet_{j-1}, bet_j = b_j - a_j gam_j) and lane s + 16 its
 //     right-hand side one level behind (dwat_{j-1} = num_{j-1}/bet_{j-1}, num_j = r_j -
 //     a_j dwat_{j-1}): the same quotient, product and difference, so a level costs one
 //     division and two FP64 instructions for all the warp's columns;
-//   * back substitution on lanes s < 16.
+//   * back substitution on the lower half-warp.
 // A warp left with one long column therefore runs it at the latency of its own chain,
 // and nothing is handed over between warps.
 //
 // The level arrays live in the warp's shared memory, [array][level][slot] with a slot
-// stride of 17 doubles: items of consecutive levels and lanes of consecutive slots are
+// stride of 9 doubles: items of consecutive levels and lanes of consecutive slots are
 // both free of bank conflicts.  The soil parameters and the water stay in the columns'
 // records (k_column_records, records.cu), which the resident columns keep in L2.
 //
@@ -30,13 +30,12 @@
 //
 // Measured per call (scale workload, steps 5-24, ms), against the kernel with one column
 // per lane and a warp-per-column finish it replaced: 61 columns 1.88 -> 0.29, 1,024 4.06
-// -> 0.46, 16,384 6.27 -> 0.97, 65,536 6.90 -> 1.7, 262,144 9.94 -> 4.3.  What bounds
+// -> 0.46, 16,384 6.27 -> 0.98, 65,536 6.90 -> 1.65, 262,144 9.94 -> 4.03.  What bounds
 // it: at few columns the longest column's attempts, one after another (8 us each, half of it
-// the forward sweep and the back substitution); at many the FP64 unit and the latency of the
-// divisions and powers at 2.4 warps per sub-partition (ncu at 262,144 columns: FP64 unit 54 %
-// busy, issue slots 35 %).  Not warps: with three level arrays in the L2-resident records and
-// 15 or 18 warps per SM the solve took 4.5 and 4.33 ms for 4.30.  Not divisions: exact
-// quotients from kept 64-bit reciprocals, half the instructions, took 4.30.
+// the forward sweep and the back substitution); at many the FP64 unit, and the latency of the
+// divisions and powers.  Three or four level arrays in the L2-resident records instead, and
+// 18 warps of 16 columns, took 3.90 ms at 262,144 columns and 1.68 at 65,536, for 27 % more
+// scratch; exact quotients from 64-bit reciprocals kept there gained nothing.
 #include "clmgb_device.cuh"
 #include "launch.h"
 
@@ -45,14 +44,19 @@ namespace clmgb {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int KS = 16, SLD = KS + 1;
-// Columns per warp up to which an attempt's quotients and powers are formed in line (FEW): the
-// warp waits for its own chain, and independent ones overlap.  ms a call in line / through the
-// shared functions, scale workload: 61 columns 0.249 / 0.268, 1,024 0.459 / 0.486, 8,000 (6 a
-// warp) 0.796 / 0.838, 12,000 (8) 0.818 / 0.832, 24,000 (16) 1.094 / 1.057, 262,144 5.1 / 4.3:
-// warps in different phases no longer find the code in the instruction cache.
-constexpr int FEW_SLOTS = 8;
-constexpr int PWARPS = 5, PBLOCK = 32 * PWARPS;   // 2 blocks, 10 warps, of 20 levels on an SM
+constexpr int KS = 8, SLD = KS + 1, HALF = 16;     // slots, their stride, lanes of a half-warp
+// Up to FEW_SLOTS columns for each of FEW_WARPS warps a block the variant with an attempt's
+// quotients and powers in line runs (FEW): a warp waits for its own chain, and independent
+// ones overlap.  ms a call in line / through the shared functions, scale workload: 61 columns
+// 0.249 / 0.268, 1,024 0.459 / 0.486, 8,000 (6 a warp) 0.796 / 0.838, 12,000 (8) 0.818 /
+// 0.832; with warps in different phases, 24,000 columns on, the code is no longer found in the
+// instruction cache (262,144 5.1 / 4.3).
+constexpr int FEW_SLOTS = 8, FEW_WARPS = 5;
+// Many columns: 2 blocks, 18 warps of 8 columns and 20 levels, in an SM's shared memory.  ms a
+// call at 65,536 / 262,144 columns of the scale workload and at 262,144 of the snow workload:
+// 16 columns and 10 warps 1.72 / 4.27 / 1.65, 12 and 12 1.65 / 4.15 / 1.57, 10 and 14 1.65 /
+// 4.14 / 1.55, 8 and 18 1.65 / 4.03 / 1.42.
+constexpr int MANY_WARPS = 9;
 
 // level arrays: the flux derivatives dqodw1, dqodw2 and the net flux (kept from a
 // refresh to the next), dt_dz, and four that the sweeps of an attempt and the passes of a
@@ -102,7 +106,7 @@ __device__ __forceinline__ void power_pair(double x1, double y1, double x2, doub
 
 // FEW: for warps of few columns, whose attempts wait for their own quotients and powers
 template <bool LOG, bool EXPENSIVE, bool FEW>
-__global__ void __launch_bounds__(PBLOCK, 2)
+__global__ void __launch_bounds__(32 * (FEW ? FEW_WARPS : MANY_WARPS), 2)
 k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_config cfg, double dtime,
                        uint32_t* col_status, int or_status, uint32_t* dev_status, unsigned long long* queue,
                        const uint32_t* order, const unsigned int* nlisted_ptr, const double* dt_init,
@@ -116,7 +120,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
   const int lower_bc = cfg.lower_boundary_condition;
   const unsigned long long nq = order ? (unsigned long long)(*(volatile const unsigned int*)nlisted_ptr)
                                       : (unsigned long long)nc;
-  const unsigned long long nwarps = (unsigned long long)gridDim.x * PWARPS;
+  const unsigned long long nwarps = (unsigned long long)gridDim.x * (FEW ? FEW_WARPS : MANY_WARPS);
   const uint32_t magic = 65536u / (uint32_t)nls + 1u;       // t / nls for t < KS * 25
   // the tolerances as keys of non-negative doubles: e > upper and e < lower for e >= 0
   const long long key_up = cfg.xTolerUpper != cfg.xTolerUpper ? 0x7fffffffffffffffLL
@@ -436,8 +440,8 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
     }
     __syncwarp();
     // ---- Thomas forward sweep (:1421-1438) ----
-    const int s = lane & (KS - 1);
-    const bool up = lane >= KS;
+    const int s = lane & (HALF - 1);                        // lanes of no slot have no levels
+    const bool up = lane >= HALF;
     const int ns = ((am >> s) & 1u) ? SA.nl[s] : 0;
     const int nmax = (int)__reduce_max_sync(FULL, (unsigned)ns);
     {
@@ -568,30 +572,33 @@ cudaError_t launch_moisture_form_packed(const Dims& D, int64_t nc, const clmgb_s
                                         const unsigned int* nlisted, const double* dt_init, const SubstepLogView* log,
                                         int max_blocks, const QueueScratch& qs, cudaStream_t s) {
   const bool expensive = cfg.flux_calculation == 42;
-  const size_t smem = (size_t)PWARPS * (size_t)warp_bytes(D.nlevsoi, expensive);
-  auto kern = log ? (expensive ? k_moisture_form_packed<true, true, false> : k_moisture_form_packed<true, false, false>)
-                  : (expensive ? k_moisture_form_packed<false, true, false> : k_moisture_form_packed<false, false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  int dev = 0, nsm = 0, nb = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, PBLOCK, smem)) != cudaSuccess) return e;
+  const bool few = !expensive && nc <= (int64_t)2 * nsm * FEW_WARPS * FEW_SLOTS;
+  const int warps = few ? FEW_WARPS : MANY_WARPS;
+  const size_t smem = (size_t)warps * (size_t)warp_bytes(D.nlevsoi, expensive);
+  auto kern = log ? (few         ? k_moisture_form_packed<true, false, true>
+                     : expensive ? k_moisture_form_packed<true, true, false>
+                                 : k_moisture_form_packed<true, false, false>)
+                  : (few         ? k_moisture_form_packed<false, false, true>
+                     : expensive ? k_moisture_form_packed<false, true, false>
+                                 : k_moisture_form_packed<false, false, false>);
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+  int nb = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * warps, smem)) != cudaSuccess) return e;
   if (nb < 1) return cudaErrorInvalidConfiguration;
   int64_t grid = (int64_t)nb * nsm;
   if (grid > max_blocks) grid = max_blocks > 0 ? max_blocks : 1;
   // as few columns per warp as the resident warps allow: a column alone in its warp
   // finishes soonest, and at most KS share one
-  int64_t kslots = (nc + grid * PWARPS - 1) / (grid * PWARPS);
+  int64_t kslots = (nc + grid * warps - 1) / (grid * warps);
   if (kslots > KS) kslots = KS;
   if (kslots < 1) kslots = 1;
-  if (!expensive && kslots <= FEW_SLOTS) {
-    kern = log ? k_moisture_form_packed<true, false, true> : k_moisture_form_packed<false, false, true>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-  }
-  kern<<<(unsigned)grid, PBLOCK, smem, s>>>(D, nc, f, cfg, dtime, col_status, or_status, dev_status, queue, order,
-                                            nlisted, dt_init, log ? *log : SubstepLogView{nullptr, nullptr, 0, 0},
-                                            (int)kslots, qs);
+  kern<<<(unsigned)grid, 32 * warps, smem, s>>>(D, nc, f, cfg, dtime, col_status, or_status, dev_status, queue, order,
+                                                nlisted, dt_init, log ? *log : SubstepLogView{nullptr, nullptr, 0, 0},
+                                                (int)kslots, qs);
   return cudaGetLastError();
 }
 
