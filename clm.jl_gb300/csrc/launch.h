@@ -109,11 +109,11 @@ enum StLog {
 };
 static_assert(ST_END <= CLMGB_LOG_ST_STRIDE, "soil_temperature! record exceeds CLMGB_LOG_ST_STRIDE");
 
-// fields of a column record (QueueScratch::pcache): the inputs dz*1000, watsat, bsw,
-// hksat, sucsat, the ice impedance, 1000*(z[j+1]-z[j]) (levels below the bottom one)
-// and qflx_rootsoi; then the column's liquid water (the state's at the start, the
+// fields of a column record (QueueScratch::pcache): dz*1000, watsat, bsw, the ice
+// impedance times hksat, sucsat, the conductivity's exponent 2 bsw + 3, 1000*(z[j+1]-z[j])
+// (levels below the bottom one) and qflx_rootsoi; then the column's liquid water (the state's at the start, the
 // solve's at its end), smp_l and hk_l (written at every hydraulic refresh)
-enum PcField { PC_DZW = 0, PC_WS, PC_BSW, PC_KS, PC_SUC, PC_IMP, PC_DEN, PC_ROOT, PC_FIELDS,
+enum PcField { PC_DZW = 0, PC_WS, PC_BSW, PC_IK, PC_SUC, PC_EXP, PC_DEN, PC_ROOT, PC_FIELDS,
                PC_LIQ = PC_FIELDS, PC_SMP, PC_HK, PC_ALL };
 
 // All launchers return the cudaError_t of the launch (cudaGetLastError()).

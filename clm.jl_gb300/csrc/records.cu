@@ -153,9 +153,9 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
     v[e][PC_DZW] = TL(RI_DZ, j, cl) * DENH2O;
     v[e][PC_WS] = TL(RI_WS, j, cl);
     v[e][PC_BSW] = TL(RI_BSW, j, cl);
-    v[e][PC_KS] = TL(RI_KS, j, cl);
+    v[e][PC_IK] = imp * TL(RI_KS, j, cl);
     v[e][PC_SUC] = TL(RI_SUC, j, cl);
-    v[e][PC_IMP] = imp;
+    v[e][PC_EXP] = 2.0 * TL(RI_BSW, j, cl) + 3.0;
     if (j < nlayers) v[e][PC_DEN] = M_TO_MM * (TL(RI_Z, j + 1, cl) - TL(RI_Z, j, cl));
     v[e][PC_ROOT] = TL(RI_ROOT, j, cl);
     v[e][PC_LIQ] = TL(RI_LIQ, j, cl);

@@ -309,17 +309,16 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
         if (it.ok) {
           const int j = it.j, s = it.s;
           double* rec = pcache + SA.c[s] * (int64_t)stride + (j - 1);
-          const double b = rec[PC_BSW * nls], imp = rec[PC_IMP * nls], ks = rec[PC_KS * nls];
+          const double b = rec[PC_BSW * nls], e = rec[PC_EXP * nls], ik = rec[PC_IK * nls];
           const double suc = rec[PC_SUC * nls], ws = rec[PC_WS * nls];
           const double sj = A(LA_A, j, s);
           double s1 = sj;
           if (j != it.nl) s1 = half_of(sj + A(LA_A, j + 1, s));
           s1 = jl_min(s1, 1.0);
           s1 = jl_max(0.01, s1);
-          const double e = 2.0 * b + 3.0;
           double p1, p2;
           power_pair<FEW>(s1, e, sj, -b, p1, p2);
-          const double hkv = imp * ks * p1;
+          const double hkv = ik * p1;
           const double smpv = -suc * p2;
           A(LA_B, j, s) = hkv;
           A(LA_R, j, s) = smpv;
