@@ -30,12 +30,15 @@
 //
 // Measured per call (scale workload, steps 5-24, ms), against the kernel with one column
 // per lane and a warp-per-column finish it replaced: 61 columns 1.88 -> 0.29, 1,024 4.06
-// -> 0.46, 16,384 6.27 -> 0.98, 65,536 6.90 -> 1.65, 262,144 9.94 -> 4.03.  What bounds
+// -> 0.46, 16,384 6.27 -> 0.98, 65,536 6.90 -> 1.65, 262,144 9.94 -> 3.84.  What bounds
 // it: at few columns the longest column's attempts, one after another (8 us each, half of it
 // the forward sweep and the back substitution); at many the FP64 unit, and the latency of the
 // divisions and powers.  Three or four level arrays in the L2-resident records instead, and
 // 18 warps of 16 columns, took 3.90 ms at 262,144 columns and 1.68 at 65,536, for 27 % more
-// scratch; exact quotients from 64-bit reciprocals kept there gained nothing.
+// scratch; exact quotients from 64-bit reciprocals kept there gained nothing.  The items'
+// loops are not unrolled: 3.84 ms against 3.99, the code stays smaller (ncu at 262,144 columns
+// with 18 warps: FP64 unit 70 % busy, issue slots 44 %, instruction fetch 1.7 of 9.8 cycles
+// a warp waits per instruction).
 #include "clmgb_device.cuh"
 #include "launch.h"
 
@@ -162,6 +165,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
   // done, with the other outputs behind the records.
   auto water_pass = [&](unsigned mask, unsigned upd, unsigned done) {
     const int T = list_slots(mask);
+#pragma unroll 1
     for (int t0 = 0; t0 < T; t0 += 32) {
       const Item it = item(t0 + lane, T);
       if (!it.ok) continue;
@@ -304,6 +308,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
     if (fm) {
       const int T = list_slots(fm);
       // hydraulic properties (:1288-1308): hk, dhkdw, smp, dsmpdw into LA_B, LA_C, LA_R, LA_FN
+#pragma unroll 1
       for (int t0 = 0; t0 < T; t0 += 32) {
         const Item it = item(t0 + lane, T);
         if (it.ok) {
@@ -337,6 +342,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
       __syncwarp();
       // fluxes and derivatives between levels (:1310-1345) and at the bottom (:1347-1370)
       constexpr int QO = EXPENSIVE ? LA_Q : LA_A;
+#pragma unroll 1
       for (int t0 = 0; t0 < T; t0 += 32) {
         const Item it = item(t0 + lane, T);
         if (it.ok) {
@@ -390,6 +396,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
       }
       __syncwarp();
       // net flux (:1372-1378); the inflow of level j > 1 is the outflow of level j-1
+#pragma unroll 1
       for (int t0 = 0; t0 < T; t0 += 32) {
         const Item it = item(t0 + lane, T);
         if (it.ok) {
@@ -407,6 +414,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
     }
     // ---- dt_dz and the matrix (:1380-1397) ----
     const int T = list_slots(am);
+#pragma unroll 1
     for (int t0 = 0; t0 < T; t0 += 32) {
       const Item it = item(t0 + lane, T);
       if (it.ok) {
@@ -491,6 +499,7 @@ k_moisture_form_packed(Dims D, int64_t nc, clmgb_soilwater_fields f, clmgb_swm_c
     // upper tolerance, not below the lower one, or NaN (which the maximum would be) ----
     bool e_up = false, e_nlo = false, e_nan = false;
     const int own0 = __popc(am & ((1u << lane) - 1u)) * nls;         // this slot's first item
+#pragma unroll 1
     for (int t0 = 0; t0 < T; t0 += 32) {
       const Item it = item(t0 + lane, T);
       bool fu = false, fl = false, fn = false;
