@@ -28,10 +28,12 @@
 // instructions and some 200 divisions one after another over a 4 KB stack: 562 us for
 // 61 columns and 700 for 1,000.  Measured per call (snow and frozen-soil columns, us),
 // that kernel and this: 61 columns 562 -> 66, 1,000 708 -> 78, 4,000 710 -> 112, 16,000 750
-// -> 187, 65,536 1,165 -> 648; 262,144 3,130 -> 2,760.  What bounds it: at few columns
+// -> 187, 65,536 1,165 -> 640; 262,144 3,130 -> 2,690.  What bounds it: at few columns
 // the chain of the banded solve (about 45 % of the time) and of the divisions; at many
-// (ncu, 131,072 columns) latency at 16 warps per SM, the FP64 unit 47 % busy, a third of
-// the warps' time at the block's barriers, most of it beside the banded solve.
+// (ncu, 262,144 columns) latency at 16 warps per SM, the FP64 unit 46 % busy, a third of
+// the warps' time at the block's barriers, most of it beside the banded solve, and a sixth
+// waiting for instructions.  The loops over patches and over single values of a level are not
+// unrolled for that reason (2.69 -> 2.62 ms).
 #include "clmgb_device.cuh"
 #include "launch.h"
 
@@ -151,6 +153,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
   double* const rec = LOG ? st_log + c * (int64_t)CLMGB_LOG_ST_STRIDE : nullptr;
   if (masked) {
     if (FRAC && t_ssbef)
+#pragma unroll 1
       for (int jj = 1 + lo; jj <= nlev; jj += nper) LV(t_ssbef, c, jj, ld) = LV(f.t_soisno, c, jj, ld);
     if (FRAC && t_h2osfc_bef && lo == 0) t_h2osfc_bef[c] = f.t_h2osfc[c];
     if (LOG && lo == 0) rec[ST_N] = 0.0;
@@ -271,6 +274,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
       if (pi < 1 || pf > D.np || pf < pi - 1) {
         bad_patches = 1;
       } else {
+#pragma unroll 1
         for (int64_t p1 = pi; p1 <= pf; p1++) {
           const int64_t p = p1 - 1;
           if (f.patch_column[p] != c + 1 + D.c0) continue;
@@ -432,6 +436,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
           if (j > jtop) {
             dzm = z0 - LVc(f.z, c, jj - 1, ld);
             if (j <= 1 && !bad_patches) {   // absorbed solar of the level (:1139-1167)
+#pragma unroll 1
               for (int64_t p1 = f.col_patchi[c]; p1 <= f.col_patchf[c]; p1++) {
                 const int64_t p = p1 - 1;
                 if (f.patch_column[p] != c + 1 + D.c0) continue;
@@ -692,6 +697,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
     }
     // the zeros phase_change_beta! starts the snow levels with, inactive ones included
     if (on)
+#pragma unroll 1
       for (int jj = 1 + lo; jj <= nlevsno; jj += nper) {
         LV(f.qflx_snomelt_lyr, c, jj, ld) = 0.0;
         LV(f.qflx_snofrz_lyr, c, jj, ld) = 0.0;
@@ -894,6 +900,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
       rec[ST_TH] = f.t_h2osfc[c];
     }
     if (snl_ok) {                                  // the levels the call may have changed
+#pragma unroll 1
       for (int jj = jtop + joff + lo; jj <= nlev; jj += nper) {
         rec[ST_T + jj - 1] = LV(f.t_soisno, c, jj, ld);
         rec[ST_LIQ + jj - 1] = LV(f.h2osoi_liq, c, jj, ld);
@@ -904,6 +911,7 @@ k_soil_temperature_packed(Dims D, int64_t nc, clmgb_soiltemp_fields f, clmgb_soi
   }
   // ---- set_soil_water_fractions! (soil_hydrology.jl:110-130) ----
   if (FRAC && in && fw.mask_hydrology[c])
+#pragma unroll 1
     for (int j = 1 + lo; j <= nlevsoi; j += nper) water_fractions_level(D, fw, c, j);
   if (in && lo == 0) {
     if (col_status) col_status[c] = st;
