@@ -599,7 +599,7 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
   const bool packed = use && qs.packed && qs.pcache && qs.poll_limit == DEFER_POLL_LIMIT && qs.publish_delay == 0;
   if (use) {
     if (packed) {
-      if ((e = launch_column_records(D, nc, f, cfg.e_ice, qs.imp, qs.capacity, qs.pcache, qs.records_tma != 0,
+      if ((e = launch_column_records(D, nc, f, cfg.e_ice, qs.pcache, qs.records_tma != 0,
                                      dev_status, s, qs.records_tma_used)) != cudaSuccess)
         return e;
     } else {

@@ -144,8 +144,8 @@ cudaError_t launch_synth_forcing(const Dims& D, int64_t nc, const clmgb_soiltemp
 // The column-record pre-pass of the work-queue Richards solve (records.cu)
 size_t column_records_smem(int nlevsoi);
 cudaError_t launch_column_records(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, double e_ice,
-                                  double* imp_cache, int64_t ld_imp, double* pcache, bool tma, uint32_t* dev_status,
-                                  cudaStream_t s, int* tma_used = nullptr);
+                                  double* pcache, bool tma, uint32_t* dev_status, cudaStream_t s,
+                                  int* tma_used = nullptr);
 bool column_records_tma_available();
 // writes the solved columns' water, smp_l and hk_l from their records to the state
 cudaError_t launch_column_outputs(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, const double* pcache,

@@ -1,8 +1,8 @@
 // records.cu — the pre-pass and the post-pass of the work-queue Richards solve.
 //
-// Pre-pass (k_column_records): every hydrology column's ice impedances (imp_cache,
-// [nlevsoi][ld_imp]) and its record (QueueScratch::pcache, [column][PC_ALL][nlevsoi]):
-// the packed refresh's inputs and the column's liquid water, by tiles of 32 columns.
+// Pre-pass (k_column_records): every hydrology column's record (QueueScratch::pcache,
+// [column][PC_ALL][nlevsoi]): the inputs of a refresh (PcField; the ice impedance formed
+// here) and the column's liquid water, by tiles of 32 columns.
 // A block stages the tile's levels of the nine fields it reads (dz, z, watsat, bsw,
 // hksat, sucsat, qflx_rootsoi, icefrac, h2osoi_liq: [level][column] arrays, columns
 // fastest) in shared memory, forms the record values of every (level, column) pair,
@@ -77,8 +77,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t phase) 
 
 template <bool TMA>
 __global__ void __launch_bounds__(RC_THREADS)
-k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, double* imp_cache, int64_t ld_imp,
-                 double* pcache, const __grid_constant__ RecordMaps maps, uint32_t* dev_status) {
+k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, double* pcache, const __grid_constant__ RecordMaps maps, uint32_t* dev_status) {
   extern __shared__ __align__(128) unsigned char rc_smem[];
   __shared__ __align__(8) unsigned long long bar;
   double* tile = reinterpret_cast<double*>(rc_smem);            // [RC_FIELDS_IN][nls][RC_COLS]
@@ -149,7 +148,6 @@ k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, dou
     const double icef = (j == nlayers) ? TL(RI_ICEF, j, cl) : 0.5 * (TL(RI_ICEF, j, cl) + TL(RI_ICEF, j + 1, cl));
     const double y = -e_ice * icef;
     const double imp = zero_bits(y) ? 1.0 : cm_pow(10.0, y);       // no ice: x^0
-    imp_cache[(int64_t)(j - 1) * ld_imp + c] = imp;
     v[e][PC_DZW] = TL(RI_DZ, j, cl) * DENH2O;
     v[e][PC_WS] = TL(RI_WS, j, cl);
     v[e][PC_BSW] = TL(RI_BSW, j, cl);
@@ -249,7 +247,7 @@ size_t column_records_smem(int nlevsoi) {
 }
 
 cudaError_t launch_column_records(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, double e_ice,
-                                  double* imp_cache, int64_t ld_imp, double* pcache, bool tma, uint32_t* dev_status,
+                                  double* pcache, bool tma, uint32_t* dev_status,
                                   cudaStream_t s, int* tma_used) {
   const int nls = D.nlevsoi;
   const size_t smem = column_records_smem(nls);
@@ -271,8 +269,7 @@ cudaError_t launch_column_records(const Dims& D, int64_t nc, const clmgb_soilwat
   auto kern = use_tma ? k_column_records<true> : k_column_records<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)((nc + RC_COLS - 1) / RC_COLS), RC_THREADS, smem, s>>>(D, nc, f, e_ice, imp_cache, ld_imp, pcache,
-                                                                          maps, dev_status);
+  kern<<<(unsigned)((nc + RC_COLS - 1) / RC_COLS), RC_THREADS, smem, s>>>(D, nc, f, e_ice, pcache, maps, dev_status);
   return cudaGetLastError();
 }
 
