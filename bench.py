@@ -711,7 +711,7 @@ def run_ours(args):
                         "fp64 is its FP64-pipe work in DFMA-equivalents (clmgb/flops_model.py, levels counted by "
                         "the kernel) over its time and the DFMA rate the probe measures on this device; its "
                         "divisions and powers run on the integer pipes (fp64.integer_pipe_divisions_per_launch), "
-                        "and the kernel is bound by the FP64 unit and their latency at 10 warps per SM; ncu "
+                        "and the kernel keeps the FP64 unit about 72 % busy at 17 warps per SM; ncu "
                         "summaries in profiles/"}
 
     # end to end with the state in pinned host memory (clmgb.hoststep): each step moves
