@@ -15,6 +15,8 @@ after every accepted substep, plus that substep's water update):
     pow of s^(2b+3) and s^(-b); fluxes and derivatives: 13 add/mul and 5 divisions; net
     flux 2; the accepted substep's water update 3:
     27 add/mul + 10 divisions + 2 pow per level
+    (three of the 27, the impedance times hksat and 2 bsw + 3, are formed once a call, in
+    the records' pre-pass)
 
 An add, subtract or multiply is one FP64 pipe instruction, as a DFMA is.  A pow
 (clm_math.h: fixed point on the integer pipes, with an FP64 fallback where its rounding
