@@ -75,8 +75,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t phase) 
   return true;
 }
 
+// three blocks per SM (80 registers): 187 us at 262,144 columns; two at the 98 registers that
+// the compiler chose otherwise 225, four at 64 191
 template <bool TMA>
-__global__ void __launch_bounds__(RC_THREADS)
+__global__ void __launch_bounds__(RC_THREADS, 3)
 k_column_records(Dims D, int64_t nc, clmgb_soilwater_fields f, double e_ice, double* pcache, const __grid_constant__ RecordMaps maps, uint32_t* dev_status) {
   extern __shared__ __align__(128) unsigned char rc_smem[];
   __shared__ __align__(8) unsigned long long bar;
