@@ -236,7 +236,7 @@ cudaError_t launch_richards_reverse(const Dims& D, int64_t nc, const clmgb_soilt
   const unsigned grid = (unsigned)((nc + RV_COLS - 1) / RV_COLS);
   const int threads = 32 * ((D.nlevsoi + 1) / 2);
   auto kern = threads <= 320 ? k_richards_reverse<320> : k_richards_reverse<32 * ((MAXSOI + 1) / 2)>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_dynamic_smem(kern, sizeof(double) * (size_t)RV_ARRAYS * (MAXSOI + 2) * RV_COLS);
   if (e != cudaSuccess) return e;
   kern<<<grid, threads, smem, s>>>(D, nc, ft, fw, cfg, dtime, adj, lg, order);
   return cudaGetLastError();

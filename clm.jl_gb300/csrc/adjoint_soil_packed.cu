@@ -298,7 +298,7 @@ cudaError_t launch_soil_reverse(const Dims& D, int64_t nc, const clmgb_soiltemp_
                                 const clmgb_soilwater_fields& fw, double dtime, int snow_method, double* t_ssbef,
                                 double* t_h2osfc_bef, const clmgb_step_adjoint& adj, const SubstepLogView& lg,
                                 const uint32_t* order, uint32_t* col_status, uint32_t* dev_status, cudaStream_t s) {
-  const cudaError_t e = cudaFuncSetAttribute(k_soil_reverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SV_SMEM);
+  const cudaError_t e = allow_dynamic_smem(k_soil_reverse, SV_SMEM);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((nc + SV_COLS - 1) / SV_COLS);
   k_soil_reverse<<<grid, SV_THREADS, SV_SMEM, s>>>(D, nc, ft, fw, dtime, snow_method, t_ssbef, t_h2osfc_bef, adj,

@@ -683,8 +683,7 @@ cudaError_t launch_tridiagonal_multi(int64_t ncols, int64_t ldc, int nlevs, doub
   else {
     const int nt = BLOCK;          // 64 KB at MAXTRI levels: three blocks on an SM
     const size_t smem = (size_t)nlevs * nt * sizeof(double);
-    const cudaError_t e = cudaFuncSetAttribute(k_tridiagonal_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+    const cudaError_t e = allow_dynamic_smem(k_tridiagonal_multi, (size_t)MAXTRI * nt * sizeof(double));
     if (e != cudaSuccess) return e;
     k_tridiagonal_multi<<<(unsigned)((ncols + nt - 1) / nt), nt, smem, s>>>(ncols, ldc, nlevs, u, a, b, c, r, jtop,
                                                                            mask);

@@ -116,6 +116,17 @@ static_assert(ST_END <= CLMGB_LOG_ST_STRIDE, "soil_temperature! record exceeds C
 enum PcField { PC_DZW = 0, PC_WS, PC_BSW, PC_IK, PC_SUC, PC_EXP, PC_DEN, PC_ROOT, PC_FIELDS,
                PC_LIQ = PC_FIELDS, PC_SMP, PC_HK, PC_ALL };
 
+// Lets a kernel be launched with up to `most` bytes of dynamic shared memory.  That limit
+// belongs to the function, and all threads and handles of the process share it: a call that
+// set it to its own need could lower it between another thread's setting and its launch,
+// which is then refused.  So `most` is the kernel's largest need, the same in every call, and
+// below what any kernel may use anyway (48 KB with its static arrays) nothing is set.
+template <class... A>
+cudaError_t allow_dynamic_smem(void (*kern)(A...), size_t most) {
+  if (most <= 40 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // All launchers return the cudaError_t of the launch (cudaGetLastError()).
 cudaError_t launch_soil_temperature(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& f, double dtime,
                                     int snow_method, uint32_t* col_status, uint32_t* dev_status,

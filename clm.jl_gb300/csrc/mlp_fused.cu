@@ -314,7 +314,7 @@ cudaError_t launch_mlp_forward(int64_t M, const void* X, const clmgb_mlp_net& ne
   if (M <= 0) return cudaSuccess;
   const bool keep = Z1 != nullptr;
   auto kern = keep ? k_mlp_forward<true> : k_mlp_forward<false>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FW_SMEM);
+  const cudaError_t e = allow_dynamic_smem(kern, FW_SMEM);
   if (e != cudaSuccess) return e;
   // two blocks fit an SM's shared memory; tiles go to blocks first, so that few of them
   // still spread over the SMs
@@ -350,9 +350,7 @@ cudaError_t launch_mlp_gradients(int64_t M, const void* X, const float* Z1, cons
     }
   }
   if (M <= 0) return cudaSuccess;
-  if ((e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BW_SMEM)) !=
-      cudaSuccess)
-    return e;
+  if ((e = allow_dynamic_smem(k_mlp_backward, BW_SMEM)) != cudaSuccess) return e;
   k_mlp_backward<<<(unsigned)((M + BR - 1) / BR), 32 * BW, BW_SMEM, s>>>(
       M, (const bf16*)X, Z1, (const bf16*)H1, Z2, (const bf16*)H2, (const bf16*)dY, (const bf16*)net.wt[1],
       (const bf16*)net.wt[2], g.dw[0], g.dw[1], g.dw[2], g.db[0], g.db[1], g.db[2]);

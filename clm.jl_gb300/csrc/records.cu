@@ -269,7 +269,7 @@ cudaError_t launch_column_records(const Dims& D, int64_t nc, const clmgb_soilwat
                  encode_map(&maps.m[RI_LIQ], f.h2osoi_liq + (int64_t)joff * ld, nc, nls, ld, nls);
   if (tma_used) *tma_used = use_tma ? 1 : 0;
   auto kern = use_tma ? k_column_records<true> : k_column_records<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_dynamic_smem(kern, column_records_smem(MAXSOI));
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)((nc + RC_COLS - 1) / RC_COLS), RC_THREADS, smem, s>>>(D, nc, f, e_ice, pcache, maps, dev_status);
   return cudaGetLastError();
@@ -280,7 +280,7 @@ bool column_records_tma_available() { return encode_fn() != nullptr; }
 cudaError_t launch_column_outputs(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f, const double* pcache,
                                   cudaStream_t s) {
   const size_t smem = (size_t)RC_COLS * (RO_FIELDS * D.nlevsoi + 1) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k_column_outputs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_dynamic_smem(k_column_outputs, (size_t)RC_COLS * (RO_FIELDS * MAXSOI + 1) * sizeof(double));
   if (e != cudaSuccess) return e;
   k_column_outputs<<<(unsigned)((nc + RC_COLS - 1) / RC_COLS), RC_THREADS, smem, s>>>(D, nc, f, pcache);
   return cudaGetLastError();

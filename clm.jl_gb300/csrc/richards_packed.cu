@@ -593,7 +593,7 @@ cudaError_t launch_moisture_form_packed(const Dims& D, int64_t nc, const clmgb_s
                   : (few         ? k_moisture_form_packed<false, false, true>
                      : expensive ? k_moisture_form_packed<false, true, false>
                                  : k_moisture_form_packed<false, false, false>);
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+  if ((e = allow_dynamic_smem(kern, (size_t)warps * (size_t)warp_bytes(MAXSOI, expensive))) != cudaSuccess) return e;
   int nb = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * warps, smem)) != cudaSuccess) return e;
   if (nb < 1) return cudaErrorInvalidConfiguration;

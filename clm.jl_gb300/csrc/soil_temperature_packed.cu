@@ -930,7 +930,8 @@ cudaError_t launch_form(const Dims& D, int64_t nc, const clmgb_soiltemp_fields& 
                         uint32_t* dev_status, double* st_log, int sh, cudaStream_t s) {
   const size_t smem = BLOCK ? (size_t)group_bytes<32>(32) : (size_t)TWARPS * (size_t)group_bytes<4>(1 << sh);
   auto kern = k_soil_temperature_packed<FRAC, LOG, BLOCK>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e =
+      allow_dynamic_smem(kern, BLOCK ? (size_t)group_bytes<32>(32) : (size_t)TWARPS * (size_t)group_bytes<4>(4));
   if (e != cudaSuccess) return e;
   const int64_t cols = BLOCK ? 32 : (int64_t)TWARPS << sh;
   int64_t grid = (nc + cols - 1) / cols;

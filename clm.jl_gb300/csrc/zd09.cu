@@ -291,7 +291,8 @@ template <bool BLOCK>
 cudaError_t launch_form(const Dims& D, int64_t nc, const clmgb_zd09_fields& f, double e_ice, double dtime, int sh,
                         cudaStream_t s) {
   const size_t smem = BLOCK ? (size_t)zd_bytes<32>(32, D.nlevsoi + 1) : (size_t)ZWARPS * (size_t)zd_bytes<4>(1 << sh, D.nlevsoi + 1);
-  const cudaError_t e = cudaFuncSetAttribute(k_zd09<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_dynamic_smem(k_zd09<BLOCK>, BLOCK ? (size_t)zd_bytes<32>(32, MAXSOI + 1)
+                                                               : (size_t)ZWARPS * (size_t)zd_bytes<4>(4, MAXSOI + 1));
   if (e != cudaSuccess) return e;
   const int64_t cols = BLOCK ? 32 : (int64_t)ZWARPS << sh;
   k_zd09<BLOCK><<<(unsigned)((nc + cols - 1) / cols), ZD_BLOCK, smem, s>>>(D, nc, f, e_ice, dtime, sh);
