@@ -594,9 +594,11 @@ cudaError_t launch_moisture_form_queue(const Dims& D, int64_t nc, const clmgb_so
   if (e != cudaSuccess) return e;
   if (log && (e = cudaMemsetAsync(log->count, 0xff, (size_t)nc * sizeof(int32_t), s)) != cudaSuccess) return e;
   const bool use = qs.capacity >= nc && qs.order && qs.bins && qs.imp;
-  // the packed kernel hands no column over; the options that test the hand-over's bounded
-  // wait (polls of a list slot, a late index) select the per-lane kernel, which does
-  const bool packed = use && qs.packed && qs.pcache && qs.poll_limit == DEFER_POLL_LIMIT && qs.publish_delay == 0;
+  // the packed kernel hands no column over, so the late index that tests the hand-over's
+  // bounded wait selects the per-lane kernel, which does; a limit of the polls alone has
+  // nothing to act on and leaves the solve to the packed kernel (65,536 columns 1.65 ms,
+  // the per-lane kernel 6.1)
+  const bool packed = use && qs.packed && qs.pcache && qs.publish_delay == 0;
   if (use) {
     if (packed) {
       if ((e = launch_column_records(D, nc, f, cfg.e_ice, qs.pcache, qs.records_tma != 0,

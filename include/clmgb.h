@@ -716,10 +716,10 @@ int32_t clmgb_last_cuda_error(clmgb_handle h);
 #define CLMGB_OPT_ATTEMPT_CAP         18 /* Richards substep attempts after which a column stops with
                                             CLMGB_COL_SUBSTEP_CAP (1..4096, default 4096: never reached by a
                                             valid configuration, whose attempts dtmin bounds) */
-#define CLMGB_OPT_QUEUE_POLL_LIMIT    19 /* polls of a deferred column's list slot before the finishing warp
-                                            gives the slot back to the deferring lane (0..2^20, default
-                                            2^20; any other value selects the per-lane kernel).
-                                            Results do not depend on it. */
+#define CLMGB_OPT_QUEUE_POLL_LIMIT    19 /* per-lane work-queue Richards kernel: polls of a deferred column's
+                                            list slot before the finishing warp gives the slot back to the
+                                            deferring lane (0..2^20, default 2^20).  Results do not depend
+                                            on it. */
 #define CLMGB_OPT_QUEUE_PUBLISH_DELAY 20 /* for tests of the bounded wait: a deferring lane counts an even
                                             list slot published before writing the column's index, and
                                             writes it once a finishing warp has taken the slot or after
