@@ -378,7 +378,7 @@ __device__ __forceinline__ StLayer st_layer(const StCol& C, const Dims& D, const
     const double cdke = spass ? (dksat - tkdry) * ddke * rm : 0.0;
     r.dl = rv_fma(kfl, (1.0 - fl) * (1.0 / DENH2O), cdke * (1.0 / DENH2O));
     r.di = rv_fma(kfl, -fl * (1.0 / DENICE), cdke * (1.0 / DENICE));
-    r.dw = rv_fma(dk, mix, -cdke * (satw0 * dzv));
+    r.dw = rv_fma(dk, mix, spass ? -cdke * (satw0 * dzv) : -0.0);      // satw0 may be infinite where it is clamped
     return r;
   }
   const double denom = jl_max(C.fse, 1.0e-6) * jl_max(LVc(f.dz, c, jj, ld), 1.0e-6);
