@@ -78,6 +78,9 @@ __device__ __forceinline__ void column_features(const Dims& D, const clmgb_soilw
     x[j - 1] = sv;
     x[19 + j] = in ? (float)LV(f.icefrac, c, j, ld) : 0.0f;
   }
+  constexpr int next = FEAT_LEVELS + 1;               // below the last level of the features
+  if (nlayers >= next)
+    s[next] = feature_saturation(liq(next), LVc(f.dz, c, D.nlevsno + next, ld), LVc(f.watsat, c, next, ld));
   for (int j = 1; j <= FEAT_LEVELS; j++)
     x[39 + j] = j > nlayers ? -30.0f
                             : feature_log_conductivity(j == nlayers, s[j], s[j + 1], LV(f.icefrac, c, j, ld),
@@ -374,7 +377,11 @@ k_mlp_features(Dims D, int64_t nc, clmgb_soilwater_fields f, float e_ice, float 
     sat[j][col] = sv[i];
     root[j][col] = in ? (float)rt[i] : 0.0f;
   }
-  if (part == 0) sat[FEAT_LEVELS + 1][col] = 0.0f;
+  constexpr int next = FEAT_LEVELS + 1;               // a level below those of the features
+  if (part == 0)
+    sat[next][col] = nl >= next ? feature_saturation(LV(f.h2osoi_liq, c, D.nlevsno + next, ld),
+                                                     LVc(f.dz, c, D.nlevsno + next, ld), LVc(f.watsat, c, next, ld))
+                                : 0.0f;
   __syncthreads();
   auto put = [&](int i, float x) { out[col][i] = __float2bfloat16((x - norm[0][i]) * norm[1][i]); };
 #pragma unroll
