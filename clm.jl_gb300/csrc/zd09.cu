@@ -150,7 +150,8 @@ k_zd09(Dims D, int64_t nc, clmgb_zd09_fields f, double e_ice, double dtime, int 
     if (deep) {
       const double suc = LVc(f.sucsat, c, j, ld), ws = LVc(f.watsat, c, j, ld), b = LVc(f.bsw, c, j, ld);
       double vwc_zwt = ws;
-      if (LVc(f.t_soisno, c, joff + jwt + 1, ld) < TFRZ) {
+      // the level below the soil column, or the last one where the grid has none below
+      if (LVc(f.t_soisno, c, joff + min(jwt + 1, nlevgrnd), ld) < TFRZ) {
         double v = A(Z_VWC, j);
         for (int k = nls; k <= nlevgrnd; k++) {
           if (zwt_m <= LVc(f.zi, c, joff_zi + k, ld)) {

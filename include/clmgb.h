@@ -859,7 +859,9 @@ int32_t clmgb_lake_temperature(clmgb_handle h, const clmgb_bounds* b, const clmg
  * aquifer recharge qcharge and the water deficit.  cfg must select
  * CLMGB_ZENGDECKER_2009 with the CLMGB_BC_AQUIFER lower boundary (the reference's
  * init_soilwater_movement rejects any other pair, :681-705).  clmgb_soil_water returns
- * CLMGB_ERR_UNSUPPORTED for this method: its fields are these. */
+ * CLMGB_ERR_UNSUPPORTED for this method: its fields are these.  Where the water table lies
+ * below the soil column the method asks for the temperature of the level below it (:289-327);
+ * with nlevsoi = nlevgrnd that is the last level's. */
 int32_t clmgb_soil_water_zd09(clmgb_handle h, const clmgb_bounds* b, const clmgb_zd09_fields* f,
                               const clmgb_swm_config* cfg, double dtime, void* stream);
 

@@ -2699,7 +2699,8 @@ int orc_soil_water_zd09(const clmgb_varpar* vp, const clmgb_bounds* b, const clm
       if (f->zwt[c] <= IX(f->zi, c, joff_zi + j, ld)) { jw = j - 1; break; }
     jwt[c] = jw;
     vwc_zwt[c] = IX(f->watsat, c, nlevsoi, ld);
-    if (IX(f->t_soisno, c, joff + jw + 1, ld) < TFRZ) {
+    /* the level below the table's, or the last ground level where the grid has none below */
+    if (IX(f->t_soisno, c, joff + (jw < nlevgrnd ? jw + 1 : nlevgrnd), ld) < TFRZ) {
       double v = SC(M[VWC], c, nlevsoi);
       for (int j = nlevsoi; j <= nlevgrnd; j++) {
         if (f->zwt[c] <= IX(f->zi, c, joff_zi + j, ld)) {
