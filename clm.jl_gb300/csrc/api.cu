@@ -1236,7 +1236,8 @@ int32_t clmgb_mlp_gradients(clmgb_handle h, int64_t M, const uint16_t* X, const 
     if (!grad->dw[i] || !grad->db[i]) return CLMGB_ERR_NULL_ARG;
   if (!aligned16({X, Z1, H1, Z2, H2, dY, net->wt[1], net->wt[2], grad->dw[0], grad->dw[1], grad->dw[2]}))
     return CLMGB_ERR_UNSUPPORTED;
-  cudaError_t ce = clmgb::launch_mlp_gradients(M, X, Z1, H1, Z2, H2, dY, *net, *grad, (cudaStream_t)stream);
+  cudaError_t ce = clmgb::launch_mlp_gradients(M, X, Z1, H1, Z2, H2, dY, *net, *grad, h->num_sms,
+                                                 (cudaStream_t)stream);
   return ce == cudaSuccess ? CLMGB_OK : cuda_fail(h, ce);
 }
 

@@ -260,7 +260,7 @@ cudaError_t launch_mlp_forward(int64_t M, const void* X, const clmgb_mlp_net& ne
                                void* H2, float* Y, int num_sms, cudaStream_t s);
 cudaError_t launch_mlp_gradients(int64_t M, const void* X, const float* Z1, const void* H1, const float* Z2,
                                  const void* H2, const void* dY, const clmgb_mlp_net& net, const clmgb_mlp_grad& g,
-                                 cudaStream_t s);
+                                 int num_sms, cudaStream_t s);
 cudaError_t launch_mlp_adam_net(const clmgb_mlp_net& net, const clmgb_mlp_grad& g, float lr, float b1, float b2,
                                 float eps, int step, cudaStream_t s);
 cudaError_t launch_richards_samples(const Dims& D, int64_t nc, const clmgb_soilwater_fields& f,

@@ -6,14 +6,14 @@
 // launches, not by its products: layer by layer each kernel read its weights and its input
 // element by element and the next one read back what it wrote.  Here the weights stay in
 // shared memory, a warp takes its rows through all layers with the activations in shared
-// memory, and operands come in 16-byte loads and ldmatrix.  The products are mma.sync
+// memory, and operands come in 16-byte loads and ldmatrix.  The layers' products are mma.sync
 // m16n8k16 (BF16 x BF16 -> FP32) in the same order as in mlp.cu, and activations round to
-// BF16 at the same places, so the forward pass and the backward signals are the same bits;
-// only the weight gradients sum their rows in another order (tensor-core partial sums per
-// 64 rows instead of CUDA-core ones per 128, then the same FP32 atomics).
+// BF16 at the same places, so the forward pass and the backward signals are the same bits; the
+// weight gradients sum their rows on the CUDA cores as there, 128 rows a block and an atomic
+// addition a block.
 //
-// Device time of a training step of 4,096 rows: about 190 -> 47 us (forward 15, loss 3,
-// backward 24, optimiser 3); the step is the host's (eight allocations and four calls,
+// Device time of a training step of 4,096 rows: about 175 -> 53 us (forward 14, loss 4,
+// backward 32, optimiser 3); the step is the host's (eight allocations and four calls,
 // 155 us against 225 us with one call per layer).  Forward of 131,072 rows without
 // activations kept: 257 -> 64 us, the warps waiting on shared memory and on the exponentials
 // and divisions of SiLU (tensor pipe 18 % active, issue 41 %).
@@ -32,10 +32,6 @@ constexpr int LDI = NI + 8, LDH = NH + 8, LDO = NO + 8;   // padded rows: ldmatr
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm(uint32_t* r, uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void ldsm_t(uint32_t* r, uint32_t a) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -170,39 +166,55 @@ k_mlp_forward(int64_t M, const bf16* __restrict__ X, const bf16* __restrict__ W1
   }
 }
 
-// dW [N x K] += the 64 rows of dz^T x: warp w of BW takes output tiles of 16 x 8, neighbours
-// in K, so that a tile row's operand is loaded once
-constexpr int BR = 64, BW = 8;                      // rows and warps of a backward block
-template <int N, int K>
-__device__ __forceinline__ void weight_gradient(const bf16* dz, int ldz, const bf16* x, int ldx, float* dW) {
-  constexpr int PER = (N / 16) * (K / 8) / BW;      // 16 x 8 tiles per warp
-  static_assert(PER * BW == (N / 16) * (K / 8) && (K / 8) % PER == 0 && PER % 2 == 0, "tiles of one row per warp");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int n0 = warp * PER / (K / 8) * 16, k0 = warp * PER % (K / 8) * 8;
-  const uint32_t za = smem_addr(dz + ((lane & 7) + (lane >> 4) * 8) * ldz + n0 + ((lane >> 3) & 1) * 8);
-  const uint32_t xa = smem_addr(x + ((lane & 7) + ((lane >> 3) & 1) * 8) * ldx + k0 + (lane >> 4) * 8);
-  float acc[PER][4];
+// T consecutive BF16 values on a boundary of their size, as floats
+template <int T>
+__device__ __forceinline__ void load_floats(const bf16* p, float* v) {
+  uint32_t u[(T + 1) / 2];
+  if constexpr (T == 1) u[0] = *reinterpret_cast<const uint16_t*>(p);
+  else if constexpr (T == 2) u[0] = *reinterpret_cast<const uint32_t*>(p);
+  else if constexpr (T == 4) *reinterpret_cast<uint2*>(u) = *reinterpret_cast<const uint2*>(p);
+  else *reinterpret_cast<uint4*>(u) = *reinterpret_cast<const uint4*>(p);
 #pragma unroll
-  for (int i = 0; i < PER; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+  for (int i = 0; i < T; i++) v[i] = __uint_as_float(i & 1 ? u[i / 2] & 0xffff0000u : u[i / 2] << 16);
+}
+
+// dW [N x K] += the block's rows of dz^T x, rows `part` of S parts of dW: a tile of TN x TK
+// for each thread, its sums in FP32 rounded to nearest, row after row, then one atomic
+// addition: the additions of k_linear_dw (mlp.cu), whose partial sums these are bit for bit.
+// (On the tensor cores, whose sums of 16 products are truncated, and by 64 rows, which
+// doubles the atomic additions, the error against 64-bit sums was 1.1 times this at 16 rows
+// and 1.4 to 1.6 times from 1,000 rows on.)
+constexpr int BR = 128, BW = 16;                    // rows and warps of a backward block
+template <int N, int K, int S>
+__device__ __forceinline__ void weight_gradient(const bf16* dz, int ldz, const bf16* x, int ldx, float* dW, int part) {
+  constexpr int PER = N / S * K / (32 * BW), TK = PER < 4 ? PER : 4, TN = PER / TK;
+  static_assert(TN * TK * 32 * BW == N / S * K && K % TK == 0, "a tile per thread");
+  const int n0 = part * (N / S) + threadIdx.x / (K / TK) * TN, k0 = threadIdx.x % (K / TK) * TK;
+  float acc[TN][TK];
 #pragma unroll
-  for (int m = 0; m < BR; m += 16) {
-    uint32_t a[4];
-    ldsm_t(a, za + m * ldz * 2);
+  for (int a = 0; a < TN; a++)
 #pragma unroll
-    for (int i = 0; i < PER / 2; i++) {
-      uint32_t b[4];
-      ldsm_t(b, xa + (m * ldx + i * 16) * 2);
-      mma(acc[2 * i], a, b[0], b[1]);
-      mma(acc[2 * i + 1], a, b[2], b[3]);
-    }
+    for (int b = 0; b < TK; b++) acc[a][b] = 0.0f;
+#pragma unroll 4
+  for (int m = 0; m < BR; m++) {
+    float zn[TN], xk[TK];
+    load_floats<TN>(dz + m * ldz + n0, zn);
+    load_floats<TK>(x + m * ldx + k0, xk);
+#pragma unroll
+    for (int a = 0; a < TN; a++)
+#pragma unroll
+      for (int b = 0; b < TK; b++) acc[a][b] = fmaf(zn[a], xk[b], acc[a][b]);
   }
 #pragma unroll
-  for (int i = 0; i < PER; i++)
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float* p = dW + (n0 + g + 8 * h) * K + k0 + i * 8 + 2 * t;
-      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(acc[i][2 * h]), "f"(acc[i][2 * h + 1]) : "memory");
-    }
+  for (int a = 0; a < TN; a++) {
+    float* p = dW + (n0 + a) * K + k0;
+    if constexpr (TK == 4)
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(acc[a][0]), "f"(acc[a][1]),
+                   "f"(acc[a][2]), "f"(acc[a][3])
+                   : "memory");
+    else
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(acc[a][0]), "f"(acc[a][1]) : "memory");
+  }
 }
 
 // db += the columns' sums over the block's rows
@@ -210,6 +222,7 @@ template <int N>
 __device__ __forceinline__ void bias_gradient(const bf16* dz, int ldz, float* db) {
   if (threadIdx.x < N) {
     float s = 0.0f;
+#pragma unroll 16
     for (int m = 0; m < BR; m++) s += __bfloat162float(dz[m * ldz + threadIdx.x]);
     atomicAdd(&db[threadIdx.x], s);
   }
@@ -243,8 +256,10 @@ __device__ __forceinline__ void signal(float (*acc)[4], const float* Z, int64_t 
 constexpr size_t BW_SMEM = sizeof(bf16) * (size_t)(NH * LDO + NH * LDH + BR * (LDO + 3 * LDH + LDI));
 
 // The backward pass over BR rows per block: dZ2 = silu'(Z2) (dY W3), dZ1 = silu'(Z1) (dZ2
-// W2) in shared memory, and the block's share of the three weight and bias gradients.
-// w3t, w2t: the transposed weights [in x out].  grad: dW1, dW2, dW3, db1, db2, db3.
+// W2) in shared memory, and the block's share of the three weight and bias gradients.  S
+// blocks share the rows' weight gradients, each with the signals formed again.
+// w3t, w2t: the transposed weights [in x out].
+template <int S>
 __global__ void __launch_bounds__(32 * BW)
 k_mlp_backward(int64_t M, const bf16* __restrict__ X, const float* __restrict__ Z1, const bf16* __restrict__ H1,
                const float* __restrict__ Z2, const bf16* __restrict__ H2, const bf16* __restrict__ dY,
@@ -269,19 +284,20 @@ k_mlp_backward(int64_t M, const bf16* __restrict__ X, const float* __restrict__ 
   // warp w: rows 16 (w / 2) .. and columns 64 (w % 2) .. of the backward signals
   const int row = (warp >> 1) * 16, half = (warp & 1) * (NH / 2);
   float acc[NH / 16][4];
+  const int part = S > 1 ? (int)blockIdx.y : 0;
   tile_product<NO, NH / 2>(acc, dy + row * LDO, LDO, s3 + half * LDO, LDO);
   signal<NH / 2>(acc, Z2 + (r0 + row) * NH + half, valid - row, dz2 + row * LDH + half);
-  weight_gradient<NO, NH>(dy, LDO, act, LDH, dW3);
-  bias_gradient<NO>(dy, LDO, db3);
+  weight_gradient<NO, NH, S>(dy, LDO, act, LDH, dW3, part);
+  if (part == 0) bias_gradient<NO>(dy, LDO, db3);
   __syncthreads();                                             // dz2 is written, H2 read
   stage<NH>(act, LDH, H1 + r0 * NH, BR, valid, tid, 32 * BW);
   tile_product<NH, NH / 2>(acc, dz2 + row * LDH, LDH, s2 + half * LDH, LDH);
   signal<NH / 2>(acc, Z1 + (r0 + row) * NH + half, valid - row, dz1 + row * LDH + half);
   __syncthreads();
-  weight_gradient<NH, NH>(dz2, LDH, act, LDH, dW2);
-  bias_gradient<NH>(dz2, LDH, db2);
-  weight_gradient<NH, NI>(dz1, LDH, xs, LDI, dW1);
-  bias_gradient<NH>(dz1, LDH, db1);
+  weight_gradient<NH, NH, S>(dz2, LDH, act, LDH, dW2, part);
+  if (part == 0) bias_gradient<NH>(dz2, LDH, db2);
+  weight_gradient<NH, NI, S>(dz1, LDH, xs, LDI, dW1, part);
+  if (part == S - 1) bias_gradient<NH>(dz1, LDH, db1);
 }
 
 // One Adam step over the six parameter arrays (the expressions of k_adam)
@@ -327,7 +343,7 @@ cudaError_t launch_mlp_forward(int64_t M, const void* X, const clmgb_mlp_net& ne
 
 cudaError_t launch_mlp_gradients(int64_t M, const void* X, const float* Z1, const void* H1, const float* Z2,
                                  const void* H2, const void* dY, const clmgb_mlp_net& net, const clmgb_mlp_grad& g,
-                                 cudaStream_t s) {
+                                 int num_sms, cudaStream_t s) {
   static const size_t wn[3] = {(size_t)NH * NI, (size_t)NH * NH, (size_t)NO * NH}, bn[3] = {NH, NH, NO};
   cudaError_t e;
   // one clear where the six arrays are one range, as the caller of this library lays them out
@@ -350,8 +366,13 @@ cudaError_t launch_mlp_gradients(int64_t M, const void* X, const float* Z1, cons
     }
   }
   if (M <= 0) return cudaSuccess;
-  if ((e = allow_dynamic_smem(k_mlp_backward, BW_SMEM)) != cudaSuccess) return e;
-  k_mlp_backward<<<(unsigned)((M + BR - 1) / BR), 32 * BW, BW_SMEM, s>>>(
+  // as many blocks to the rows as keep all of them resident at once (a block fills an SM); us
+  // for 1, 2 and 4: 4,096 rows 49 / 38 / 32, 9,000 50 / 38 / 61, 16,384 50 / 74 / 117
+  const int64_t blocks = (M + BR - 1) / BR;
+  const int split = blocks * 4 <= num_sms ? 4 : blocks * 2 <= num_sms ? 2 : 1;
+  auto kern = split == 4 ? k_mlp_backward<4> : split == 2 ? k_mlp_backward<2> : k_mlp_backward<1>;
+  if ((e = allow_dynamic_smem(kern, BW_SMEM)) != cudaSuccess) return e;
+  kern<<<dim3((unsigned)blocks, (unsigned)split), 32 * BW, BW_SMEM, s>>>(
       M, (const bf16*)X, Z1, (const bf16*)H1, Z2, (const bf16*)H2, (const bf16*)dY, (const bf16*)net.wt[1],
       (const bf16*)net.wt[2], g.dw[0], g.dw[1], g.dw[2], g.db[0], g.db[1], g.db[2]);
   return cudaGetLastError();
