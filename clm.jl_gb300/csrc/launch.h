@@ -45,8 +45,9 @@ struct QueueScratch {
   // production: it lets a test make that wait run out)
   int poll_limit = DEFER_POLL_LIMIT;
   int publish_delay = 0;
-  // CLMGB_OPT_COUNT_WORK: when set, the packed kernel adds the levels of every substep
-  // attempt to work[0] and of every hydraulic refresh to work[1] (the FP64 work model of the solve, clmgb/flops_model.py); NULL otherwise
+  // CLMGB_OPT_COUNT_WORK: when set, the packed kernel and the warp-per-column finish add
+  // the levels of every substep attempt to work[0] and of every hydraulic refresh to
+  // work[1] (the FP64 work model of the solve, clmgb/flops_model.py); NULL otherwise
   unsigned long long* work = nullptr;
   // CLMGB_OPT_RECORDS_TMA: the column-record pre-pass stages its tiles with tensor copies
   int records_tma = 1;

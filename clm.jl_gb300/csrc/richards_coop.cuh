@@ -115,6 +115,10 @@ __device__ __noinline__ void coop_finish_column(const Dims& D, const clmgb_soilw
       dt_dz = jl_div(dtsub, M_TO_MM * dzv);
       dt_cur = dtsub;
     }
+    if (qs.work && lane == 0) {
+      atomicAdd(qs.work, (unsigned long long)n);             // an attempt over n levels
+      if (fresh) atomicAdd(qs.work + 1, (unsigned long long)n);
+    }
     if (fresh) {
       // hydraulic properties (mf_refresh, :1280-1308)
       double s2 = 0.0;

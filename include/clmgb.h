@@ -727,10 +727,11 @@ int32_t clmgb_last_cuda_error(clmgb_handle h);
                                             as long (0..1e7, default 0: index first, no lingering; any
                                             other value selects the per-lane kernel).  Results do not
                                             depend on it. */
-#define CLMGB_OPT_COUNT_WORK          21 /* 1: the work-queue Richards kernel with reserved scratch (the packed
-                                            kernel) counts, over the calls that follow, the levels of every
-                                            substep attempt and of every hydraulic refresh (setting 1 zeroes
-                                            the counts; 0 = off, the default) */
+#define CLMGB_OPT_COUNT_WORK          21 /* 1: the packed work-queue Richards kernel (reserved scratch) counts,
+                                            over the calls that follow, the levels of every substep attempt
+                                            and of every hydraulic refresh; with the per-lane kernel only
+                                            the warp-per-column finish of the columns that it hands over
+                                            does (setting 1 zeroes the counts; 0 = off, the default) */
 #define CLMGB_OPT_WORK_LEVEL_ATTEMPTS 22 /* read-only (synchronises): that count of attempt levels */
 #define CLMGB_OPT_WORK_LEVEL_REFRESHES 23 /* read-only (synchronises): that count of refreshed levels */
 #define CLMGB_OPT_RECORDS_TMA         24 /* the Richards pre-pass stages each tile of 32 columns with 2-D
