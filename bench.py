@@ -88,6 +88,7 @@ def richards_launch_count(h, nc):
     """This library's kernels in one clmgb_soil_water call under the handle's schedule."""
     from clmgb import abi
     if h.get_option(abi.OPT_STEP_SCHEDULE) == abi.SCHEDULE_QUEUE and h.get_option(abi.OPT_RESERVED_COLUMNS) >= nc:
+        # one kernel up to ORDER_ONE_MAX columns (csrc/work_order.cuh)
         order = (1 if nc <= 4096 else 2) if h.get_option(abi.OPT_QUEUE_ORDER) == 1 else 0
         packed = h.get_option(abi.OPT_QUEUE_PACKED_REFRESH) == 1
         return 1 + order + 1 + (1 if packed else 0)
@@ -704,11 +705,13 @@ def run_ours(args):
                 "step_achieved_gbs": step_bytes / (elapsed_ms / args.steps / 1000.0) / 1e9,
                 "fp64": fp64, "fp64_frac": fp64["frac"] if fp64 else None,
                 "note": "HBM is not the bound: the kernel runs thousands of FP64 operations per 2 KB of traffic. "
-                        "fp64 is its FP64-pipe work in DFMA-equivalents (clmgb/flops_model.py, levels counted by "
-                        "the kernel) over its time and the DFMA rate the probe measures on this device; its "
-                        "divisions and powers run on the integer pipes (fp64.integer_pipe_divisions_per_launch), "
-                        "and the kernel keeps the FP64 unit about 72 % busy at 17 warps per SM; ncu "
-                        "summaries in profiles/"}
+                        "fp64 is the solve's arithmetic in DFMA-equivalents (clmgb/flops_model.py, levels counted by "
+                        "the kernel; a power is charged its measured time) over its time and the "
+                        "DFMA rate the probe measures on this device. Its divisions and powers run on the integer "
+                        "pipes (fp64.integer_pipe_divisions_per_launch, integer_pipe_powers_per_launch); what it "
+                        "issues to the FP64 pipe is fp64.fp64_operations_per_launch, counted by working lanes. The "
+                        "FP64 unit is busy for longer (70 to 72 % in ncu at 17 warps per SM), since an instruction "
+                        "holds it the same time whatever the lanes; ncu summaries in profiles/"}
 
     # end to end with the state in pinned host memory (clmgb.hoststep): each step moves
     # the fields it reads that the rest of the model changes (parameters, geometry and
