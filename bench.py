@@ -710,7 +710,7 @@ def run_ours(args):
                         "DFMA rate the probe measures on this device. Its divisions and powers run on the integer "
                         "pipes (fp64.integer_pipe_divisions_per_launch, integer_pipe_powers_per_launch); what it "
                         "issues to the FP64 pipe is fp64.fp64_operations_per_launch, counted by working lanes. The "
-                        "FP64 unit is busy for longer (70 to 72 % in ncu at 17 warps per SM), since an instruction "
+                        "FP64 unit is busy for longer (73 % in ncu at 17 warps per SM), since an instruction "
                         "holds it the same time whatever the lanes; ncu summaries in profiles/"}
 
     # end to end with the state in pinned host memory (clmgb.hoststep): each step moves

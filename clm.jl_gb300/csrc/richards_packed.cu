@@ -50,15 +50,18 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr int KS = 8, SLD = KS + 1, HALF = 16;     // slots, their stride, lanes of a half-warp
 // Up to FEW_SLOTS columns for each of FEW_WARPS warps a block the variant with an attempt's
 // quotients and powers in line runs (FEW): a warp waits for its own chain, and independent
-// ones overlap.  ms a call in line / through the shared functions, scale workload: 61 columns
-// 0.249 / 0.268, 1,024 0.459 / 0.486, 8,000 (6 a warp) 0.796 / 0.838, 12,000 (8) 0.818 /
-// 0.832; with warps in different phases, 24,000 columns on, the code is no longer found in the
-// instruction cache (262,144 5.1 / 4.3).
+// ones overlap.  ms a call in line / through the shared functions with MANY_WARPS, scale
+// workload: 61 columns 0.250 / 0.266, 1,024 0.457 / 0.480, 4,000 0.635 / 0.666, 8,000 0.800 /
+// 0.825, 12,000 0.790 / 0.822; with warps in different phases the code is no longer found in
+// the instruction cache: 16,000 1.003 / 0.995, 24,000 1.06 / 1.03, 65,536 1.83 / 1.57, 262,144
+// 5.56 / 3.79.
 constexpr int FEW_SLOTS = 8, FEW_WARPS = 5;
 // Many columns: 2 blocks, 18 warps of 8 columns and 20 levels, in an SM's shared memory.  ms a
 // call at 65,536 / 262,144 columns of the scale workload and at 262,144 of the snow workload:
 // 16 columns and 10 warps 1.72 / 4.27 / 1.65, 12 and 12 1.65 / 4.15 / 1.57, 10 and 14 1.65 /
-// 4.14 / 1.55, 8 and 18 1.65 / 4.03 / 1.42.
+// 4.14 / 1.55, 8 and 18 1.65 / 4.03 / 1.42.  With 22 to 25 levels, or 20 and the expensive flux
+// estimate, one such block fits: 25 levels 2.4 / 7.2 ms, the expensive estimate 2.1 / 6.1 (the
+// kernel with a column per lane 6.4 / 18.7 and 5.6 / 12.8).
 constexpr int MANY_WARPS = 9;
 
 // level arrays: the flux derivatives dqodw1, dqodw2 and the net flux (kept from a

@@ -682,7 +682,7 @@ int32_t clmgb_last_cuda_error(clmgb_handle h);
 #define   CLMGB_SCHEDULE_WAVES         2  /*   cooperative kernel, all columns in synchronous rounds of
                                               uniform phases (needs clmgb_reserve; otherwise QUEUE runs) */
 #define CLMGB_OPT_QUEUE_BLOCKS_PER_SM  2  /* resident blocks per SM of the queue kernel (0 = occupancy limit) */
-#define CLMGB_OPT_QUEUE_OCCUPANCY      3  /* read-only: occupancy limit of the queue kernel */
+#define CLMGB_OPT_QUEUE_OCCUPANCY      3  /* read-only: occupancy limit of the per-lane queue kernel */
 #define CLMGB_OPT_NUM_SMS              4  /* read-only: SMs of the handle's device */
 #define CLMGB_OPT_QUEUE_ORDER          5  /* with reserved scratch: 1 = hand out columns longest-expected-first
                                              (by the previous call's num_substeps, default), 0 = index order */
